@@ -58,7 +58,21 @@ struct SolveConst {
     float e_max;    // exp(max_sim / tau), +inf when unbounded
     float inv_c;    // 1 / c
     bool fast;      // c > 0: the provable rejections below are valid
+    // Of may_cross (set_screen_const):
+    float c4s;         // 4c (1 - 2^-20)
+    float kappa;       // 2^-22 / c
+    unsigned b2_span;  // length of the range of fl(b*b), as float bits from SCREEN_B2_LO on, in which claims are made
 };
+
+// fl(b*b) in [2^-100, 2^120), as float bits.
+constexpr unsigned SCREEN_B2_LO = (127u - 100u) << 23, SCREEN_B2_HI = (127u + 120u) << 23;
+
+inline void set_screen_const(SolveConst& k) {
+    const bool on = k.fast && k.c >= 0x1p-60f && k.c <= 0x1p60f;
+    k.c4s = (4.0f * k.c) * (1.0f - 0x1p-20f);
+    k.kappa = on ? 0x1p-22f / k.c : 0.0f;
+    k.b2_span = on ? SCREEN_B2_HI - SCREEN_B2_LO : 0u;
+}
 
 // True when the reference solver provably accepts no crossing in the window (t_last, t_next] for the
 // state (a, b), so that its exact evaluation can be skipped without changing any result. With
@@ -150,6 +164,91 @@ __device__ __forceinline__ bool no_crossing_at(float a, float b, const EventWind
         left_of_window = ql < -errl || (ql > errl && w.tcZl > b * (1.0f + 0x1p-21f));
     }
     return usable && (level1 || right_of_window || left_of_window);
+}
+
+// (event_window and no_crossing_at state the claims that may_cross, below, rests on; the host tests compare them.)
+
+// The screen of the streaming forward kernels: whether a crossing after an event has to be looked for. It makes the
+// claims of no_crossing (same window margins: Z = min(e_next, e_max) (1 + 1.5 2^-19) < 2980 right of the window,
+// Zl = e_start (1 - 2^-17) < 2981 left of it), in a form that costs half the instructions, since the kernels are
+// bound by instruction issue and run it once per (event, neuron): every test is one comparison with constants formed
+// once per event (cross_window). False means that the reference solver provably accepts no crossing in the window.
+//
+// With B = fl(b*b) in [2^-100, 2^120), |a| <= 2^60 and 2^-60 <= c <= 2^60, no crossing is accepted when one holds:
+//   1. a <= 0: x = sqrt(tmp) >= |b|, so x + b == 0 or z = 2a/(x + b) <= 0, rejected by sign or by its logarithm.
+//   2. b < 2c Zl (1 - 2^-20) (a > 0): b < 0 gives z <= 0; else the solver goes on only if 4ac <= b^2 (1 + 2^-22)
+//      (FC: the discriminant has its exact sign; conv: formed in float), and then z <= 2a/b (1 + 2^-23) lies below
+//      b/(2c) (1 + 2^-21) < Zl: the smaller root lies left of the parabola's vertex, and the vertex left of the
+//      window. (tczl = 0, i.e. b < 0, where Zl is not usable.)
+//   3. fl(a c4s) > B: 4ac > B (1 + 2^-21), so tmp <= -2^-22 B < 0 in every evaluation order.
+//   4. b > 2c Z (1 + 2^-20) and fl(a + c Z^2) > fl(b Zw), Zw = Z (1 + 2^-18): the vertex lies right of Z and
+//      Q(Z) = c Z^2 - b Z + a > 1.5 2^-19 b Z, so Q(Z) > 2^-21 (c Z^2 + b Z + a) (directly if the sum is below
+//      3 b Z, else because Q exceeds a third of it): the right-of-window claim of no_crossing.
+//   5. fl(a + c Zl^2) < fl(b Zl (1 - 2^-18)): Q(Zl) < -2^-21 (c Zl^2 + b Zl + a), Zl between the roots: its
+//      left-of-window claim.
+// CONV adds kappa B >= 2^-23 B / c to the larger side of 4 and 5 for the float discriminant, as no_crossing<true>.
+// Every comparison is false for NaN, and the range tests reject infinities: such states are looked at exactly.
+struct __align__(16) CrossWindow {
+    float es, e;             // the event's exponentials
+    float czz, zw, tcz;      // c Z^2, Z (1 + 2^-18), 2c Z (1 + 2^-20); tcz +inf where test 4 does not apply
+    float czzl, zl, tczl;    // c Zl^2, Zl (1 - 2^-18) (NaN where test 5 does not apply), 2c Zl (1 - 2^-20) or 0
+};
+__device__ __forceinline__ CrossWindow cross_window(float es, float e, float e_start, float e_next,
+                                                    const SolveConst& k) {
+    CrossWindow w;
+    w.es = es;
+    w.e = e;
+    const float Z = fminf(e_next, k.e_max) * (1.0f + 0x1.8p-19f);
+    w.czz = (k.c * Z) * Z;
+    w.zw = Z * (1.0f + 0x1p-18f);
+    w.tcz = Z < 2980.0f ? ((2.0f * k.c) * Z) * (1.0f + 0x1p-20f) : BATS_INF;
+    const float zl = e_start * (1.0f - 0x1p-17f);
+    const bool left = zl > 0.0f && zl < 2981.0f;
+    w.czzl = (k.c * zl) * zl;
+    w.zl = left ? zl * (1.0f - 0x1p-18f) : __int_as_float(0x7fc00000);
+    w.tczl = left ? ((2.0f * k.c) * zl) * (1.0f - 0x1p-20f) : 0.0f;
+    return w;
+}
+// bit if a crossing after the event has to be looked for, else 0. On the device the comparisons are one chain of
+// predicates: nvcc makes branches and integer selects of the same boolean expression (twice the instructions).
+template <bool CONV = false>
+__device__ __forceinline__ unsigned cross_bit(float a, float b, const CrossWindow& w, const SolveConst& k,
+                                              unsigned bit) {
+    const float B = __fmul_rn(b, b);
+    const float p = __fmul_rn(a, k.c4s);
+    const float sr = a + w.czz, bl = __fmul_rn(b, w.zl);
+    float br = __fmul_rn(b, w.zw), sl = a + w.czzl;
+    if (CONV) {
+        br = fmaf(k.kappa, B, br);
+        sl = fmaf(k.kappa, B, sl);
+    }
+    const unsigned off = __float_as_uint(B) - SCREEN_B2_LO;
+#if defined(__CUDA_ARCH__)
+    unsigned r;
+    asm("{\n\t.reg .pred p, q;\n\t.reg .f32 m;\n\t"
+        "abs.f32 m, %1;\n\t"
+        "setp.gt.f32 q, %2, %5;\n\t"          // 4.
+        "setp.gt.and.f32 q, %3, %4, q;\n\t"
+        "setp.le.or.f32 q, %1, 0f00000000, q;\n\t"  // 1.
+        "setp.lt.or.f32 q, %2, %6, q;\n\t"    // 2.
+        "setp.gt.or.f32 q, %7, %8, q;\n\t"    // 3.
+        "setp.lt.or.f32 q, %9, %10, q;\n\t"   // 5.
+        "setp.le.and.f32 q, m, 0f5D800000, q;\n\t"  // |a| <= 2^60
+        "setp.lt.and.u32 q, %11, %12, q;\n\t"
+        "selp.b32 %0, 0, %13, q;\n\t}"
+        : "=r"(r)
+        : "f"(a), "f"(b), "f"(sr), "f"(br), "f"(w.tcz), "f"(w.tczl), "f"(p), "f"(B), "f"(sl), "f"(bl), "r"(off),
+          "r"(k.b2_span), "r"(bit));
+    return r;
+#else
+    bool none = a <= 0.0f || b < w.tczl || p > B || (b > w.tcz && sr > br) || sl < bl;
+    none = none && fabsf(a) <= 0x1p60f && off < k.b2_span;
+    return none ? 0u : bit;
+#endif
+}
+template <bool CONV = false>
+__device__ __forceinline__ bool may_cross(float a, float b, const CrossWindow& w, const SolveConst& k) {
+    return cross_bit<CONV>(a, b, w, k, 1u) != 0u;
 }
 
 // Screen of a run of consecutive events (FC layer, tau = 2 tau_s): true when the reference solver provably
@@ -271,32 +370,22 @@ __device__ __forceinline__ bool solve_crossings_conv_at(float a, float& b, float
         a_out, x_out, t_out, z_out);
 }
 
-// solve_crossings<false> with the event's window constants formed once per stage (event_window).
-__device__ __forceinline__ bool solve_crossings_at(float a, float& b, float last_t, float next_t, const EventWindow& w,
-                                                const SolveConst& k, int& n, int k_post,
+// The solver at an event for which may_cross has just been true: solve_crossings without screening that state
+// again; the states after its spikes are screened by may_cross. base: the neuron's first slot in the outputs.
+template <bool CONV>
+__device__ __forceinline__ bool solve_candidate(float a, float& b, float last_t, float next_t, const CrossWindow& w,
+                                                const SolveConst& k, int& n, int k_post, long long base,
                                                 float* __restrict__ a_out, float* __restrict__ x_out,
                                                 float* __restrict__ t_out, float* __restrict__ z_out) {
-    while (true) {
-        if (no_crossing_at<true>(a, b, w, k)) return false;
-        float tmp;
-        tmp = fc_discriminant(__fmul_rn(b, b), a, k.c);  // == (float)((double)fl(b*b) - 4.0*a*c)
-        if (tmp < 0) return false;
-        const float x_tmp = sqrtf(tmp);
-        tmp = x_tmp + b;
-        if (tmp == 0.0f) return false;
-        const float inside_log = 2 * a / tmp;
-        if (inside_log < 0) return false;
-        tmp = k.tau * __logf(inside_log);
-        if (tmp <= last_t || tmp > k.max_sim || tmp > next_t) return false;
-        a_out[n] = a;
-        x_out[n] = x_tmp;
-        t_out[n] = tmp;
-        z_out[n] = inside_log;
-        last_t = tmp;
-        b -= k.dtt * inside_log;
-        n++;
-        if (n >= k_post) return true;
-    }
+    bool known = true;
+    return solve_crossings_screened<CONV>(
+        a, b, last_t, next_t,
+        [&](float a_, float b_) {
+            const bool none = !known && !may_cross<CONV>(a_, b_, w, k);
+            known = false;
+            return none;
+        },
+        k, n, k_post, a_out + base, x_out + base, t_out + base, z_out + base);
 }
 
 // Position of one post neuron's spike train relative to a time-ordered scan of pre spikes: p = first

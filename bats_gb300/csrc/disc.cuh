@@ -4,14 +4,15 @@
 // (bats/CudaKernels/CuFiles/Inference/compute_spike_times.cu:57): the product 4ac is exact in double,
 // the difference is rounded once to double and then to float. GB300's FP64 rate is a small fraction of
 // its FP32 rate, and in strongly driven layers this line runs after most input events, so it is
-// computed here from FP32 error-free transformations:
-//   P = 4a*c = ph + pl exactly (ph = fl(4a*c), pl = fma(4a, c, -ph)),
-//   B2 - ph = s + e exactly (TwoSum), e - pl = u + f exactly, s + u = r + g exactly,
-// so V = B2 - 4ac = r + g + f exactly and r = fl(s + u). If |g| + |f| stays below half an ulp of r by
-// a margin of 2^-20 of that half ulp (which is far larger than double's rounding of V, 2^-53 |V|),
-// then both fl(V) and fl(fl_double(V)) equal r. Otherwise (V near a midpoint between floats, or
-// operands outside the ranges where the transformations are exact) the double expression itself is
-// evaluated. The result is bit-identical to the reference's expression for every input.
+// computed here from FP32 operations:
+//   r = fma(-4a, c, B2) is V = B2 - 4ac rounded once to float; it differs from the reference only if rounding V to
+//   double first (by at most 2^-53 |V|) reaches a midpoint between floats.
+//   d = V - r up to 2^-46 B2 + 2^-24 |d|: B2 - r = t + te exactly (TwoSum), so V - r = (t - 4ac) + te, and
+//   fma(-4a, c, t) rounds t - 4ac, which is below |V - r| + ulp(t)/2, by 2^-24 of itself.
+// If |d| + 2^-46 B2 stays below half the float spacing around r by a margin of 2^-20 of it (far larger than
+// double's rounding), then fl(V) and fl(fl_double(V)) are both r. Otherwise (V near a midpoint, strong
+// cancellation, operands out of range) the double expression itself is evaluated. The result is bit-identical to
+// the reference's expression for every input; 21 operations in place of the 45 of exact sums of every term.
 #pragma once
 
 #if defined(__CUDACC__)
@@ -60,32 +61,16 @@ float fc_discriminant_ref64(float b2, float a, float c) {
 
 BATS_HD float fc_discriminant(float b2, float a, float c) {
     const float a4 = BATS_FMUL(4.0f, a);
-    const float ph = BATS_FMUL(a4, c);
-    const float pl = BATS_FMA(a4, c, -ph);
-    const float s = BATS_FADD(b2, -ph);
-    const float e = two_sum_err(b2, -ph, s);
-    const float u = BATS_FADD(e, -pl);
-    const float f = two_sum_err(e, -pl, u);
-    const float r = BATS_FADD(s, u);
-    const float g = two_sum_err(s, u, r);
-    const float ab2 = b2 < 0.0f ? -b2 : b2;
-    const float aph = ph < 0.0f ? -ph : ph;
+    const float r = BATS_FMA(-a4, c, b2);
+    const float t = BATS_FADD(b2, -r);
+    const float te = two_sum_err(b2, -r, t);
+    const float d = BATS_FADD(BATS_FMA(-a4, c, t), te);
     const float ar = r < 0.0f ? -r : r;
-    // Ranges where every step above is exact and r is a normal float well above the subnormals:
-    // |b2|, |ph| < 2^120 (no overflow in the sums); 4a*c exactly zero or |ph| >= 2^-90 (pl exact);
-    // |r| >= 2^-90.
-    const bool in_range = ab2 < 0x1p120f && aph < 0x1p120f && (a4 == 0.0f || c == 0.0f || aph >= 0x1p-90f) &&
-                          ar >= 0x1p-90f;
-    // Half the spacing of the floats around r: 2^(exponent(r) - 24), halved on the side towards zero
-    // when r is a power of two (the spacing below a power of two is half the spacing above it).
-    const int rbits = BATS_F2I(ar);
-    float lim = BATS_I2F((rbits & 0x7f800000) - (24 << 23));
-    const float d = BATS_FADD(g, f);
-    const bool toward_zero = (r > 0.0f) ? (d < 0.0f) : (d > 0.0f);
-    if ((rbits & 0x007fffff) == 0 && toward_zero) lim = BATS_FMUL(lim, 0.5f);
-    const float ag = g < 0.0f ? -g : g;
-    const float af = f < 0.0f ? -f : f;
-    const bool safe = in_range && BATS_FADD(ag, af) < BATS_FMUL(lim, 1.0f - 0x1p-20f);
+    const float ad = d < 0.0f ? -d : d;
+    // Half the spacing of the floats on r's side towards zero (half as wide when r is a power of two).
+    const float lim = BATS_I2F(((BATS_F2I(ar) - 1) & 0x7f800000) - (24 << 23));
+    const bool safe = b2 < 0x1p120f && ar < 0x1p120f && ar >= 0x1p-90f &&
+                      BATS_FMA(0x1p-46f, b2, ad) < BATS_FMUL(lim, 1.0f - 0x1p-20f);
     if (safe) return r;
     return fc_discriminant_ref64(b2, a, c);
 }

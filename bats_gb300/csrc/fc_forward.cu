@@ -7,13 +7,13 @@
 //
 // Grid (ceil(N_post / TILE), B): one CTA per (post-neuron tile, sample). The reference gathers a
 // dense (B, N_post, S) weight array first; here a producer warp streams, for every event of the
-// sample in time order, the event record and the weight-row segment wt[j, tile] (TILE floats) into a
-// ring of shared-memory stages with bulk copies (cp.async.bulk, completing on an mbarrier), running
+// sample in time order, its window constants and the weight-row segment wt[j, tile] (TILE floats) into a
+// ring of shared-memory stages (the rows with bulk copies, cp.async.bulk, completing on an mbarrier), running
 // up to STAGES * SEV events ahead of the consumers, so no weight load sits on the consumers' path.
 // Each consumer thread owns one post neuron and runs the reference's recurrence
 // a += w*exp(t/tau_s), b += w*exp(t/tau), crossing search in (t_event, t_next_event].
-// Per stage the consumer first accumulates all SEV events and evaluates the provable no-crossing
-// test on each intermediate state; only if some event may cross does it replay the stage from its
+// Per stage the consumer first accumulates all SEV events and evaluates the provable screen
+// (may_cross) on each intermediate state; only if some event may cross does it replay the stage from its
 // saved state with the exact solver. The accumulation is the same FMA sequence either way, so the
 // results are those of the reference's one-event-at-a-time loop.
 //
@@ -31,18 +31,147 @@
 
 namespace bats {
 
-// Consumer warps' part of one work item (sample s, post neurons tile0 .. tile0 + TILE - 1): thread = post
-// neuron. The item's event stages are stages k0 .. k0 + ceil(E / SEV) - 1 of the CTA's ring (k0 = 0 when the
-// CTA has one item). Returns false when a wait gave up (the CTA is aborting).
+// Shared memory of one CTA: a ring of STAGES stages of SEV events, each with its weight-row segments (bulk copies),
+// its window constants and times (written by the producer), and the full / empty mbarriers.
+template <int TILE, int SEV, int STAGES>
+struct FwdSmem {
+    float rows[STAGES][SEV][TILE];
+    CrossWindow win[STAGES][SEV];
+    float t[STAGES][SEV + 1];  // t[u + 1]: the end of event u's window
+    uint64_t full[STAGES];
+    uint64_t empty[STAGES];
+    int abort;
+    int stop_at;              // ring position of the marker that ended an item early (forward_produce)
+    int finished[TILE / 32];  // per consumer warp: the last work item whose remaining events it does not need
+};
+
+// Position in the ring: the running stage count, its slot and the slot's phase parity.
+template <int STAGES>
+struct RingPos {
+    int k = 0, slot = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void next() {
+        ++k;
+        if (++slot == STAGES) {
+            slot = 0;
+            phase ^= 1u;
+        }
+    }
+};
+
+template <int TILE, int SEV, int STAGES>
+__device__ __forceinline__ void forward_init(FwdSmem<TILE, SEV, STAGES>& sm, int consumer_warps) {
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < STAGES; ++q) {
+            mbar_init(&sm.full[q], 1);
+            mbar_init(&sm.empty[q], consumer_warps);
+        }
+        sm.abort = 0;
+        sm.stop_at = -1;
+        for (int w = 0; w < TILE / 32; ++w) sm.finished[w] = -1;
+        fence_barrier_init();
+    }
+}
+
+// Producer warp, one work item: streams the events' weight-row segments wt[j, tile0 : tile0 + TILE] and window
+// constants through the ring. Lane l handles event l of each block of 32 (its record is loaded two blocks ahead, its
+// window constants are formed once for all consumer warps), and copies its row when the block's stage is due.
+// When every consumer warp has marked the item in sm.finished (its neurons all have k_post spikes, so no later event
+// can change an output), the item's next stage becomes a marker without data (sm.stop_at, then one arrival on its
+// full barrier) and the item ends with it; the consumers acquire every stage up to the marker, so no copy is in
+// flight when they leave the item. Returns false when a wait gave up (the CTA abort flag is raised).
+template <int TILE, int SEV, int STAGES>
+__device__ __forceinline__ bool forward_produce(FwdSmem<TILE, SEV, STAGES>& sm, RingPos<STAGES>& pos, int it,
+                                                const Event* __restrict__ evs, int E, const float* __restrict__ wt,
+                                                int ld, int tile0, int consumer_warps, const SolveConst& sk, int lane,
+                                                int* status) {
+    constexpr int SPB = 32 / SEV;  // stages per block of 32 events
+    const uint32_t row_bytes = (uint32_t)min(TILE, ld - tile0) * 4u;
+    const int n_stages = (E + SEV - 1) / SEV;
+    const float4* src = reinterpret_cast<const float4*>(evs);
+    const float4 none = make_float4(BATS_INF, 0.0f, 0.0f, BATS_INF);
+    float4 nx1 = lane < E ? __ldg(src + lane) : none;
+    float4 nx2 = lane + 32 < E ? __ldg(src + lane + 32) : none;
+    for (int kb = 0; kb < n_stages; kb += SPB) {
+        const float4 ev = nx1;  // (t, j, es, e)
+        const int m = kb * SEV + lane;
+        nx1 = nx2;
+        nx2 = m + 64 < E ? __ldg(src + m + 64) : none;
+        float t_next = __shfl_down_sync(0xffffffffu, ev.x, 1), e_next = __shfl_down_sync(0xffffffffu, ev.w, 1);
+        const float t_blk = __shfl_sync(0xffffffffu, nx1.x, 0), e_blk = __shfl_sync(0xffffffffu, nx1.w, 0);
+        if (lane == 31) {
+            t_next = t_blk;
+            e_next = e_blk;
+        }
+        const CrossWindow w = cross_window(ev.z, ev.w, ev.w, e_next, sk);
+        const float* row = wt + (long long)__float_as_int(ev.y) * ld + tile0;
+#pragma unroll
+        for (int i = 0; i < SPB; ++i) {
+            if (kb + i >= n_stages) break;
+            const bool ok = mbar_wait(&sm.empty[pos.slot], pos.phase ^ 1u, &sm.abort, status);
+            if (!__all_sync(0xffffffffu, ok)) return false;
+            if (i == 0) {
+                const bool fin = lane >= consumer_warps || *(volatile int*)&sm.finished[lane] == it;
+                if (__all_sync(0xffffffffu, fin)) {
+                    if (lane == 0) {
+                        *(volatile int*)&sm.stop_at = pos.k;
+                        mbar_arrive(&sm.full[pos.slot]);  // release: stop_at is visible to the acquiring waits
+                    }
+                    __syncwarp();
+                    pos.next();
+                    return true;
+                }
+            }
+            const bool mine = lane / SEV == i && m < E;
+            if (mine) {
+                const int u = lane % SEV;
+                sm.win[pos.slot][u] = w;
+                sm.t[pos.slot][u] = ev.x;
+                if (u == SEV - 1 || m == E - 1) sm.t[pos.slot][u + 1] = t_next;
+            }
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive_expect_tx(&sm.full[pos.slot], (uint32_t)min(SEV, E - (kb + i) * SEV) * row_bytes);
+            __syncwarp();
+            if (mine) bulk_copy_g2s(&sm.rows[pos.slot][lane % SEV][0], row, row_bytes, &sm.full[pos.slot]);
+            pos.next();
+        }
+    }
+    return true;
+}
+
+// After an abort: bounded waits for the copies of the last STAGES issued stages, so that no bulk copy into shared
+// memory is in flight when the CTA exits.
+template <int TILE, int SEV, int STAGES>
+__device__ __forceinline__ void forward_drain(FwdSmem<TILE, SEV, STAGES>& sm, int issued) {
+    for (int k = max(0, issued - STAGES); k < issued; ++k) {
+        volatile int dummy = 0;
+        mbar_wait(&sm.full[k % STAGES], (k / STAGES) & 1, &dummy, nullptr);
+    }
+}
+
+constexpr int STOP_EVERY = 8;  // stages between two looks at whether every neuron of a warp is done
+
+// Consumer warps' part of one work item (sample s, post neurons tile0 .. tile0 + TILE - 1): thread = post neuron.
+// Returns false when a wait gave up (the CTA is aborting).
+//
+// Pass 1 accumulates a stage's events (the reference's FMA sequence) and marks every event after which a crossing
+// cannot be ruled out (may_cross): branch-free, so the per-event tests of the stage overlap. Pass 2, for the neurons
+// with a marked event, is the reference's event-by-event loop from that event on.
 // SCREEN: every full stage first runs only the accumulation, tracking the smallest a and |a| and the largest
 // b of its states, and skips the per-event tests when stage_no_crossing rules out a crossing after any of
 // its events (quiet neurons: one test per stage instead of one per event); otherwise the stage is
 // evaluated as without SCREEN. The FMA sequence is the same either way, so results are bit-identical.
-// Each warp forms the window constants of the stage's events once (event_window, lane u for event u) and every
-// neuron's per-event test reads them (no_crossing_at: the answers of no_crossing, with fewer instructions).
-template <int TILE, int SEV, int STAGES, bool SCREEN = false>
-__device__ __forceinline__ bool forward_tile_item(StreamSmem<TILE, SEV, STAGES>& sm, int k0, int s, int tile0, int E,
-                                                  int n_post, int k_post, const SolveConst& sk,
+// A neuron with k_post spikes is done; a warp whose neurons are all done only passes stages on (see forward_produce).
+//
+// What bounds it: instruction issue (76 % of the issue slots), 590 warp instructions per warp and 8-event stage of an
+// active 800 x 800 layer (batch 256, 652 events a sample, 1.4 spikes per warp and stage), 884 with a screen per
+// event twice as long, without the left-of-window test in pass 1 (whose false candidates then ran pass 2) and with
+// the window constants formed by every consumer warp: 0.587 -> 0.396 ms there, 3.43 -> 2.26 ms on 1024 x 1024 with
+// 4096 uneven samples. Two neurons per thread: 0.349 and 2.34 ms, and slower on every smaller grid.
+template <int TILE, int SEV, int STAGES, bool SCREEN>
+__device__ __forceinline__ bool forward_tile_item(FwdSmem<TILE, SEV, STAGES>& sm, RingPos<STAGES>& pos, int it, int s,
+                                                  int tile0, int E, int n_post, int k_post, const SolveConst& sk,
                                                   int* __restrict__ n_spikes, float* __restrict__ a_out,
                                                   float* __restrict__ x_out, float* __restrict__ t_out,
                                                   float* __restrict__ z_out, int* status, int pad) {
@@ -52,102 +181,92 @@ __device__ __forceinline__ bool forward_tile_item(StreamSmem<TILE, SEV, STAGES>&
     const int i = tile0 + tid;
     const bool active = i < n_post;
     const long long obase = ((long long)s * n_post + (active ? i : 0)) * k_post;
-    float* ao = a_out + obase;
-    float* xo = x_out + obase;
-    float* to = t_out + obase;
-    float* zo = z_out + obase;
     float a = 0.0f, b = 0.0f;
     int n = 0;
     bool done = !active;
-    __shared__ EventWindow s_win[TILE / 32][SEV];
-    EventWindow* wv = s_win[warp];
+    bool all_done = false;  // warp-uniform
     for (int k = 0; k < n_stages; ++k) {
-        const int kg = k0 + k;  // the stage's place in the CTA's ring
-        const int slot = kg % STAGES;
-        if (!stream_acquire(sm, kg, status)) return false;
-        const int m0 = k * SEV;
-        const int cnt = min(SEV, E - m0);
-        const Event* se = sm.evs[slot];
-        // The window constants of the stage's events, formed once per warp (lane u: event u).
-        if (lane < SEV) {
-            const float e_nx = (m0 + lane + 1 < E) ? se[lane + 1].e : BATS_INF;
-            wv[lane] = event_window(se[lane].e, e_nx, sk);
-        }
-        __syncwarp();
-        if (!done) {
-            // Pass 1: accumulate the stage's events (the reference's FMA sequence) and mark every event
-            // after which a crossing cannot be ruled out. Branch-free, so the per-event tests of the
-            // stage overlap; events past the sample's end (last stage) leave the state unchanged.
+        const int slot = pos.slot;
+        const bool ok = mbar_wait(&sm.full[slot], pos.phase, &sm.abort, status);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        const bool stop = all_done && *(volatile int*)&sm.stop_at == pos.k;  // the marker of an item ended early
+        if (!all_done && !done) {
+            const int cnt = min(SEV, E - k * SEV);
+            const CrossWindow* win = sm.win[slot];
+            const float* row = &sm.rows[slot][0][tid];
             float aa = a, bb = b;
             unsigned cand = 0u;
+            auto step = [&](int u) {
+                const CrossWindow c = win[u];
+                const float w = row[u * TILE];
+                aa = fmaf(w, c.es, aa);
+                bb = fmaf(w, c.e, bb);
+                cand |= cross_bit(aa, bb, c, sk, 1u << u);
+            };
             bool screened = false;
-            if (SCREEN && m0 + SEV < E) {
+            if (SCREEN && (k + 1) * SEV < E) {
                 float amin = BATS_INF, bmax = -BATS_INF, amag = BATS_INF;
 #pragma unroll
                 for (int u = 0; u < SEV; ++u) {
-                    const float w = sm.rows[slot][u][tid];
-                    aa = fmaf(w, se[u].es, aa);
-                    bb = fmaf(w, se[u].e, bb);
+                    const float w = row[u * TILE];
+                    aa = fmaf(w, win[u].es, aa);
+                    bb = fmaf(w, win[u].e, bb);
                     amin = fminf(amin, aa);
                     amag = fminf(amag, fabsf(aa));
                     bmax = fmaxf(bmax, bb);
                 }
-                screened = stage_no_crossing(amin, bmax, amag, aa, bb, se[0].e, sk);
+                screened = stage_no_crossing(amin, bmax, amag, aa, bb, win[0].e, sk);
                 if (!screened) {
                     aa = a;
                     bb = b;
                 }
             }
-            if (screened) {
-                // no event of the stage can cross: aa, bb hold the state after the stage
-            } else if (m0 + SEV < E) {
-                // A full stage followed by more events (every stage but the last): no bounds to select on.
+            if (!screened) {
+                if (cnt == SEV) {
 #pragma unroll
-                for (int u = 0; u < SEV; ++u) {
-                    const float4 e4 = *reinterpret_cast<const float4*>(&se[u]);  // (t, j, es, e)
-                    const float w = sm.rows[slot][u][tid];
-                    aa = fmaf(w, e4.z, aa);
-                    bb = fmaf(w, e4.w, bb);
-                    cand |= no_crossing_at<false>(aa, bb, wv[u], sk) ? 0u : (1u << u);
-                }
-            } else {
+                    for (int u = 0; u < SEV; ++u) step(u);
+                } else {  // the sample's last stage
 #pragma unroll
-                for (int u = 0; u < SEV; ++u) {
-                    const float4 e4 = *reinterpret_cast<const float4*>(&se[u]);
-                    const float w = sm.rows[slot][u][tid];
-                    const bool in = u < cnt;
-                    const float a2 = fmaf(w, e4.z, aa);
-                    const float b2 = fmaf(w, e4.w, bb);
-                    aa = in ? a2 : aa;
-                    bb = in ? b2 : bb;
-                    const bool maybe = !no_crossing_at<false>(aa, bb, wv[u], sk);
-                    cand |= (in && maybe) ? (1u << u) : 0u;
+                    for (int u = 0; u < SEV; ++u)
+                        if (u < cnt) step(u);
                 }
             }
-            if (cand == 0u) {
-                a = aa;
-                b = bb;
-            } else {
-                // Pass 2: no crossing is possible before the first marked event, so its state is
-                // reached by the plain accumulation; from there on, the reference's event-by-event loop.
+            if (cand) {
+                // No crossing is possible before the first marked event: its state is reached by plain accumulation.
                 const int first = __ffs(cand) - 1;
-                for (int u = 0; u < first; ++u) {
-                    const float wu = sm.rows[slot][u][tid];
-                    a = fmaf(wu, se[u].es, a);
-                    b = fmaf(wu, se[u].e, b);
+                aa = a;
+                bb = b;
+                for (int u = 0; u <= first; ++u) {
+                    const float w = row[u * TILE];
+                    aa = fmaf(w, win[u].es, aa);
+                    bb = fmaf(w, win[u].e, bb);
                 }
-                for (int u = first; u < cnt; ++u) {
-                    const Event e = se[u];
-                    const float wu = sm.rows[slot][u][tid];
-                    a = fmaf(wu, e.es, a);
-                    b = fmaf(wu, e.e, b);
-                    const float t_next = m0 + u + 1 < E ? se[u + 1].t : BATS_INF;
-                    done = solve_crossings_at(a, b, e.t, t_next, wv[u], sk, n, k_post, ao, xo, to, zo);
-                    if (done) break;
+                bool cross = true;
+                for (int u = first;;) {
+                    if (cross && solve_candidate<false>(aa, bb, sm.t[slot][u], sm.t[slot][u + 1], win[u], sk, n, k_post,
+                                                        obase, a_out, x_out, t_out, z_out)) {
+                        done = true;
+                        break;
+                    }
+                    if (++u >= cnt) break;
+                    const CrossWindow c = win[u];
+                    const float w = row[u * TILE];
+                    aa = fmaf(w, c.es, aa);
+                    bb = fmaf(w, c.e, bb);
+                    cross = may_cross(aa, bb, c, sk);
                 }
             }
+            a = aa;
+            b = bb;
         }
-        stream_release(sm, kg);
+        if ((k & (STOP_EVERY - 1)) == STOP_EVERY - 1 && !all_done) {
+            all_done = __all_sync(0xffffffffu, done);
+            if (all_done && lane == 0) *(volatile int*)&sm.finished[warp] = it;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.empty[slot]);
+        pos.next();
+        if (stop) break;
     }
     if (active) n_spikes[(long long)s * n_post + i] = n;
     // +inf past each neuron's spikes. The warp's 32 neurons own contiguous rows of k_post slots, so the
@@ -173,23 +292,24 @@ lif_fc_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_c
                       float* __restrict__ t_out, float* __restrict__ z_out, int* __restrict__ status, int pad) {
     pdl_prologue();
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    using Smem = StreamSmem<TILE, SEV, STAGES>;
+    using Smem = FwdSmem<TILE, SEV, STAGES>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     constexpr int CONSUMER_WARPS = TILE / 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int s = blockIdx.y;
     const int tile0 = blockIdx.x * TILE;
     const int E = ev_count[s];
-    const int n_stages = (E + SEV - 1) / SEV;
-    const Event* evs = ev + (long long)s * ev_cap;
-    stream_init(sm, CONSUMER_WARPS);
+    forward_init(sm, CONSUMER_WARPS);
     __syncthreads();
+    RingPos<STAGES> pos;
     if (warp == CONSUMER_WARPS) {
-        stream_produce(sm, evs, E, wt, ld, tile0, n_stages, lane, status);
+        if (!forward_produce(sm, pos, 0, ev + (long long)s * ev_cap, E, wt, ld, tile0, CONSUMER_WARPS, sk, lane,
+                             status))
+            forward_drain(sm, pos.k);
         return;
     }
-    forward_tile_item<TILE, SEV, STAGES, SCREEN>(sm, 0, s, tile0, E, n_post, k_post, sk, n_spikes, a_out, x_out, t_out,
-                                                z_out, status, pad);
+    forward_tile_item<TILE, SEV, STAGES, SCREEN>(sm, pos, 0, s, tile0, E, n_post, k_post, sk, n_spikes, a_out,
+                                                      x_out, t_out, z_out, status, pad);
 }
 
 // Persistent variant over a work queue, for batches whose samples carry very different numbers of events.
@@ -228,7 +348,7 @@ lif_fc_forward_queue_kernel(const Event* __restrict__ ev, const int* __restrict_
                             const int* __restrict__ order, int* __restrict__ head, int n_tiles, int n_items) {
     pdl_prologue();
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    using Smem = StreamSmem<TILE, SEV, STAGES>;
+    using Smem = FwdSmem<TILE, SEV, STAGES>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
     ItemMailbox& box = *reinterpret_cast<ItemMailbox*>(smem_raw + mailbox_offset<Smem>());
     constexpr int CONSUMER_WARPS = TILE / 32;
@@ -239,10 +359,10 @@ lif_fc_forward_queue_kernel(const Event* __restrict__ ev, const int* __restrict_
             mbar_init(&box.empty[q], CONSUMER_WARPS);
         }
     }
-    stream_init(sm, CONSUMER_WARPS);  // thread 0: the stage barriers, then the barrier-init fence
+    forward_init(sm, CONSUMER_WARPS);  // thread 0: the stage barriers, then the barrier-init fence
     __syncthreads();
+    RingPos<STAGES> pos;
     if (warp == CONSUMER_WARPS) {
-        int issued = 0;  // stages issued by this CTA so far
         for (int it = 0;; ++it) {
             int item = 0;
             if (lane == 0) item = atomicAdd(head, 1);
@@ -262,16 +382,13 @@ lif_fc_forward_queue_kernel(const Event* __restrict__ ev, const int* __restrict_
                 mbar_arrive(&box.full[q]);  // release: the item is visible to the consumers' acquiring wait
             }
             if (w.s < 0) break;
-            const int n_stages = (w.E + SEV - 1) / SEV;
-            const int done = stream_produce_at(sm, ev + (long long)w.s * ev_cap, w.E, wt, ld, w.tile0, n_stages,
-                                               issued, lane, status);
-            issued += done;
-            if (done < n_stages) break;
+            if (!forward_produce(sm, pos, it, ev + (long long)w.s * ev_cap, w.E, wt, ld, w.tile0, CONSUMER_WARPS, sk,
+                                 lane, status))
+                break;
         }
-        if (sm.abort) stream_drain(sm, issued);
+        if (sm.abort) forward_drain(sm, pos.k);
         return;
     }
-    int k0 = 0;  // the current item's first stage in the ring
     for (int it = 0;; ++it) {
         const int q = it & 1;
         const bool ok = mbar_wait(&box.full[q], (it >> 1) & 1, &sm.abort, status);
@@ -281,10 +398,9 @@ lif_fc_forward_queue_kernel(const Event* __restrict__ ev, const int* __restrict_
         __syncwarp();
         if (lane == 0) mbar_arrive(&box.empty[q]);
         if (s < 0) return;
-        if (!forward_tile_item<TILE, SEV, STAGES, SCREEN>(sm, k0, s, tile0, E, n_post, k_post, sk, n_spikes, a_out,
-                                                         x_out, t_out, z_out, status, pad))
+        if (!forward_tile_item<TILE, SEV, STAGES, SCREEN>(sm, pos, it, s, tile0, E, n_post, k_post, sk, n_spikes,
+                                                               a_out, x_out, t_out, z_out, status, pad))
             return;
-        k0 += (E + SEV - 1) / SEV;
     }
 }
 
@@ -471,7 +587,7 @@ template <int TILE, int SEV, int STAGES, bool SCREEN>
 static int launch_forward(const void* events, const int* ev_count, long long ev_cap, const float* wt, int ld, int batch,
                           int n_post, int k_post, const SolveConst& sk, int* n_spikes, float* a, float* x,
                           float* times, float* post_exp_tau, int* status, int pad, cudaStream_t stream) {
-    const size_t smem = sizeof(StreamSmem<TILE, SEV, STAGES>);
+    const size_t smem = sizeof(FwdSmem<TILE, SEV, STAGES>);
     BATS_CUDA((cudaError_t)max_dynamic_smem_set((const void*)lif_fc_forward_kernel<TILE, SEV, STAGES, SCREEN>,
                                                 (int)smem));
     dim3 grid((n_post + TILE - 1) / TILE, batch);
@@ -489,7 +605,7 @@ static int launch_forward_queue(const void* events, const int* ev_count, long lo
                                 int batch, int n_post, int k_post, const SolveConst& sk, int* n_spikes, float* a,
                                 float* x, float* times, float* post_exp_tau, int* status, int pad, int* order,
                                 int* head, cudaStream_t stream) {
-    using Smem = StreamSmem<TILE, SEV, STAGES>;
+    using Smem = FwdSmem<TILE, SEV, STAGES>;
     const size_t smem = mailbox_offset<Smem>() + sizeof(ItemMailbox);
     const void* kern = (const void*)lif_fc_forward_queue_kernel<TILE, SEV, STAGES, SCREEN>;
     BATS_CUDA((cudaError_t)max_dynamic_smem_set(kern, (int)smem));
@@ -534,6 +650,7 @@ SolveConst make_solve_const(float c, float dtt, float tau, float max_sim) {
     k.e_max = std::isfinite(em) && em < 3.0e38 ? (float)em : std::numeric_limits<float>::infinity();
     k.inv_c = c > 0.0f ? 1.0f / c : 0.0f;
     k.fast = c > 0.0f && tau > 0.0f;
+    set_screen_const(k);
     return k;
 }
 

@@ -87,7 +87,8 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
 // Event stream: a producer warp copies, stage by stage, SEV time-sorted event records (plus the next
 // one, for the window end) and their weight-row segments wt[j, tile0 : tile0 + TILE] into a ring of
 // STAGES shared-memory stages; consumer warps acquire a stage (full barrier), read it, and release it
-// (empty barrier, one arrival per consumer warp). Used by the forward and error-propagation kernels.
+// (empty barrier, one arrival per consumer warp). Used by the error-propagation kernel (the forward kernels have
+// a ring of their own, with window constants in place of the records: fc_forward.cu).
 #include "common.cuh"
 
 namespace bats {
@@ -127,16 +128,14 @@ __device__ __forceinline__ void stream_drain(StreamSmem<TILE, SEV, STAGES>& sm, 
 // global load takes, so with one stage of look-ahead every stage waited for its load; eight stages cover it.
 constexpr int STREAM_PREFETCH = 8;
 
-// Producer of stages k0 .. k0 + n_stages - 1 of the ring (k0 = 0: one work item per CTA; persistent kernels
-// continue the running stage count of earlier items, so slot and phase follow it). Lane u issues the row
-// copy of the stage's event u (SEV <= 32); the pre-neuron indices of the next STREAM_PREFETCH stages are in
-// flight in registers (a ring indexed statically by unrolling). Returns the number of stages whose copies
-// were issued: n_stages, or fewer when a wait gave up (the CTA abort flag is then raised; drain with
-// stream_drain).
+// Producer warp. Lane u issues the row copy of the stage's event u (SEV <= 32); the pre-neuron indices of the next
+// STREAM_PREFETCH stages are in flight in registers (a ring indexed statically by unrolling). When a wait gives up
+// (the CTA abort flag is then raised) the issued copies are drained: it never returns with copies in flight into
+// shared memory after an abort.
 template <int TILE, int SEV, int STAGES>
-__device__ __forceinline__ int stream_produce_at(StreamSmem<TILE, SEV, STAGES>& sm, const Event* __restrict__ evs,
-                                                 int E, const float* __restrict__ wt, int ld, int tile0,
-                                                 int n_stages, int k0, int lane, int* status) {
+__device__ __forceinline__ void stream_produce(StreamSmem<TILE, SEV, STAGES>& sm, const Event* __restrict__ evs, int E,
+                                               const float* __restrict__ wt, int ld, int tile0, int n_stages,
+                                               int lane, int* status) {
     static_assert(SEV <= 32, "one event per producer lane");
     constexpr int D = STREAM_PREFETCH;
     const uint32_t row_bytes = (uint32_t)min(TILE, ld - tile0) * 4u;
@@ -151,13 +150,15 @@ __device__ __forceinline__ int stream_produce_at(StreamSmem<TILE, SEV, STAGES>& 
         for (int d = 0; d < D; ++d) {
             const int k = kb + d;
             if (k >= n_stages) break;
-            const int kg = k0 + k;
-            const int slot = kg % STAGES;
+            const int slot = k % STAGES;
             const int j = jr[d];
             const int m_ahead = (k + D) * SEV + lane;
             jr[d] = (lane < SEV && m_ahead < E) ? __ldg(&evs[m_ahead].j) : 0;
-            const bool ok = mbar_wait(&sm.empty[slot], ((kg / STAGES) & 1) ^ 1, &sm.abort, status);
-            if (!__all_sync(0xffffffffu, ok)) return k;
+            const bool ok = mbar_wait(&sm.empty[slot], ((k / STAGES) & 1) ^ 1, &sm.abort, status);
+            if (!__all_sync(0xffffffffu, ok)) {
+                stream_drain(sm, k);
+                return;
+            }
             const int m0 = k * SEV;
             const int cnt = min(SEV, E - m0);
             const int cnt_ev = min(SEV + 1, E - m0);
@@ -169,16 +170,7 @@ __device__ __forceinline__ int stream_produce_at(StreamSmem<TILE, SEV, STAGES>& 
                 bulk_copy_g2s(&sm.rows[slot][lane][0], wt + (long long)j * ld + tile0, row_bytes, &sm.full[slot]);
         }
     }
-    return n_stages;
-}
-
-// Producer warp body of a CTA with one work item. Never returns with copies in flight into shared memory.
-template <int TILE, int SEV, int STAGES>
-__device__ __forceinline__ void stream_produce(StreamSmem<TILE, SEV, STAGES>& sm, const Event* __restrict__ evs, int E,
-                                               const float* __restrict__ wt, int ld, int tile0, int n_stages,
-                                               int lane, int* status) {
-    const int issued = stream_produce_at(sm, evs, E, wt, ld, tile0, n_stages, 0, lane, status);
-    if (sm.abort) stream_drain(sm, issued);
+    if (sm.abort) stream_drain(sm, n_stages);
 }
 
 // Consumer side: wait for stage k (all lanes of the warp agree on the outcome).
