@@ -2,7 +2,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <utility>
 #include "abi_util.h"
 
 namespace bats {
@@ -13,26 +15,23 @@ void set_last_error(int status, const char* where, const char* what) {
     std::snprintf(g_last_error, sizeof(g_last_error), "%s: %s (status %d)", where, what, status);
 }
 
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device), for any dynamic size: a kernel's
-// static shared memory counts toward the 48 KB that needs no opt-in. Returns a cudaError_t.
+// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) per (kernel, device), for any dynamic size: a kernel's static
+// shared memory counts toward the 48 KB that needs no opt-in. The attribute belongs to the process and setting it
+// to a smaller size also lowers the limit, so the largest size asked for by any thread is kept: a call from one thread
+// (torch runs backward passes in its own) never lowers it under another's. Returns a cudaError_t.
 int max_dynamic_smem_set(const void* func, int bytes) {
     if (bytes <= 0) return (int)cudaSuccess;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    struct Entry {
-        const void* f;
-        int dev;
-        int bytes;
-    };
-    static thread_local Entry cache[64];
-    static thread_local int used = 0;
-    for (int q = 0; q < used; ++q)
-        if (cache[q].f == func && cache[q].dev == dev && cache[q].bytes >= bytes) return (int)cudaSuccess;
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, int> largest;
+    std::lock_guard<std::mutex> lock(mu);
+    int& have = largest[{func, dev}];
+    if (have >= bytes) return (int)cudaSuccess;
     e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return (int)e;
-    if (used < 64) cache[used++] = Entry{func, dev, bytes};
-    return (int)cudaSuccess;
+    if (e == cudaSuccess) have = bytes;
+    return (int)e;
 }
 
 bool pdl_enabled() {
