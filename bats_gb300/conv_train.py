@@ -23,7 +23,7 @@ import torch
 
 from . import kernels as K
 from ._lib import call, ptr, stream_ptr
-from .train import FCLayerSpec, enqueue_launches
+from .train import FCLayerSpec, enqueue_launches, no_collection
 
 
 @dataclass
@@ -260,7 +260,7 @@ class ConvTrainStep:
             g = torch.cuda.CUDAGraph()
             side = torch.cuda.Stream()
             side.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(side):
+            with torch.cuda.stream(side), no_collection():
                 with torch.cuda.graph(g, stream=side):
                     enqueue_launches(self.launches, self._side_launches(), side, self.aux)
             torch.cuda.current_stream().wait_stream(side)

@@ -10,6 +10,8 @@ its hidden layers (self.out) hold valid times only below their spike counts (no 
 """
 from __future__ import annotations
 
+import contextlib
+import gc
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -356,7 +358,7 @@ class FCTrainStep:
             g = torch.cuda.CUDAGraph()
             side = torch.cuda.Stream()
             side.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(side):
+            with torch.cuda.stream(side), no_collection():
                 with torch.cuda.graph(g, stream=side):
                     self._enqueue(side, self.aux)
             torch.cuda.current_stream().wait_stream(side)
@@ -495,6 +497,20 @@ class FCTrainStep:
     @property
     def d2h_bytes(self) -> int:
         return self.h_loss.numel() * 4
+
+
+@contextlib.contextmanager
+def no_collection():
+    """Automatic garbage collection off (restored afterwards): a collection during a graph capture may free an older
+    step (its launch list holds it in a reference cycle) with its CUDA graph, and the calls that frees it with
+    invalidate the capture."""
+    was = gc.isenabled()
+    gc.disable()
+    try:
+        yield
+    finally:
+        if was:
+            gc.enable()
 
 
 def enqueue_launches(launches, side, main, aux=None) -> None:
