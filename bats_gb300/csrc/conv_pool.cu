@@ -31,116 +31,258 @@
 
 namespace bats {
 
-struct ConvEvent {
+// An event inside the receptive field of a CTA's positions.
+struct __align__(16) ConvEvent {
     float t, es, e;
-    int xyc;  // x | y << 10 | c << 20
+    int xyc;  // x | y << 10 | c << 20; bit 31: an exponential is not finite (relevant to every neuron)
 };
 
-constexpr int CONV_CHUNK = 256;
+constexpr int CONV_SUB = 64;               // kept events per round of the lists
+constexpr int CONV_GROUP = 8;              // list entries per pass of the screen
+constexpr int CONV_LIST = CONV_SUB + CONV_GROUP;
+constexpr int CONV_POSITIONS = 32;         // positions per CTA at most (2.9 KB of list each)
 
-__global__ void conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_count, long long ev_cap,
-                                    const float* __restrict__ W, int X, int Y, int C, int fx, int fy, int C_out,
-                                    int Xo, int Yo, int TX, int TY, int tiles_y, int k_post, SolveConst sk,
-                                    int w_in_smem, int* __restrict__ n_spikes,
-                                    float* __restrict__ a_out, float* __restrict__ x_out, float* __restrict__ t_out,
-                                    float* __restrict__ z_out) {
+// One position's list of relevant events, in time order: window constants (the window ends at the next relevant
+// event), times and filter rows ((dx fy + dy) C + c, or -1: weight 0).
+struct ConvList {
+    CrossWindow win[CONV_LIST];
+    float t[CONV_LIST + 1];
+    int row[CONV_LIST];
+    int n;       // entries
+    int groups;  // groups of CONV_GROUP entries that may be processed (the last entry waits for its window's end)
+    int pad_[5];
+};
+
+// Appends the kept events sev[0 .. cnt) that are relevant to position (xo, yo) to its list (one warp): the entries not
+// processed yet move to the front, the new ones follow, and the window constants are formed. last: no event follows,
+// so the last window ends at +inf and the last group may be short.
+__device__ __forceinline__ void conv_list_append(ConvList& l, const ConvEvent* sev, int cnt, bool last, int xo, int yo,
+                                                 int fx, int fy, int C, const SolveConst& sk, int lane) {
+    int n = l.n;
+    const int from = l.groups * CONV_GROUP;
+    float t = 0.0f, es = 0.0f, e = 0.0f;
+    int row = 0;
+    n -= from;  // at most CONV_GROUP entries are left over
+    if (lane < n) {
+        t = l.t[from + lane];
+        row = l.row[from + lane];
+        es = l.win[from + lane].es;
+        e = l.win[from + lane].e;
+    }
+    __syncwarp();
+    if (lane < n) {
+        l.t[lane] = t;
+        l.row[lane] = row;
+        l.win[lane].es = es;
+        l.win[lane].e = e;
+    }
+    for (int q0 = 0; q0 < cnt; q0 += 32) {
+        ConvEvent ev = {0.0f, 0.0f, 0.0f, 0};
+        bool rel = false;
+        if (q0 + lane < cnt) {
+            ev = sev[q0 + lane];
+            const int dx = (ev.xyc & 1023) - xo, dy = ((ev.xyc >> 10) & 1023) - yo;
+            const bool in = dx >= 0 && dx < fx && dy >= 0 && dy < fy;
+            row = in ? (dx * fy + dy) * C + ((ev.xyc >> 20) & 2047) : -1;
+            rel = in || ev.xyc < 0;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, rel);
+        if (rel) {
+            const int at = n + __popc(bal & lanemask_lt());
+            l.t[at] = ev.t;
+            l.row[at] = row;
+            l.win[at].es = ev.es;
+            l.win[at].e = ev.e;
+        }
+        n += __popc(bal);
+    }
+    __syncwarp();
+    for (int u = lane; u < n; u += 32) {
+        const float e_u = l.win[u].e;
+        const float e_next = u + 1 < n ? l.win[u + 1].e : BATS_INF;
+        const CrossWindow w = cross_window(0.0f, 0.0f, e_u, e_next, sk);
+        l.win[u].czz = w.czz;
+        l.win[u].zw = w.zw;
+        l.win[u].tcz = w.tcz;
+        l.win[u].czzl = w.czzl;
+        l.win[u].zl = w.zl;
+        l.win[u].tczl = w.tczl;
+    }
+    const int groups = last ? (n + CONV_GROUP - 1) / CONV_GROUP : max(0, n - 1) / CONV_GROUP;
+    // A short last group is filled up with events of weight and exponentials 0, which leave the state unchanged.
+    for (int u = n + lane; u < groups * CONV_GROUP; u += 32) {
+        l.row[u] = -1;
+        l.win[u] = CrossWindow{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    }
+    if (lane == 0) {
+        l.t[n] = BATS_INF;
+        l.n = n;
+        l.groups = groups;
+    }
+}
+
+// CTA per (tile of TX x TY positions, sample), thread = (position, output channel). The sample's events inside the
+// tile's receptive field are compacted into shared memory; CONV_SUB of them at a time, a warp per position builds the
+// position's own list of relevant events, which its C_out threads then run through in groups of CONV_GROUP, as the
+// fully-connected tile kernel runs through a stage: a branch-free pass with the screen of every event, and the exact
+// loop from the first event after which a crossing cannot be ruled out. A warp's lanes may belong to two positions:
+// they step through their own lists side by side.
+// What bounds it: instruction issue. 12 x 12 x 15 -> 5 x 5 x 40, batch 128: 1.78 -> 0.76 ms; before, every thread tested
+// every event of the tile for its own field and ran the screen one event at a time, lanes of two positions after one
+// another. CONV_SUB 32: 0.90 ms (more barriers).
+template <bool W_SMEM>
+__global__ void __launch_bounds__(1024)
+conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_count, long long ev_cap,
+                    const float* __restrict__ W, int X, int Y, int C, int fx, int fy, int C_out, int Xo, int Yo,
+                    int TX, int TY, int tiles_y, int k_post, SolveConst sk, int* __restrict__ n_spikes,
+                    float* __restrict__ a_out, float* __restrict__ x_out, float* __restrict__ t_out,
+                    float* __restrict__ z_out) {
     pdl_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ConvEvent* sev = reinterpret_cast<ConvEvent*>(smem_raw);
-    float2* szw = reinterpret_cast<float2*>(sev + CONV_CHUNK);  // each kept event's window constants
-    int* swarp = reinterpret_cast<int*>(szw + CONV_CHUNK);
-    float* sW = reinterpret_cast<float*>(swarp + 32);
+    __shared__ int swarp[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarps = (blockDim.x + 31) >> 5;
+    const int nwarps = blockDim.x >> 5;
+    const int P = TX * TY;
+    ConvList* lists = reinterpret_cast<ConvList*>(smem_raw);
+    ConvEvent* sev = reinterpret_cast<ConvEvent*>(lists + P);  // CONV_SUB + blockDim entries
+    float* sW = reinterpret_cast<float*>(sev + CONV_SUB + blockDim.x);
     const int s = blockIdx.y;
     const int tx0 = (blockIdx.x / tiles_y) * TX, ty0 = (blockIdx.x % tiles_y) * TY;
-    const int nw = C_out * fx * fy * C;
-    const float* Wsrc = W;
-    if (w_in_smem) {
-        for (int q = tid; q < nw; q += blockDim.x) sW[q] = W[q];
-        Wsrc = sW;
-    }
+    const int R = fx * fy * C, ldw = W_SMEM ? (R | 1) : R;  // odd: a row's channels lie in different banks
+    if (W_SMEM)
+        for (int co = warp; co < C_out; co += nwarps)
+            for (int q = lane; q < R; q += 32) sW[co * ldw + q] = W[co * R + q];
+    for (int p = tid; p < P; p += blockDim.x) lists[p].n = lists[p].groups = 0;
     const int co = tid % C_out, pl = tid / C_out;
     const int xo = tx0 + pl / TY, yo = ty0 + pl % TY;
-    const bool active = pl < TX * TY && xo < Xo && yo < Yo;
+    const bool active = pl < P && xo < Xo && yo < Yo;
     const int n_post = Xo * Yo * C_out;
     const int post = (xo * Yo + yo) * C_out + co;
     const long long obase = ((long long)s * n_post + (active ? post : 0)) * k_post;
-    float* ao = a_out + obase;
-    float* xo_ = x_out + obase;
-    float* to = t_out + obase;
-    float* zo = z_out + obase;
+    const ConvList& l = lists[active ? pl : 0];
+    const float* wrow = (W_SMEM ? sW : W) + (active ? co * ldw : 0);
+    auto weight = [&](int row) { return row >= 0 ? wrow[row] : 0.0f; };
     // Receptive field of the whole tile.
     const int rx0 = tx0, rx1 = min(X, tx0 + TX + fx - 1), ry0 = ty0, ry1 = min(Y, ty0 + TY + fy - 1);
 
-    float a = 0.0f, b = 0.0f, last_t = 0.0f;
-    bool has_prev = false;
+    float a = 0.0f, b = 0.0f;
     int n = 0;
     bool done = !active;
     const int E = ev_count[s];
     const Event* evs = ev + (long long)s * ev_cap;
-    for (int m0 = 0; m0 < E; m0 += CONV_CHUNK) {
-        // Stage the chunk's events that fall in the tile's receptive field, in time order.
-        __syncthreads();
-        int kept = 0;
-        for (int r0 = 0; r0 < CONV_CHUNK && m0 + r0 < E; r0 += blockDim.x) {
-            const int q = r0 + tid;
-            bool keep = false;
-            ConvEvent ce;
-            if (q < CONV_CHUNK && m0 + q < E) {
-                const Event e = evs[m0 + q];
-                const int j = e.j;
-                const int cc = j % C, xy = j / C, yy = xy % Y, xx = xy / Y;
-                // In the tile's receptive field, or relevant to every neuron (a non-finite exponential).
-                keep = (xx >= rx0 && xx < rx1 && yy >= ry0 && yy < ry1) || !(isfinite(e.es) && isfinite(e.e));
-                ce.t = e.t;
-                ce.es = e.es;
-                ce.e = e.e;
-                // bit 31: an exponential is not finite (the event is relevant to every neuron)
-                ce.xyc = xx | (yy << 10) | (cc << 20) | ((isfinite(e.es) && isfinite(e.e)) ? 0 : (int)0x80000000u);
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-            if (lane == 0) swarp[warp] = __popc(bal);
-            __syncthreads();
-            int off = kept;
-            int tot = 0;
-            for (int w = 0; w < nwarps; ++w) {
-                if (w < warp) off += swarp[w];
-                tot += swarp[w];
-            }
-            if (keep) {
-                const int pos = off + __popc(bal & lanemask_lt());
-                sev[pos] = ce;
-                szw[pos] = conv_window(ce.e, sk);  // the window that ends at this event, once per CTA
-            }
-            __syncthreads();
-            kept += tot;
+    int kept = 0;  // events in sev
+    for (int m0 = 0;; m0 += blockDim.x) {
+        // Keep the events of this round that fall in the tile's receptive field, in time order.
+        const bool last_round = m0 + (int)blockDim.x >= E;
+        bool keep = false;
+        ConvEvent ce = {0.0f, 0.0f, 0.0f, 0};
+        if (m0 + tid < E) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(evs + m0 + tid));  // (t, j, es, e)
+            const int j = __float_as_int(v.y);
+            const int cc = j % C, xy = j / C, yy = xy % Y, xx = xy / Y;
+            const bool finite = isfinite(v.z) && isfinite(v.w);
+            // In the tile's receptive field, or relevant to every neuron (a non-finite exponential).
+            keep = (xx >= rx0 && xx < rx1 && yy >= ry0 && yy < ry1) || !finite;
+            ce = {v.x, v.z, v.w, xx | (yy << 10) | (cc << 20) | (finite ? 0 : (int)0x80000000u)};
         }
+        const unsigned bal = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) swarp[warp] = __popc(bal);
         __syncthreads();
-        if (done) continue;
-        for (int m = 0; m < kept && !done; ++m) {
-            const ConvEvent e = sev[m];
-            const int dx = (e.xyc & 1023) - xo, dy = ((e.xyc >> 10) & 1023) - yo;
-            const bool in_field = dx >= 0 && dx < fx && dy >= 0 && dy < fy;
-            if (!in_field && e.xyc >= 0) continue;  // weight 0 times a finite value
-            if (has_prev) {
-                done = solve_crossings_conv_at(a, b, last_t, e.t, szw[m], sk, n, k_post, ao, xo_, to, zo);
-                if (done) break;
-            }
-            const float w = in_field ? Wsrc[((co * fx + dx) * fy + dy) * C + ((e.xyc >> 20) & 2047)] : 0.0f;
-            a += w * e.es;
-            b += w * e.e;
-            last_t = e.t;
-            has_prev = true;
+        int off = kept, tot = 0;
+        for (int w = 0; w < nwarps; ++w) {
+            off += w < warp ? swarp[w] : 0;
+            tot += swarp[w];
         }
+        if (keep) sev[off + __popc(bal & lanemask_lt())] = ce;
+        kept += tot;
+        __syncthreads();
+        int head = 0;
+        while (kept - head >= CONV_SUB || (last_round && head < kept) || (last_round && kept == 0)) {
+            const int cnt = min(CONV_SUB, kept - head);
+            const bool last = last_round && head + cnt == kept;
+            for (int p = warp; p < P; p += nwarps)
+                conv_list_append(lists[p], sev + head, cnt, last, tx0 + p / TY, ty0 + p % TY, fx, fy, C, sk, lane);
+            __syncthreads();
+            if (!done) {
+                const int groups = l.groups, total = l.n;
+                for (int g = 0; g < groups && !done; ++g) {
+                    const CrossWindow* win = l.win + g * CONV_GROUP;
+                    const int* row = l.row + g * CONV_GROUP;
+                    const float* tt = l.t + g * CONV_GROUP;
+                    const int cnt_g = min(CONV_GROUP, total - g * CONV_GROUP);
+                    float aa = a, bb = b;
+                    unsigned cand = 0u;
+#pragma unroll
+                    for (int u = 0; u < CONV_GROUP; ++u) {
+                        const CrossWindow c = win[u];
+                        const float w = weight(row[u]);
+                        aa = fmaf(w, c.es, aa);
+                        bb = fmaf(w, c.e, bb);
+                        cand |= cross_bit<true>(aa, bb, c, sk, 1u << u);
+                    }
+                    cand &= (2u << (cnt_g - 1)) - 1u;  // not the events that fill up the last group
+                    if (cand) {
+                        const int first = __ffs(cand) - 1;
+                        aa = a;
+                        bb = b;
+                        for (int u = 0; u <= first; ++u) {
+                            const float w = weight(row[u]);
+                            aa = fmaf(w, win[u].es, aa);
+                            bb = fmaf(w, win[u].e, bb);
+                        }
+                        bool cross = true;
+                        for (int u = first;;) {
+                            if (cross && solve_candidate<true>(aa, bb, tt[u], tt[u + 1], win[u], sk, n, k_post, obase,
+                                                               a_out, x_out, t_out, z_out)) {
+                                done = true;
+                                break;
+                            }
+                            if (++u >= cnt_g) break;
+                            const CrossWindow c = win[u];
+                            const float w = weight(row[u]);
+                            aa = fmaf(w, c.es, aa);
+                            bb = fmaf(w, c.e, bb);
+                            cross = may_cross<true>(aa, bb, c, sk);
+                        }
+                    }
+                    a = aa;
+                    b = bb;
+                }
+            }
+            head += cnt;
+            if (__syncthreads_and(done) || last) {  // every buffer full, or no event left
+                kept = head = 0;
+                m0 = E;
+                break;
+            }
+        }
+        if (m0 >= E || last_round) break;
+        // The events not in a list yet move to the front (fewer than CONV_SUB).
+        ConvEvent mv;
+        const int rest = kept - head;
+        if (tid < rest) mv = sev[head + tid];
+        __syncthreads();
+        if (tid < rest) sev[tid] = mv;
+        kept = rest;
     }
-    if (active) {
-        if (has_prev && !done)
-            solve_crossings<true>(a, b, last_t, BATS_INF, 0.0f, BATS_INF, sk, n, k_post, ao, xo_, to, zo);
-        n_spikes[(long long)s * n_post + post] = n;
-        for (int k = n; k < k_post; ++k) {
-            to[k] = BATS_INF;
-            zo[k] = BATS_INF;
+    if (active) n_spikes[(long long)s * n_post + post] = n;
+    // +inf past each neuron's spikes: the lanes run along the warp's 32 rows of k_post slots, most of which lie next to
+    // one another (a store per lane and slot of its own row would touch 32 lines).
+    const int free_from = active ? n : k_post;
+    int r = lane / k_post, k = lane - r * k_post;  // the warp's row and slot of this lane
+    const int dr = 32 / k_post, dk = 32 - dr * k_post;
+    for (int q = 0; q < k_post; ++q) {
+        const int nr = __shfl_sync(0xffffffffu, free_from, r & 31);
+        const long long pr = (long long)s * n_post + __shfl_sync(0xffffffffu, post, r & 31);
+        if (k >= nr) {
+            t_out[pr * k_post + k] = BATS_INF;
+            z_out[pr * k_post + k] = BATS_INF;
+        }
+        r += dr;
+        k += dk;
+        if (k >= k_post) {
+            k -= k_post;
+            ++r;
         }
     }
 }
@@ -520,12 +662,33 @@ __global__ void pool_backward_kernel(const float* __restrict__ errors, const int
 // ---------------------------------------------------------------------------------------------
 // C-ABI
 
-static void conv_tile(int C_out, int& TX, int& TY) {
-    int P = 512 / C_out;
-    if (P < 1) P = 1;
+// Positions per CTA: as many as give at most `threads` threads (at least one position; a layer of more output channels
+// runs one position with C_out threads), in a tile close to a square (the smallest receptive field).
+static void conv_tile(int C_out, int threads, int& TX, int& TY) {
+    const int P = std::max(1, std::min(bats::CONV_POSITIONS, threads / C_out));
     TX = 1;
     while ((TX + 1) * (TX + 1) <= P) ++TX;
     TY = P / TX;
+}
+
+// Larger tiles read the sample's events fewer times and share more of each receptive field; smaller ones give more CTAs
+// and shorter waits at the barriers. 512 threads pay only where a sample can carry many events (12 x 12 x 15 x 40 slots,
+// 768 CTAs: 0.76 ms, 256 threads 0.87; 28 x 28 x 1 slots: 0.099 ms, 256 threads 0.087) and the grid still fills two
+// CTAs on each of the 152 SMs; below that the tile is halved (42 CTAs of 512 threads: 0.142 ms, 168 of 128: 0.095).
+static void conv_plan(int batch, int Xo, int Yo, int C_out, long long ev_cap, int& TX, int& TY) {
+    for (int threads = ev_cap >= 8192 ? 512 : 256;; threads /= 2) {
+        conv_tile(C_out, threads, TX, TY);
+        const long long ctas = (long long)((Xo + TX - 1) / TX) * ((Yo + TY - 1) / TY) * batch;
+        if (ctas >= 2 * 152 || threads <= 128) return;
+    }
+}
+
+template <bool W_SMEM, typename... Args>
+static cudaError_t launch_conv_forward(dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+    const cudaError_t e =
+        (cudaError_t)bats::max_dynamic_smem_set((const void*)bats::conv_forward_kernel<W_SMEM>, (int)smem);
+    if (e != cudaSuccess) return e;
+    return bats::launch(bats::conv_forward_kernel<W_SMEM>, grid, threads, smem, stream, args...);
 }
 
 extern "C" int bats_conv_forward(const void* events, const int* ev_count, long long ev_cap, const float* weights,
@@ -540,19 +703,22 @@ extern "C" int bats_conv_forward(const void* events, const int* ev_count, long l
                  "conv_forward: null pointer");
     const int Xo = X - fx + 1, Yo = Y - fy + 1;
     int TX, TY;
-    conv_tile(C_out, TX, TY);
+    conv_plan(batch, Xo, Yo, C_out, ev_cap, TX, TY);
     const int threads = ((TX * TY * C_out + 31) / 32) * 32;
     const int tiles_x = (Xo + TX - 1) / TX, tiles_y = (Yo + TY - 1) / TY;
-    const size_t nw = (size_t)C_out * fx * fy * C;
-    const size_t base_smem = bats::CONV_CHUNK * (sizeof(bats::ConvEvent) + sizeof(float2)) + 32 * sizeof(int);
-    const int w_in_smem = (base_smem + nw * sizeof(float)) <= 200 * 1024;
-    const size_t smem = base_smem + (w_in_smem ? nw * sizeof(float) : 0);
-    BATS_CUDA((cudaError_t)bats::max_dynamic_smem_set((const void*)bats::conv_forward_kernel, (int)smem));
+    const size_t base_smem = TX * TY * sizeof(bats::ConvList) + (bats::CONV_SUB + threads) * sizeof(bats::ConvEvent);
+    const size_t w_smem = (size_t)C_out * ((fx * fy * C) | 1) * sizeof(float);
+    const bool w_in_smem = base_smem + w_smem <= 200 * 1024;
+    const size_t smem = base_smem + (w_in_smem ? w_smem : 0);
     dim3 grid(tiles_x * tiles_y, batch);
-    BATS_CUDA(bats::launch(bats::conv_forward_kernel, grid, threads, smem, stream,
-        reinterpret_cast<const bats::Event*>(events), ev_count, ev_cap, weights, X, Y, C, fx, fy, C_out, Xo, Yo, TX, TY,
-        tiles_y, k_post, bats::make_solve_const(c, delta_theta_tau, tau, max_simulation), w_in_smem, n_spikes, a, x,
-        times, post_exp_tau));
+    const bats::SolveConst sk = bats::make_solve_const(c, delta_theta_tau, tau, max_simulation);
+    const bats::Event* evs = reinterpret_cast<const bats::Event*>(events);
+    BATS_CUDA(w_in_smem ? launch_conv_forward<true>(grid, threads, smem, stream, evs, ev_count, ev_cap, weights, X, Y,
+                                                    C, fx, fy, C_out, Xo, Yo, TX, TY, tiles_y, k_post, sk, n_spikes, a,
+                                                    x, times, post_exp_tau)
+                        : launch_conv_forward<false>(grid, threads, smem, stream, evs, ev_count, ev_cap, weights, X, Y,
+                                                     C, fx, fy, C_out, Xo, Yo, TX, TY, tiles_y, k_post, sk, n_spikes, a,
+                                                     x, times, post_exp_tau));
     BATS_CUDA(cudaGetLastError());
     return BATS_OK;
 }
