@@ -433,6 +433,18 @@ struct PostCursor {
     __device__ __forceinline__ bool valid() const { return p < n; }
 };
 
+// Post-spike position of a post neuron for a pre spike at time t: p = number of valid post spikes
+// with t_k <= t (the first k with t_k > t), by binary search over the neuron's leading valid spikes.
+__device__ __forceinline__ int post_position(const float* __restrict__ tk, int n, float t) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (tk[mid] <= t) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
 // Sum over the 32 lanes of v[e] for e = 0..N-1 (N = 32 or 16), leaving lane l with the total for
 // e = l mod N. N - 1 shuffles (N for N = 16: the two half-warps are added last) instead of N separate
 // butterflies; the summation order is fixed.

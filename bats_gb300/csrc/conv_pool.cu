@@ -344,8 +344,9 @@ __global__ void conv_backward_kernel(const Event* __restrict__ ev, const int* __
 
 // Conv backward on a cluster of CONV_BWD_CLUSTER CTAs per sample (thread-block cluster, distributed
 // shared memory). Thread = filter tap (co, dx, dy); the sample's events are dealt to the cluster's CTAs in
-// groups of 32 (group g to CTA rank g % CONV_BWD_CLUSTER), so that eight times as many CTAs hide the
-// latency of the post-spike lookups. Every CTA accumulates its events' gradient terms in a shared-memory
+// groups of CONV_BWD_EVENTS (group g to CTA rank g % CONV_BWD_CLUSTER), so that eight times as many CTAs hide the
+// latency of the post-spike lookups, which bounds the kernel; small groups deal the 150 events of an MNIST-shaped
+// sample evenly (groups of 32 left three of the eight CTAs idle). Every CTA accumulates its events' gradient terms in a shared-memory
 // copy of the per-sample filter gradient (taps x C), in event order; at the end each CTA sums one slice of
 // the gradient over the cluster's copies in rank order (deterministic) and writes it. The pre-spike errors
 // of a group of events are reduced over the taps inside the CTA that owns the group. Four events are
@@ -353,6 +354,7 @@ __global__ void conv_backward_kernel(const Event* __restrict__ ev, const int* __
 // entries) are in flight together.
 constexpr int CONV_BWD_CLUSTER = 8;
 constexpr int CONV_BWD_ILP = 4;
+constexpr int CONV_BWD_EVENTS = 8;
 
 __global__ void __launch_bounds__(1024)
 conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_slot,
@@ -365,8 +367,8 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) float Gs[];  // taps * C
-    __shared__ Event sev[32];
-    __shared__ float sred[32][33];
+    __shared__ Event sev[CONV_BWD_EVENTS];
+    __shared__ float sred[CONV_BWD_EVENTS][33];
     const unsigned rank = cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nwarps = blockDim.x >> 5;
@@ -380,9 +382,9 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
     for (int s = (int)blockIdx.y * group; s < s_end; ++s) {
     const int E = ev_count[s];
     const Event* evs = ev + (long long)s * ev_cap;
-    for (int g = (int)rank; g * 32 < E; g += CONV_BWD_CLUSTER) {
-        const int m0 = g * 32;
-        const int cnt = min(32, E - m0);
+    for (int g = (int)rank; g * CONV_BWD_EVENTS < E; g += CONV_BWD_CLUSTER) {
+        const int m0 = g * CONV_BWD_EVENTS;
+        const int cnt = min(CONV_BWD_EVENTS, E - m0);
         if (tid < cnt) sev[tid] = evs[m0 + tid];
         __syncthreads();
         for (int q0 = 0; q0 < cnt; q0 += CONV_BWD_ILP) {
@@ -463,132 +465,272 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
 
 // Conv backward over events grouped by input position (the bucketed copy of the sort with
 // bucket_width = C: one bucket per (x, y), time order inside), on a cluster of CONV_BWD_CLUSTER CTAs per
-// sample (position groups dealt to the ranks). Thread = filter tap (co, dx, dy). Within a position group
-// every tap sees one and the same post neuron (x - dx, y - dy, co), so its spike data is set up once per
-// group and followed by a forward-only cursor over the group's time-ordered events, instead of a search
-// per (event, tap). A spike's slot (neuron j, k-th spike of j) follows from the order of appearance of j
-// in the group. The per-sample gradient copies are combined over the cluster as in
-// conv_backward_cluster_kernel; pre errors are reduced over the taps in the CTA that owns the group.
+// sample (position groups dealt to the ranks). Within a position group every filter tap sees one and the same post
+// neuron (x - dx, y - dy, co). A warp owns 32 consecutive taps ((dx fy + dy) C_out + co); its lanes are the group's
+// events, 32 at a time, and it goes through those of its taps whose post neuron lies inside the output and spiked: the
+// neuron's spike times and table rows lie on the lanes (K <= 32; loaded one neuron ahead), every lane finds its event's
+// place among them by a binary search over shuffles, adds its gradient term to the tap's row of the CTA's gradient copy
+// in shared memory ([tap][channel]: lanes of one channel are first added up along precomputed links, so that one lane
+// per channel updates its entry) and its pre-error term to a register.
+// The rank's events are taken in batches of whole positions (at most `batch_ev` events; a larger position in segments):
+// staged once for all warps with their channel decoded and their slots ranked (slot k of neuron j: the k-th event of j in
+// the group); the warps' pre-error terms of the batch meet in sred and are added at its end. Three barriers per batch.
+// The per-sample gradient copies are combined over the cluster as in conv_backward_cluster_kernel.
+// What bounds it: instruction issue (64 %). 12 x 12 x 15 -> 5 x 5 x 40, batch 128: 0.94 ms, 571 M warp instructions. A
+// thread per tap with a cursor over the post spikes took 2.65 ms (1.2 G warp instructions: with about ten post spikes
+// and twenty events per tap and position, some lane's cursor moved at every event, and half of the lanes lay outside the
+// output); the same with the output channels on the lanes and these batches 1.71 ms.
+struct ConvBwdShape {
+    int Y, C, fx, fy, C_out, Xo, Yo, k_pre, k_post, n_pos;
+};
+
+constexpr int CONV_BWD_POS = 255;  // positions of a layer at most (the buckets of the sort)
+
+// ROWS: K <= 32, a neuron's rows fit the lanes; TOP: the largest power of two <= K (at most 16), the search's first step.
+template <bool ROWS, int TOP, bool PRE, bool W_SMEM>
 __global__ void __launch_bounds__(1024)
-conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restrict__ boff, int n_pos,
-                             long long ev_cap, const float* __restrict__ W, int Y, int C, int fx, int fy, int C_out,
-                             int Xo, int Yo, int k_pre, const float* __restrict__ post_t,
-                             const float2* __restrict__ tab, const int* __restrict__ nvalid, int k_post,
-                             float tau_s, float tau, long long pre_slots, float* __restrict__ grad,
-                             float* __restrict__ pre_err, int batch, int group, int w_in_smem) {
+conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restrict__ boff, long long ev_cap,
+                             const float* __restrict__ W, ConvBwdShape sh, const float* __restrict__ post_t,
+                             const float2* __restrict__ tab, const int* __restrict__ nvalid, float tau_s, float tau,
+                             long long pre_slots, float* __restrict__ grad, float* __restrict__ pre_err, int batch,
+                             int group, int batch_ev, int step) {
     pdl_prologue();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ __align__(16) float Gs[];  // taps * C, then C spike counters
-    __shared__ Event sev[32];
-    __shared__ float sred[32][33];
-    __shared__ int sslot[32];
-    __shared__ int scc[32];
+    extern __shared__ __align__(16) float4 cb_smem[];
+    __shared__ int s_beg[CONV_BWD_POS], s_len[CONV_BWD_POS];
     const float inv_tau_s = 1.0f / tau_s, inv_tau = 1.0f / tau;  // the error terms' factors, as reciprocals
-    const unsigned rank = cluster.block_rank();
+    const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarps = blockDim.x >> 5;
-    const int taps = C_out * fx * fy;
+    const int nwarps = blockDim.x >> 5, red_ld = nwarps | 1;
+    const int C = sh.C, taps = sh.C_out * sh.fx * sh.fy, K = sh.k_post;
     const int total = taps * C;
-    int* kcount = reinterpret_cast<int*>(Gs + total);
-    const int n_post = Xo * Yo * C_out;
+    const int n_post = sh.Xo * sh.Yo * sh.C_out;
+    float4* sE = cb_smem;                                      // staged events: (t, es, e, channel)
+    float* sred = reinterpret_cast<float*>(sE + batch_ev);     // [event][warp]
+    int* sslot = reinterpret_cast<int*>(sred + batch_ev * red_ld);
+    int* kcount = sslot + batch_ev;                            // per channel: a split position's earlier events
+    float* Gs = reinterpret_cast<float*>(kcount + C);          // [tap][channel]
+    const bool has_tap = tid < taps;
+    const int co = tid % sh.C_out, dxy = tid / sh.C_out;
+    const int dx = dxy / sh.fy, dy = dxy % sh.fy;
     for (int q = tid; q < total; q += blockDim.x) Gs[q] = 0.0f;
-    // The filters, for the pre-spike error terms: in shared memory after the counters when they fit (a
-    // thread's weight reads are C floats apart, one cache sector per lane from global memory).
+    const int wbase = ((co * sh.fx + dx) * sh.fy + dy) * C;  // the tap's place in the filters
     const float* Wk = W;
-    if (w_in_smem) {
-        float* sWf = reinterpret_cast<float*>(kcount + C);
-        for (int q = tid; q < total; q += blockDim.x) sWf[q] = W[q];
+    if (W_SMEM) {
+        float* sWf = Gs + total;
+        if (has_tap)
+            for (int c = 0; c < C; ++c) sWf[tid * C + c] = W[wbase + c];
         Wk = sWf;
     }
-    // At most one tap per thread here (taps <= blockDim checked by the launcher).
-    const int tp = tid;
-    const bool has_tap = tp < taps;
-    const int co = has_tap ? tp / (fx * fy) : 0, dx = has_tap ? (tp / fy) % fx : 0, dy = has_tap ? tp % fy : 0;
-    __syncthreads();
+    // The rank's positions in a scattered order (step is coprime to n_pos), so that every batch holds positions from all
+    // over the input: at the border only some taps reach an output, and their warps would wait for the others.
+    auto position = [&](int i) { return (int)((unsigned)(rank + i * ranks) * (unsigned)step % (unsigned)sh.n_pos); };
+    const int n_mine = rank < sh.n_pos ? (sh.n_pos - 1 - rank) / ranks + 1 : 0;
     // The cluster's samples (one with group == 1: the per-sample gradient), accumulated in order.
     const int s_end = min(batch, ((int)blockIdx.y + 1) * group);
     for (int s = (int)blockIdx.y * group; s < s_end; ++s) {
-    const int* bo = boff + (long long)s * (n_pos + 1);
-    const Event* evs = ev_b + (long long)s * ev_cap;
-    for (int g = (int)rank; g < n_pos; g += CONV_BWD_CLUSTER) {
-        const int beg = bo[g], end = bo[g + 1];
-        if (beg >= end) continue;  // uniform over the CTA
-        const int xx = g / Y, yy = g % Y;
-        const int xo = xx - dx, yo = yy - dy;
-        const bool in = has_tap && xo >= 0 && yo >= 0 && xo < Xo && yo < Yo;
-        PostCursor cur;
-        const long long pn = in ? (long long)s * n_post + (xo * Yo + yo) * C_out + co : 0;
-        cur.init(post_t + pn * k_post, tab + pn * (k_post + 1), in ? nvalid[pn] : 0);
-        // Two barriers per chunk: after warp 0 stages it (every thread reads it), and after the error terms are in
-        // sred (every thread is done with the chunk's records; the chunk's events then sum the terms). The next
-        // chunk's first barrier orders those sums' reads of sred and sslot before anything overwrites them (warp 0
-        // sums, then stages; the other warps write sred only after that barrier).
-        for (int m0 = beg; m0 < end; m0 += 32) {
-            const int cnt = min(32, end - m0);
-            if (warp == 0) {
-                if (m0 == beg) {  // the position's spike counters per channel: warp 0's alone
-                    for (int q = lane; q < C; q += 32) kcount[q] = 0;
-                    __syncwarp();
-                }
-                // Stage the chunk; the spikes' slots: j * k_pre + the order of appearance of j in the group (all
-                // events of a position share x and y, so j is fixed by the channel: earlier chunks' counts plus
-                // the rank among this chunk's events of the same channel).
-                Event e;
-                int c = -1;
-                if (lane < cnt) {
-                    e = evs[m0 + lane];
-                    c = e.j % C;
-                    sev[lane] = e;
-                    scc[lane] = c;
-                }
-                const unsigned peers = __match_any_sync(0xffffffffu, c);
-                const int rank = __popc(peers & lanemask_lt());
-                int base = 0;
-                if (lane < cnt) base = kcount[c];
-                __syncwarp();
-                if (lane < cnt) {
-                    sslot[lane] = e.j * k_pre + base + rank;
-                    if (rank == __popc(peers) - 1) kcount[c] = base + __popc(peers);
-                }
+        const int* bo = boff + (long long)s * (sh.n_pos + 1);
+        const Event* evs = ev_b + (long long)s * ev_cap;
+        const long long pn_s = (long long)s * n_post;
+        const float* t_lane = post_t + pn_s * K + lane;
+        const float2* tab_lane = tab + pn_s * (K + 1) + lane;
+        __syncthreads();
+        for (int i = tid; i < n_mine; i += blockDim.x) {
+            const int g = position(i);
+            s_beg[i] = bo[g];
+            s_len[i] = bo[g + 1] - bo[g];
+        }
+        __syncthreads();
+        // i0, off0: the first position of the batch and its first event not taken yet (uniform over the CTA).
+        for (int i0 = 0, off0 = 0; i0 < n_mine;) {
+            int i1 = i0, cnt = 0;  // positions i0 .. i1 - 1 whole, or one segment of position i0
+            const bool split = off0 > 0 || s_len[i0] > batch_ev;
+            if (split) {
+                cnt = min(batch_ev, s_len[i0] - off0);
+                i1 = i0 + 1;
+            } else {
+                while (i1 < n_mine && cnt + s_len[i1] <= batch_ev) cnt += s_len[i1++];
             }
-            __syncthreads();
-            float term[32];
-#pragma unroll
-            for (int q = 0; q < 32; ++q) {
-                term[q] = 0.0f;
-                if (q < cnt && in) {
-                    const Event e = sev[q];
-                    cur.advance_past(e.t);
-                    if (cur.valid()) {
-                        const int cc = scc[q];
-                        Gs[tp * C + cc] += fmaf(e.es, cur.AB.x, -(e.e * cur.AB.y));
-                        if (pre_err)
-                            term[q] = Wk[tp * C + cc] * (cur.AB.x * e.es * inv_tau_s - cur.AB.y * e.e * inv_tau);
+            if (cnt > 0) {
+                if (split && off0 == 0)
+                    for (int q = tid; q < C; q += blockDim.x) kcount[q] = 0;
+                // Stage the batch: a warp per position (a split one: 32 events per warp).
+                for (int w = warp; w < (split ? (cnt + 31) / 32 : i1 - i0); w += nwarps) {
+                    int at = 0, len = cnt, src = s_beg[i0] + off0;
+                    if (split) {
+                        at = w * 32;
+                        len = min(32, cnt - at);
+                        src += at;
+                    } else {
+                        for (int i = i0; i < i0 + w; ++i) at += s_len[i];
+                        len = s_len[i0 + w];
+                        src = s_beg[i0 + w];
+                    }
+                    for (int q = lane; q < len; q += 32) {
+                        const float4 e = __ldg(reinterpret_cast<const float4*>(evs + src + q));  // (t, j, es, e)
+                        const int j = __float_as_int(e.y);
+                        sE[at + q] = make_float4(e.x, e.z, e.w, __int_as_float(j % C));
+                        sslot[at + q] = j * sh.k_pre;
+                    }
+                    if (PRE && !split) {
+                        __syncwarp();
+                        for (int q = lane; q < len; q += 32) {
+                            const int c = __float_as_int(sE[at + q].w);
+                            int earlier = 0;
+                            for (int r = 0; r < q; ++r) earlier += __float_as_int(sE[at + r].w) == c ? 1 : 0;
+                            sslot[at + q] += earlier;
+                        }
                     }
                 }
+                __syncthreads();
+                if (PRE && split) {
+                    for (int q = tid; q < cnt; q += blockDim.x) {
+                        const int c = __float_as_int(sE[q].w);
+                        int earlier = kcount[c];
+                        for (int r = 0; r < q; ++r) earlier += __float_as_int(sE[r].w) == c ? 1 : 0;
+                        sslot[q] += earlier;
+                    }
+                    __syncthreads();
+                    for (int c = tid; c < C; c += blockDim.x) {
+                        int more = 0;
+                        for (int r = 0; r < cnt; ++r) more += __float_as_int(sE[r].w) == c ? 1 : 0;
+                        kcount[c] += more;
+                    }
+                }
+                // Every warp through the batch's positions.
+                int at = 0;
+                for (int i = i0; i < i1; ++i) {
+                    const int len = split ? cnt : s_len[i];
+                    if (len == 0) continue;
+                    // Lane: one of the warp's taps, its post neuron (within the sample) and that neuron's spike count.
+                    const int g = position(i);
+                    const int xo = g / sh.Y - dx, yo = g % sh.Y - dy;
+                    const bool in = has_tap && xo >= 0 && yo >= 0 && xo < sh.Xo && yo < sh.Yo;
+                    const int pn_l = in ? (xo * sh.Yo + yo) * sh.C_out + co : 0;
+                    const int n_l = in ? __ldg(nvalid + pn_s + pn_l) : 0;
+                    const unsigned spiking = __ballot_sync(0xffffffffu, n_l > 0);
+                    if (!spiking) {  // no spike under the warp's taps
+                        if (PRE)
+                            for (int q = lane; q < len; q += 32) sred[(at + q) * red_ld + warp] = 0.0f;
+                        at += len;
+                        continue;
+                    }
+                    for (int q0 = 0; q0 < len; q0 += 32) {
+                        const bool on = q0 + lane < len;
+                        const float4 e = on ? sE[at + q0 + lane] : make_float4(-BATS_INF, 0.0f, 0.0f, __int_as_float(-1));
+                        const int c = __float_as_int(e.w);
+                        const float f1 = e.y * inv_tau_s, f2 = e.z * inv_tau;
+                        // Lanes of the same channel, as links to the next lane, the 2nd, 4th, 8th and 16th after it
+                        // (32: none); head: the first lane of its channel.
+                        const unsigned peers = __match_any_sync(0xffffffffu, c);
+                        const unsigned after = peers & ~(2u * lanemask_lt() + 1u);
+                        const bool head = on && (peers & lanemask_lt()) == 0u;
+                        int link[5];
+                        link[0] = after ? __ffs(after) - 1 : 32;
+#pragma unroll
+                        for (int m = 1; m < 5; ++m) {
+                            const int far = __shfl_sync(0xffffffffu, link[m - 1], link[m - 1] & 31);
+                            link[m] = link[m - 1] < 32 ? far : 32;
+                        }
+                        const int longest = (int)__reduce_max_sync(0xffffffffu, on ? (unsigned)__popc(peers) : 0u);
+                        float* g_lane = Gs + warp * 32 * C + (on ? c : 0);       // + tap lane * C
+                        const float* w_lane = Wk + (W_SMEM ? warp * 32 * C : 0) + (on ? c : 0);
+                        float acc = 0.0f;
+                        // Rows of the neuron of tap lane b: K spike times and table entries on the lanes, +inf and 0
+                        // past its spikes.
+                        float t_row, a_row, b_row;
+                        int n_row, pn_row;
+                        auto load = [&](int b) {
+                            n_row = __shfl_sync(0xffffffffu, n_l, b);
+                            pn_row = __shfl_sync(0xffffffffu, pn_l, b);
+                            t_row = BATS_INF;
+                            a_row = b_row = 0.0f;
+                            if (ROWS && lane < n_row) {
+                                t_row = __ldg(t_lane + pn_row * K);
+                                const float2 ab = __ldg(tab_lane + pn_row * (K + 1));
+                                a_row = ab.x;
+                                b_row = ab.y;
+                            }
+                        };
+                        unsigned todo = spiking;
+                        load(__ffs(todo) - 1);
+                        while (todo) {
+                            const int b = __ffs(todo) - 1;
+                            todo &= todo - 1u;
+                            const float t_cur = t_row, a_cur = a_row, b_cur = b_row;
+                            const int n = n_row, pn = pn_row;
+                            if (todo) load(__ffs(todo) - 1);
+                            // The event's place among the spikes: p = #{k : t_k <= t}.
+                            float A, B;
+                            bool valid;
+                            if (ROWS) {
+                                int last = -1;  // p - 1
+#pragma unroll
+                                for (int step = TOP; step > 0; step >>= 1) {
+                                    const float tk = __shfl_sync(0xffffffffu, t_cur, last + step);
+                                    if (tk <= e.x) last += step;
+                                }
+                                if (TOP == 16 && K == 32) {  // the 32nd spike
+                                    const float t31 = __shfl_sync(0xffffffffu, t_cur, 31);
+                                    last += last == 30 && t31 <= e.x ? 1 : 0;
+                                }
+                                A = __shfl_sync(0xffffffffu, a_cur, last + 1);
+                                B = __shfl_sync(0xffffffffu, b_cur, last + 1);
+                                valid = on && last + 1 < n;
+                            } else {
+                                const long long r = pn_s + pn;
+                                const int p = post_position(post_t + r * K, n, e.x);
+                                const float2 ab = p < n ? __ldg(tab + r * (K + 1) + p) : make_float2(0.0f, 0.0f);
+                                A = ab.x;
+                                B = ab.y;
+                                valid = on && p < n;
+                            }
+                            float v = valid ? fmaf(e.y, A, -(e.z * B)) : 0.0f;
+                            if (PRE) {
+                                const float w = w_lane[W_SMEM ? b * C : __shfl_sync(0xffffffffu, wbase, b)];
+                                const float term = A * f1 - B * f2;
+                                if (valid) acc = fmaf(w, term, acc);
+                            }
+                            // The channel's terms meet on its first lane.
+#pragma unroll
+                            for (int m = 0; m < 5; ++m) {
+                                if (longest <= (1 << m)) break;
+                                const float vn = __shfl_sync(0xffffffffu, v, link[m] & 31);
+                                if (link[m] < 32) v += vn;
+                            }
+                            if (head) g_lane[b * C] += v;
+                        }
+                        if (PRE && on) sred[(at + q0 + lane) * red_ld + warp] = acc;
+                    }
+                    at += len;
+                }
+                __syncthreads();
+                if (PRE)
+                    for (int q = tid; q < cnt; q += blockDim.x) {
+                        float acc = 0.0f;
+                        for (int w = 0; w < nwarps; ++w) acc += sred[q * red_ld + w];
+                        pre_err[(long long)s * pre_slots + sslot[q]] = acc;
+                    }
+                __syncthreads();  // the next batch's staging overwrites sE and sslot
             }
-            if (pre_err) {
-                // The chunk's 32 error terms summed over the warp at once (lane q: event q), then over the warps.
-                const float v = warp_transpose_reduce<32>(term);
-                sred[lane][warp] = v;
-            }
-            __syncthreads();  // every thread is done with the chunk's records (warp 0 may restage them next)
-            if (pre_err && tid < cnt) {
-                float acc = 0.0f;
-                for (int w = 0; w < nwarps; ++w) acc += sred[tid][w];
-                pre_err[(long long)s * pre_slots + sslot[tid]] = acc;
+            if (split && off0 + cnt < s_len[i0]) {
+                off0 += cnt;
+            } else {
+                i0 = i1;
+                off0 = 0;
             }
         }
     }
-    }
     cluster.sync();
-    const int per = (total + CONV_BWD_CLUSTER - 1) / CONV_BWD_CLUSTER;
-    const int q_end = min(total, ((int)rank + 1) * per);
-    for (int q = (int)rank * per + tid; q < q_end; q += blockDim.x) {
+    const int per = (total + ranks - 1) / ranks;
+    const int q_end = min(total, (rank + 1) * per);
+    for (int q = rank * per + tid; q < q_end; q += blockDim.x) {
         float acc = 0.0f;
-        for (int r = 0; r < CONV_BWD_CLUSTER; ++r) acc += cluster.map_shared_rank(Gs, r)[q];
-        grad[(long long)blockIdx.y * total + q] = acc;
+        for (int r = 0; r < ranks; ++r) acc += cluster.map_shared_rank(Gs, r)[q];
+        const int tp = q / C, c = q - tp * C;
+        const int oc = tp % sh.C_out, od = tp / sh.C_out;
+        grad[(long long)blockIdx.y * total + ((long long)oc * sh.fx * sh.fy + od) * C + c] = acc;
     }
     cluster.sync();
 }
@@ -773,6 +915,88 @@ extern "C" int bats_conv_backward(const void* events, const int* ev_slot, const 
     return BATS_OK;
 }
 
+// Shared memory of conv_backward_grouped_kernel: the gradient copy always, the filters where they fit beside it, and the
+// largest batch of events that the rest holds (at least 32).
+static size_t conv_grouped_smem(long long taps, int C, int batch_ev, bool w) {
+    const size_t warps = (size_t)(taps + 31) / 32;
+    return (size_t)batch_ev * (sizeof(float4) + sizeof(float) * (warps | 1) + sizeof(int)) + (size_t)C * sizeof(int) +
+           (size_t)taps * C * sizeof(float) * (w ? 2 : 1);
+}
+
+template <bool PRE, bool W_SMEM>
+static auto* conv_grouped_kernel(int k_post) {
+    return k_post > 32    ? bats::conv_backward_grouped_kernel<false, 16, PRE, W_SMEM>
+           : k_post >= 16 ? bats::conv_backward_grouped_kernel<true, 16, PRE, W_SMEM>
+           : k_post >= 8  ? bats::conv_backward_grouped_kernel<true, 8, PRE, W_SMEM>
+                          : bats::conv_backward_grouped_kernel<true, 4, PRE, W_SMEM>;
+}
+
+// A step coprime to n near n times the golden ratio's fraction: multiples of it visit 0 .. n - 1 in a scattered order.
+static int scatter_step(int n) {
+    for (int s = std::max(1, (int)(0.618 * n));; ++s) {
+        int a = s, b = n;
+        while (b) {
+            const int r = a % b;
+            a = b;
+            b = r;
+        }
+        if (a == 1) return s;
+    }
+}
+
+// CTAs per sample group (the cluster size, 1 to 8): the one that leaves the least of the GPU idle in its last wave, the
+// smaller of equals. per_sm: CTAs of this size an SM holds; clusters of 8 find room on about 128 of the 152 SMs (they
+// lie within one GPC). 64 groups of 1024 threads: 2 (128 CTAs in one wave; 512 CTAs of clusters of 8 took four).
+static int conv_bwd_ranks(int groups, int threads, size_t smem) {
+    const long long per_sm = std::max<long long>(1, std::min<long long>(1024 / threads, 228 * 1024 / (long long)(smem + 4096)));
+    int best = 1;
+    double best_use = 0.0;
+    for (int r = 1; r <= bats::CONV_BWD_CLUSTER; r *= 2) {
+        const long long ctas = (long long)groups * r, slots = per_sm * (r == 8 ? 128 : 152);
+        const double use = (double)ctas / (double)((ctas + slots - 1) / slots * slots) * (r == 8 ? 128.0 / 152 : 1.0);
+        if (use > best_use * 1.02) {
+            best_use = use;
+            best = r;
+        }
+    }
+    return best;
+}
+
+static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* bucket_offsets, long long ev_cap,
+                                       const float* weights, const bats::ConvBwdShape& sh, const float* post_times,
+                                       const void* tables, const int* nvalid, float tau_s, float tau,
+                                       long long pre_slots, float* grad, float* pre_errors, int batch, int group,
+                                       cudaStream_t stream) {
+    const long long taps = (long long)sh.C_out * sh.fx * sh.fy;
+    constexpr size_t LIMIT = 224 * 1024;
+    const bool w = pre_errors && conv_grouped_smem(taps, sh.C, 64, true) <= LIMIT;
+    int batch_ev = 512;
+    while (batch_ev > 32 && conv_grouped_smem(taps, sh.C, batch_ev, w) > LIMIT) batch_ev /= 2;
+    const size_t smem = conv_grouped_smem(taps, sh.C, batch_ev, w);
+    auto* kernel = !pre_errors ? conv_grouped_kernel<false, false>(sh.k_post)
+                   : w         ? conv_grouped_kernel<true, true>(sh.k_post)
+                               : conv_grouped_kernel<true, false>(sh.k_post);
+    cudaError_t e = (cudaError_t)bats::max_dynamic_smem_set((const void*)kernel, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int groups = (batch + group - 1) / group, threads = (int)(((taps + 31) / 32) * 32);
+    const int ranks = conv_bwd_ranks(groups, threads, smem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ranks, groups);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ranks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1 + (unsigned)bats::pdl_attribute(attr + 1);
+    return cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const bats::Event*>(events_bucketed), bucket_offsets, ev_cap,
+                              weights, sh, post_times, reinterpret_cast<const float2*>(tables), nvalid, tau_s, tau,
+                              pre_slots, grad, pre_errors, batch, group, batch_ev, scatter_step(sh.n_pos));
+}
+
 extern "C" int bats_conv_backward_grouped(const void* events_bucketed, const int* bucket_offsets, long long ev_cap,
                                           const float* weights, int batch, int X, int Y, int C, int fx, int fy,
                                           int C_out, int k_pre, const float* post_times, const void* tables,
@@ -791,28 +1015,10 @@ extern "C" int bats_conv_backward_grouped(const void* events_bucketed, const int
     const long long pre_slots = (long long)X * Y * C * k_pre;
     const size_t gsmem = (size_t)taps * C * sizeof(float) + (size_t)C * sizeof(int);
     BATS_REQUIRE(gsmem <= 160 * 1024, BATS_ERR_BAD_SHAPE, "conv_backward_grouped: filter gradient too large");
-    const int w_in_smem = pre_errors && gsmem + (size_t)taps * C * sizeof(float) <= 200 * 1024;
-    const size_t smem = gsmem + (w_in_smem ? (size_t)taps * C * sizeof(float) : 0);
     if (pre_errors) BATS_CUDA(cudaMemsetAsync(pre_errors, 0, (size_t)batch * pre_slots * sizeof(float), stream));
-    BATS_CUDA((cudaError_t)bats::max_dynamic_smem_set((const void*)bats::conv_backward_grouped_kernel, (int)smem));
-    const int threads = (int)(((taps + 31) / 32) * 32);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(bats::CONV_BWD_CLUSTER, batch);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = bats::CONV_BWD_CLUSTER;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1 + (unsigned)bats::pdl_attribute(attr + 1);
-    BATS_CUDA(cudaLaunchKernelEx(&cfg, bats::conv_backward_grouped_kernel,
-                                 reinterpret_cast<const bats::Event*>(events_bucketed), bucket_offsets, X * Y, ev_cap,
-                                 weights, Y, C, fx, fy, C_out, Xo, Yo, k_pre, post_times,
-                                 reinterpret_cast<const float2*>(tables), nvalid, k_post, tau_s, tau, pre_slots,
-                                 grad_per_sample, pre_errors, batch, 1, w_in_smem));
+    const bats::ConvBwdShape sh = {Y, C, fx, fy, C_out, Xo, Yo, k_pre, k_post, X * Y};
+    BATS_CUDA(launch_conv_grouped(events_bucketed, bucket_offsets, ev_cap, weights, sh, post_times, tables, nvalid,
+                                  tau_s, tau, pre_slots, grad_per_sample, pre_errors, batch, 1, stream));
     return BATS_OK;
 }
 
@@ -861,32 +1067,26 @@ extern "C" int bats_conv_backward_adam(const void* events, const int* ev_slot, c
     if (pre_errors) BATS_CUDA(cudaMemsetAsync(pre_errors, 0, (size_t)batch * pre_slots * sizeof(float), stream));
     const bool grouped = events_bucketed && bucket_offsets && taps <= 1024 && (long long)X * Y <= 255 &&
                          (size_t)taps * C * sizeof(float) + (size_t)C * sizeof(int) <= 160 * 1024;
-    const size_t gbytes = (size_t)taps * C * sizeof(float) + (grouped ? (size_t)C * sizeof(int) : 0);
+    const size_t gbytes = (size_t)taps * C * sizeof(float);
     BATS_REQUIRE(gbytes <= 160 * 1024, BATS_ERR_BAD_SHAPE, "conv_backward_adam: filter gradient too large");
-    const int threads = (int)std::min<long long>(1024, ((taps + 31) / 32) * 32);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(bats::CONV_BWD_CLUSTER, groups);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = gbytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = bats::CONV_BWD_CLUSTER;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1 + (unsigned)bats::pdl_attribute(attr + 1);
     if (grouped) {
-        const int w_in_smem = pre_errors && gbytes + (size_t)taps * C * sizeof(float) <= 200 * 1024;
-        if (w_in_smem) cfg.dynamicSmemBytes = gbytes + (size_t)taps * C * sizeof(float);
-        BATS_CUDA((cudaError_t)bats::max_dynamic_smem_set((const void*)bats::conv_backward_grouped_kernel,
-                                                          (int)cfg.dynamicSmemBytes));
-        BATS_CUDA(cudaLaunchKernelEx(&cfg, bats::conv_backward_grouped_kernel,
-                                     reinterpret_cast<const bats::Event*>(events_bucketed), bucket_offsets, X * Y,
-                                     ev_cap, (const float*)weights, Y, C, fx, fy, C_out, Xo, Yo, k_pre, post_times,
-                                     reinterpret_cast<const float2*>(tables), nvalid, k_post, tau_s, tau, pre_slots,
-                                     part, pre_errors, batch, group, w_in_smem));
+        const bats::ConvBwdShape sh = {Y, C, fx, fy, C_out, Xo, Yo, k_pre, k_post, X * Y};
+        BATS_CUDA(launch_conv_grouped(events_bucketed, bucket_offsets, ev_cap, weights, sh, post_times, tables, nvalid,
+                                      tau_s, tau, pre_slots, part, pre_errors, batch, group, stream));
     } else {
+        const int threads = (int)std::min<long long>(1024, ((taps + 31) / 32) * 32);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(bats::CONV_BWD_CLUSTER, groups);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = gbytes;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = bats::CONV_BWD_CLUSTER;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1 + (unsigned)bats::pdl_attribute(attr + 1);
         BATS_CUDA((cudaError_t)bats::max_dynamic_smem_set((const void*)bats::conv_backward_cluster_kernel, (int)gbytes));
         int top = 1;
         while (top * 2 <= k_post) top *= 2;

@@ -748,18 +748,6 @@ bwd_pre_err_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_coun
 // (The weight gradient of narrow layers keeps the thread-per-neuron merge of bwd_grad_warp_kernel,
 // which costs a few instructions per event for all neurons at once, with more sample groups instead.)
 
-// Post-spike position of every post neuron for a pre spike at time t: p = number of valid post spikes
-// with t_k <= t (the first k with t_k > t), by binary search over the neuron's leading valid spikes.
-__device__ __forceinline__ int post_position(const float* __restrict__ tk, int n, float t) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (tk[mid] <= t) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // Shared-memory copy of one sample's post-neuron data: times (N_post, K), tables (N_post, K + 1),
 // counts (N_post), issued as asynchronous copies (cp.async, no register round trip, all in flight at
 // once); the caller waits with cp_async_wait_all() and a barrier.
