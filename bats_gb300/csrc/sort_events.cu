@@ -54,7 +54,11 @@ struct SortShared {
     int wcnt[T / 32][SORT_BINS];
     int wofs[T / 32][SORT_BINS];
     int warp_tot[T / 32];
+    int appended;         // items found (gather_items)
+    unsigned kmin, kmax;  // their smallest and largest key
+    int pad_;             // the items behind are read as uint4
 };
+static_assert(sizeof(SortShared<256>) % 16 == 0 && sizeof(SortShared<512>) % 16 == 0, "uint4 reads of the items");
 
 template <int T>
 __device__ __forceinline__ int block_exclusive_flag_scan(bool f, SortShared<T>& sh, int& block_total) {
@@ -212,7 +216,213 @@ struct BucketDigit {
     __device__ int operator()(uint32_t, uint32_t slot) const { return (int)slot / div; }
 };
 
+// Appends the calling warp's items (up to 8 per lane, those with t[u] < +inf and u < 8) to the list, in no particular
+// order: one atomic per warp. Items past the room are only counted.
+template <int T, typename V, int N>
+__device__ __forceinline__ void append_items(const float (&t)[N], const uint32_t (&slot)[N], uint32_t* keys, V* vals,
+                                             int room, SortShared<T>& sh, unsigned& kmin, unsigned& kmax) {
+    const int lane = threadIdx.x & 31;
+    int c = 0;
+#pragma unroll
+    for (int u = 0; u < N; ++u) c += t[u] < BATS_INF ? 1 : 0;
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    int base = 0;
+    if (lane == 31) base = atomicAdd(&sh.appended, incl);
+    int pos = __shfl_sync(0xffffffffu, base, 31) + incl - c;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        if (t[u] < BATS_INF) {
+            const uint32_t key = float_to_key(t[u]);
+            kmin = min(kmin, key);
+            kmax = max(kmax, key);
+            if (pos < room) {
+                keys[pos] = key;
+                vals[pos] = (V)slot[u];
+            }
+            ++pos;
+        }
+    }
+}
+
+// The sample's valid slots as an unordered list in shared memory (at most room items), with their number and their
+// smallest and largest key in sh. One pass over the slots (with the pre layer's spike counts: over those below them),
+// several loads in flight per thread.
+template <int T, typename V>
+__device__ __forceinline__ void gather_items(const float* __restrict__ tsrc, const int* __restrict__ cnt_src, int n_slots,
+                                             int k_pre, uint32_t* keys, V* vals, int room, SortShared<T>& sh) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned kmin = 0xffffffffu, kmax = 0u;
+    if (cnt_src) {
+        const int n_pre = n_slots / k_pre;
+        for (int r0 = warp * 32; r0 < n_pre; r0 += T) {
+            const int j = r0 + lane;
+            const int c = j < n_pre ? min(max(cnt_src[j], 0), k_pre) : 0;
+            const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)c);
+            for (int q0 = 0; q0 < most; q0 += 8) {
+                float t[8];
+                uint32_t slot[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    slot[u] = (uint32_t)(j * k_pre + q0 + u);
+                    t[u] = q0 + u < c ? tsrc[slot[u]] : BATS_INF;
+                }
+                append_items<T, V, 8>(t, slot, keys, vals, room, sh, kmin, kmax);
+            }
+        }
+    } else if ((n_slots & 3) == 0) {
+        const float4* t4 = reinterpret_cast<const float4*>(tsrc);
+        const int n4 = n_slots >> 2;
+        for (int q0 = warp * 32; q0 < n4; q0 += 2 * T) {
+            float t[8];
+            uint32_t slot[8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int q = q0 + h * T + lane;
+                const float4 v = q < n4 ? t4[q] : make_float4(BATS_INF, BATS_INF, BATS_INF, BATS_INF);
+                t[4 * h] = v.x;
+                t[4 * h + 1] = v.y;
+                t[4 * h + 2] = v.z;
+                t[4 * h + 3] = v.w;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) slot[4 * h + u] = (uint32_t)(4 * q + u);
+            }
+            append_items<T, V, 8>(t, slot, keys, vals, room, sh, kmin, kmax);
+        }
+    } else {
+        for (int q0 = warp * 32; q0 < n_slots; q0 += 4 * T) {
+            float t[4];
+            uint32_t slot[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int q = q0 + h * T + lane;
+                slot[h] = (uint32_t)q;
+                t[h] = q < n_slots ? tsrc[q] : BATS_INF;
+            }
+            append_items<T, V, 4>(t, slot, keys, vals, room, sh, kmin, kmax);
+        }
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) {
+        atomicMin(&sh.kmin, kmin);
+        atomicMax(&sh.kmax, kmax);
+    }
+}
+
+// A time's bucket among `buckets` equal parts of [t_min, t_max]: every step is monotone in t, so that the buckets are
+// in time order whatever the roundings.
+__device__ __forceinline__ int time_bucket(uint32_t key, float t_min, float scale, int buckets) {
+    return (int)fminf((key_to_float(key) - t_min) * scale, (float)(buckets - 1));
+}
+
+constexpr int SORT_BUCKET_LIMIT = 384;  // items of one bucket up to which ranking them by comparison is taken
+
+// Sorts the n gathered items (ka, va) by (key, slot) with (kb, vb) as the second buffer, leaving them in (ka, va):
+// the items are dealt into buckets of equal time spans, and each finds its place inside its bucket by counting the
+// smaller ones. Six barriers whatever n, against three per 512 items and pass of a radix sort. False (nothing sorted)
+// when one bucket holds more than SORT_BUCKET_LIMIT items or the times span no finite range.
+template <int T, typename V>
+__device__ __forceinline__ bool bucket_sort(uint32_t* ka, V* va, uint32_t* kb, V* vb, int n, SortShared<T>& sh) {
+    constexpr int NB = T / 32 * SORT_BINS;  // as many buckets as the counters of the counting passes hold
+    constexpr int PER = NB / T;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int* count = &sh.wcnt[0][0];
+    int* start = &sh.wofs[0][0];
+    const float t_min = key_to_float(sh.kmin), span = key_to_float(sh.kmax) - t_min;
+    const bool usable = span > 0.0f && span <= 3.0e38f;  // uniform
+    const float scale = usable ? fminf((float)NB / span, 3.0e38f) : 0.0f;
+    for (int q = tid; q < NB; q += T) count[q] = 0;
+    __syncthreads();
+    if (!usable && n > SORT_BUCKET_LIMIT) return false;
+    for (int i = tid; i < n; i += T) atomicAdd(&count[time_bucket(ka[i], t_min, scale, NB)], 1);
+    __syncthreads();
+    // Exclusive scan: thread tid owns buckets PER * tid ..
+    int own[PER], sum = 0;
+    bool over = false;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        own[u] = count[PER * tid + u];
+        over |= own[u] > SORT_BUCKET_LIMIT;
+        sum += own[u];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) sh.warp_tot[warp] = incl;
+    if (__syncthreads_or(over)) return false;
+    int base = incl - sum;
+    for (int w = 0; w < warp; ++w) base += sh.warp_tot[w];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        start[PER * tid + u] = base;
+        count[PER * tid + u] = base;  // the scatter's cursor; afterwards the bucket's end
+        base += own[u];
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += T) {
+        const uint32_t key = ka[i];
+        const int pos = atomicAdd(&count[time_bucket(key, t_min, scale, NB)], 1);
+        kb[pos] = key;
+        vb[pos] = va[i];
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += T) {
+        const uint32_t key = kb[i];
+        const V val = vb[i];
+        const int b = time_bucket(key, t_min, scale, NB);
+        const int lo = start[b], hi = count[b];
+        int r = lo;
+        for (int q = lo; q < hi; ++q) {
+            const uint32_t kq = kb[q];
+            r += (kq < key || (kq == key && vb[q] < val)) ? 1 : 0;
+        }
+        ka[r] = key;
+        va[r] = val;
+    }
+    __syncthreads();
+    return true;
+}
+
+struct SlotDigit {
+    int shift;
+    __device__ int operator()(uint32_t, uint32_t slot) const { return (int)((slot >> shift) & 255u); }
+};
+
+// LSD radix sort of the items by (digits of the slot, if SLOTS, then) the time key, 8 bits a pass; passes whose digit is
+// uniform are skipped. With SLOTS the result does not depend on the order the items came in; without, ties keep it.
+template <int T, typename V, bool SLOTS>
+__device__ __forceinline__ void radix_sort(uint32_t*& ka, V*& va, uint32_t*& kb, V*& vb, int n, SortShared<T>& sh) {
+    const int tid = threadIdx.x;
+    for (int pass = SLOTS ? -(int)sizeof(V) : 0; pass < 4; ++pass) {
+        const int shift = pass < 0 ? (pass + (int)sizeof(V)) * 8 : pass * 8;
+        if (tid < SORT_BINS) sh.hist[tid] = 0;
+        __syncthreads();
+        for (int i = tid; i < n; i += T)
+            atomicAdd(&sh.hist[((pass < 0 ? (uint32_t)va[i] : ka[i]) >> shift) & 255u], 1);
+        __syncthreads();
+        if (__syncthreads_or(tid < SORT_BINS && sh.hist[tid] == n)) continue;
+        scan_bins<T>(sh);
+        if (pass < 0)
+            stable_pass<T>(ka, va, kb, vb, n, sh, SlotDigit{shift});
+        else
+            stable_pass<T>(ka, va, kb, vb, n, sh, TimeDigit{shift});
+        uint32_t* t0 = ka; ka = kb; kb = t0;
+        V* t1 = va; va = vb; vb = t1;
+    }
+}
+
 // V: type of the slot values (uint16_t when n_slots <= 65536). smem_cap: items held in shared memory.
+// Samples of up to smem_cap valid slots: gathered into shared memory in any order, then bucket_sort (or, where the times
+// crowd too much, radix_sort over slot and time). Larger ones: compacted in slot order into the global scratch and
+// sorted there by radix_sort over the time alone. The order is by time, ties by slot, either way.
 template <typename V, int T>
 __global__ void __launch_bounds__(T)
 sort_events_kernel(const float* __restrict__ times, const int* __restrict__ pre_counts, int n_slots, int k_pre,
@@ -223,7 +433,7 @@ sort_events_kernel(const float* __restrict__ times, const int* __restrict__ pre_
                    unsigned char* __restrict__ scratch, const int* __restrict__ sample_order) {
     pdl_prologue();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int SORT_THREADS = T, SORT_WARPS = T / 32;
+    constexpr int SORT_THREADS = T;
     SortShared<T>& sh = *reinterpret_cast<SortShared<T>*>(smem_raw);
     unsigned char* smem_items = smem_raw + sizeof(SortShared<T>);
 
@@ -232,45 +442,24 @@ sort_events_kernel(const float* __restrict__ times, const int* __restrict__ pre_
     const int tid = threadIdx.x;
     const long long sample_off = (long long)s * n_slots;
     const float* tsrc = times + sample_off;
-
-    // Count valid slots first so that the buffers can be chosen. With the pre layer's spike counts, neuron
-    // j's valid slots are its first pre_counts[j] (the forward kernels write +inf after them), so only
-    // those are read. Otherwise, with 16-byte rows (n_slots % 4 == 0) each warp counts, and later
-    // compacts, its own contiguous range of slots, so neither pass needs a block-wide barrier per round.
-    int n = 0;
     const int n_pre = n_slots / k_pre;
+    // With the pre layer's spike counts, neuron j's valid slots are among its first pre_counts[j] (the forward kernels
+    // write +inf after them), so only those are read.
     const int* cnt_src = pre_counts ? pre_counts + (long long)s * n_pre : nullptr;
-    const bool vec = !cnt_src && (n_slots & 3) == 0;
-    const int n4 = n_slots >> 2;
-    const int per_warp4 = (n4 + SORT_WARPS - 1) / SORT_WARPS;
-    const int w_lo = min(n4, (tid >> 5) * per_warp4), w_hi = min(n4, w_lo + per_warp4);
-    const float4* t4 = reinterpret_cast<const float4*>(tsrc);
-    if (vec) {
-        int c = 0;
-        for (int q = w_lo + (tid & 31); q < w_hi; q += 32) {
-            const float4 v = t4[q];
-            c += (v.x < BATS_INF) + (v.y < BATS_INF) + (v.z < BATS_INF) + (v.w < BATS_INF);
-        }
-        for (int o = 16; o >= 1; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if ((tid & 31) == 0) sh.warp_tot[tid >> 5] = c;
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < SORT_WARPS; ++w) n += sh.warp_tot[w];
-    } else if (cnt_src) {
-        int c = 0;
-        for (int j = tid; j < n_pre; j += SORT_THREADS) c += leading_valid(cnt_src, tsrc, j, k_pre);
-        for (int o = 16; o >= 1; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if ((tid & 31) == 0) sh.warp_tot[tid >> 5] = c;
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < SORT_WARPS; ++w) n += sh.warp_tot[w];
-        __syncthreads();
-    } else {
-        for (int r0 = 0; r0 < n_slots; r0 += SORT_THREADS) {
-            const int slot = r0 + tid;
-            n += __syncthreads_count(slot < n_slots && tsrc[slot] < BATS_INF);
-        }
+
+    uint32_t* ka = reinterpret_cast<uint32_t*>(smem_items);
+    uint32_t* kb = ka + smem_cap;
+    V* va = reinterpret_cast<V*>(kb + smem_cap);
+    V* vb = va + smem_cap;
+    if (tid == 0) {
+        sh.appended = 0;
+        sh.kmin = 0xffffffffu;
+        sh.kmax = 0u;
     }
+    __syncthreads();
+    gather_items<T, V>(tsrc, cnt_src, n_slots, k_pre, ka, va, smem_cap, sh);
+    __syncthreads();
+    const int n = sh.appended;
     if (n == 0) {
         // No spike in this sample: empty event list (and empty buckets).
         if (tid == 0) ev_count[s] = 0;
@@ -278,121 +467,80 @@ sort_events_kernel(const float* __restrict__ times, const int* __restrict__ pre_
             for (int q = tid; q <= n_buckets; q += SORT_THREADS) bucket_off[(long long)s * (n_buckets + 1) + q] = 0;
         return;
     }
-
-    // Two key and two value buffers: in shared memory when the sample's items fit, else in this sample's
-    // part of the global scratch (cap items each).
-    uint32_t *ka, *kb;
-    V *va, *vb;
-    {
-        const long long room = n <= smem_cap ? smem_cap : cap;
-        unsigned char* base = n <= smem_cap ? smem_items : scratch + (long long)s * cap * (8 + 2 * sizeof(V));
-        ka = reinterpret_cast<uint32_t*>(base);
-        kb = ka + room;
-        va = reinterpret_cast<V*>(kb + room);
-        vb = va + room;
-    }
-
-    // Compaction in slot order (stable).
-    if (cnt_src) {
-        // Thread per pre neuron, rounds of SORT_THREADS neurons; each copies its leading valid slots.
-        int base = 0;
-        for (int r0 = 0; r0 < n_pre; r0 += SORT_THREADS) {
-            const int j = r0 + tid;
-            const int c = j < n_pre ? leading_valid(cnt_src, tsrc, j, k_pre) : 0;
-            int tot;
-            int pos = base + block_exclusive_scan(c, sh, tot);
-            const int slot0 = j * k_pre;
-            const int lim = c > 0 ? min(max(cnt_src[j], 0), k_pre) : 0;
-            for (int q0 = 0; q0 < lim; q0 += 8) {
-                float tv[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) tv[u] = q0 + u < lim ? tsrc[slot0 + q0 + u] : BATS_INF;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (tv[u] < BATS_INF) {
-                        ka[pos] = float_to_key(tv[u]);
-                        va[pos] = (V)(slot0 + q0 + u);
-                        ++pos;
-                    }
-                }
-            }
-            base += tot;
-        }
-    } else if (vec) {
-        int base = 0;
-        for (int w = 0; w < (tid >> 5); ++w) base += sh.warp_tot[w];
-        const int lane = tid & 31;
-        for (int q0 = w_lo; q0 < w_hi; q0 += 32) {
-            const int q = q0 + lane;
-            float4 v = make_float4(BATS_INF, BATS_INF, BATS_INF, BATS_INF);
-            if (q < w_hi) v = t4[q];
-            const int c = (v.x < BATS_INF) + (v.y < BATS_INF) + (v.z < BATS_INF) + (v.w < BATS_INF);
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            int pos = base + incl - c;
-            const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (vv[u] < BATS_INF) {
-                    ka[pos] = float_to_key(vv[u]);
-                    va[pos] = (V)(4 * q + u);
-                    ++pos;
-                }
-            }
-            base += __shfl_sync(0xffffffffu, incl, 31);
-        }
-    } else {
-        int base = 0;
-        for (int r0 = 0; r0 < n_slots; r0 += SORT_THREADS) {
-            const int slot = r0 + tid;
-            float t = BATS_INF;
-            if (slot < n_slots) t = tsrc[slot];
-            const bool f = t < BATS_INF;
-            int tot;
-            const int pos = block_exclusive_flag_scan(f, sh, tot);
-            if (f) {
-                ka[base + pos] = float_to_key(t);
-                va[base + pos] = (V)slot;
-            }
-            base += tot;
-        }
-    }
-    __syncthreads();
-
-    if (n <= SORT_THREADS) {
-        // One item per thread: its rank is the number of smaller keys plus the equal keys before it in
-        // compaction order, which is the stable order of the radix passes below, with one barrier.
+    if (n <= 256) {
+        // At most one item per thread: its rank is the number of smaller items, with one barrier.
+        if (tid < ((4 - n) & 3)) ka[n + tid] = 0xffffffffu;  // up to a multiple of four
+        __syncthreads();
         const uint32_t key = tid < n ? ka[tid] : 0u;
         const V val = tid < n ? va[tid] : V(0);
-        int rank = 0;
-        if (tid < n)
-            for (int q = 0; q < n; ++q) {
-                const uint32_t kq = ka[q];
-                rank += (kq < key || (kq == key && q < tid)) ? 1 : 0;
-            }
         if (tid < n) {
+            int rank = 0, same = 0;
+            const uint4* k4 = reinterpret_cast<const uint4*>(ka);
+#pragma unroll 2
+            for (int q = 0; q < (n + 3) >> 2; ++q) {
+                const uint4 k = k4[q];
+                rank += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
+                same += (k.x == key) + (k.y == key) + (k.z == key) + (k.w == key);
+            }
+            if (same > 1)  // equal times: by slot
+                for (int q = 0; q < n; ++q) rank += (ka[q] == key && va[q] < val) ? 1 : 0;
             kb[rank] = key;
             vb[rank] = val;
         }
         __syncthreads();
         uint32_t* t0 = ka; ka = kb; kb = t0;
         V* t1 = va; va = vb; vb = t1;
-    }
-    // LSD radix sort on the time key, 4 passes of 8 bits; passes whose digit is uniform are skipped.
-    for (int shift = 0; n > SORT_THREADS && shift < 32; shift += 8) {
-        if (tid < SORT_BINS) sh.hist[tid] = 0;
+    } else if (n <= smem_cap) {
+        if (!bucket_sort<T, V>(ka, va, kb, vb, n, sh)) radix_sort<T, V, true>(ka, va, kb, vb, n, sh);
+    } else {
+        // Two key and two value buffers in this sample's part of the global scratch (cap items each); compaction in
+        // slot order (stable).
+        ka = reinterpret_cast<uint32_t*>(scratch + (long long)s * cap * (8 + 2 * sizeof(V)));
+        kb = ka + cap;
+        va = reinterpret_cast<V*>(kb + cap);
+        vb = va + cap;
+        int base = 0;
+        if (cnt_src) {
+            // Thread per pre neuron, rounds of SORT_THREADS neurons; each copies its leading valid slots.
+            for (int r0 = 0; r0 < n_pre; r0 += SORT_THREADS) {
+                const int j = r0 + tid;
+                const int c = j < n_pre ? leading_valid(cnt_src, tsrc, j, k_pre) : 0;
+                int tot;
+                int pos = base + block_exclusive_scan(c, sh, tot);
+                const int slot0 = j * k_pre;
+                const int lim = c > 0 ? min(max(cnt_src[j], 0), k_pre) : 0;
+                for (int q0 = 0; q0 < lim; q0 += 8) {
+                    float tv[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) tv[u] = q0 + u < lim ? tsrc[slot0 + q0 + u] : BATS_INF;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (tv[u] < BATS_INF) {
+                            ka[pos] = float_to_key(tv[u]);
+                            va[pos] = (V)(slot0 + q0 + u);
+                            ++pos;
+                        }
+                    }
+                }
+                base += tot;
+            }
+        } else {
+            for (int r0 = 0; r0 < n_slots; r0 += SORT_THREADS) {
+                const int slot = r0 + tid;
+                float t = BATS_INF;
+                if (slot < n_slots) t = tsrc[slot];
+                const bool f = t < BATS_INF;
+                int tot;
+                const int pos = block_exclusive_flag_scan(f, sh, tot);
+                if (f) {
+                    ka[base + pos] = float_to_key(t);
+                    va[base + pos] = (V)slot;
+                }
+                base += tot;
+            }
+        }
         __syncthreads();
-        for (int i = tid; i < n; i += SORT_THREADS) atomicAdd(&sh.hist[(ka[i] >> shift) & 255u], 1);
-        __syncthreads();
-        if (__syncthreads_or(tid < SORT_BINS && sh.hist[tid] == n)) continue;
-        scan_bins<T>(sh);
-        stable_pass<T>(ka, va, kb, vb, n, sh, TimeDigit{shift});
-        uint32_t* t0 = ka; ka = kb; kb = t0;
-        V* t1 = va; va = vb; vb = t1;
+        radix_sort<T, V, false>(ka, va, kb, vb, n, sh);
     }
 
     Event* eo = ev_out + (long long)s * cap;
