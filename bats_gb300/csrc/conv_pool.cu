@@ -344,9 +344,8 @@ __global__ void conv_backward_kernel(const Event* __restrict__ ev, const int* __
 
 // Conv backward on a cluster of CONV_BWD_CLUSTER CTAs per sample (thread-block cluster, distributed
 // shared memory). Thread = filter tap (co, dx, dy); the sample's events are dealt to the cluster's CTAs in
-// groups of CONV_BWD_EVENTS (group g to CTA rank g % CONV_BWD_CLUSTER), so that eight times as many CTAs hide the
-// latency of the post-spike lookups, which bounds the kernel; small groups deal the 150 events of an MNIST-shaped
-// sample evenly (groups of 32 left three of the eight CTAs idle). Every CTA accumulates its events' gradient terms in a shared-memory
+// groups of 32 (group g to CTA rank g % CONV_BWD_CLUSTER), so that eight times as many CTAs hide the
+// latency of the post-spike lookups. Every CTA accumulates its events' gradient terms in a shared-memory
 // copy of the per-sample filter gradient (taps x C), in event order; at the end each CTA sums one slice of
 // the gradient over the cluster's copies in rank order (deterministic) and writes it. The pre-spike errors
 // of a group of events are reduced over the taps inside the CTA that owns the group. Four events are
@@ -354,7 +353,6 @@ __global__ void conv_backward_kernel(const Event* __restrict__ ev, const int* __
 // entries) are in flight together.
 constexpr int CONV_BWD_CLUSTER = 8;
 constexpr int CONV_BWD_ILP = 4;
-constexpr int CONV_BWD_EVENTS = 8;
 
 __global__ void __launch_bounds__(1024)
 conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_slot,
@@ -367,8 +365,8 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) float Gs[];  // taps * C
-    __shared__ Event sev[CONV_BWD_EVENTS];
-    __shared__ float sred[CONV_BWD_EVENTS][33];
+    __shared__ Event sev[32];
+    __shared__ float sred[32][33];
     const unsigned rank = cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nwarps = blockDim.x >> 5;
@@ -382,9 +380,9 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
     for (int s = (int)blockIdx.y * group; s < s_end; ++s) {
     const int E = ev_count[s];
     const Event* evs = ev + (long long)s * ev_cap;
-    for (int g = (int)rank; g * CONV_BWD_EVENTS < E; g += CONV_BWD_CLUSTER) {
-        const int m0 = g * CONV_BWD_EVENTS;
-        const int cnt = min(CONV_BWD_EVENTS, E - m0);
+    for (int g = (int)rank; g * 32 < E; g += CONV_BWD_CLUSTER) {
+        const int m0 = g * 32;
+        const int cnt = min(32, E - m0);
         if (tid < cnt) sev[tid] = evs[m0 + tid];
         __syncthreads();
         for (int q0 = 0; q0 < cnt; q0 += CONV_BWD_ILP) {
@@ -466,25 +464,30 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
 // Conv backward over events grouped by input position (the bucketed copy of the sort with
 // bucket_width = C: one bucket per (x, y), time order inside), on a cluster of CONV_BWD_CLUSTER CTAs per
 // sample (position groups dealt to the ranks). Within a position group every filter tap sees one and the same post
-// neuron (x - dx, y - dy, co). A warp owns 32 consecutive taps ((dx fy + dy) C_out + co); its lanes are the group's
-// events, 32 at a time, and it goes through those of its taps whose post neuron lies inside the output and spiked: the
-// neuron's spike times and table rows lie on the lanes (K <= 32; loaded one neuron ahead), every lane finds its event's
-// place among them by a binary search over shuffles, adds its gradient term to the tap's row of the CTA's gradient copy
-// in shared memory ([tap][channel]: lanes of one channel are first added up along precomputed links, so that one lane
-// per channel updates its entry) and its pre-error term to a register.
+// neuron (x - dx, y - dy, co). A warp's lanes are the group's events, 32 at a time, and it goes through those taps whose
+// post neuron lies inside the output and spiked: the neuron's spike times and table rows lie on the lanes (K <= 32;
+// loaded one neuron ahead), every lane finds its event's place among them by a binary search over shuffles and leaves its
+// gradient term in shared memory. The events of a group are staged by (channel, time), so that a channel's terms are
+// neighbours: its first lane adds them in time order to the CTA's gradient copy in shared memory ([tap][channel]).
+// The pre-error of an event is its taps' terms summed as a balanced tree over each tile of 32 consecutive taps
+// ((co fx + dx) fy + dy; pairs 16 apart first, as warp_transpose_reduce adds lanes), the tiles then in order: a warp walks
+// the taps in the order of the tree's leaves and keeps the open subtrees' sums, so the errors do not depend on which taps
+// take part. The work is dealt in units of CONV_BWD_UNIT taps that form a subtree of a tile, taken by the warps from a
+// counter: output channels spike very unevenly, and with a tile per warp the warps waited for the busiest one 70 % of the
+// time (units of 32 taps 3.28 ms, of 16 2.29, of 8 2.35 at the size below).
 // The rank's events are taken in batches of whole positions (at most `batch_ev` events; a larger position in segments):
 // staged once for all warps with their channel decoded and their slots ranked (slot k of neuron j: the k-th event of j in
-// the group); the warps' pre-error terms of the batch meet in sred and are added at its end. Three barriers per batch.
-// The per-sample gradient copies are combined over the cluster as in conv_backward_cluster_kernel.
-// What bounds it: instruction issue (64 %). 12 x 12 x 15 -> 5 x 5 x 40, batch 128: 0.94 ms, 571 M warp instructions. A
-// thread per tap with a cursor over the post spikes took 2.65 ms (1.2 G warp instructions: with about ten post spikes
-// and twenty events per tap and position, some lane's cursor moved at every event, and half of the lanes lay outside the
-// output); the same with the output channels on the lanes and these batches 1.71 ms.
+// the group); the units' pre-error sums of the batch meet in sred and are added in order at its end. Three barriers per
+// batch. The per-sample gradient copies are combined over the cluster as in conv_backward_cluster_kernel.
+// What bounds it: instruction issue (4.7 M pairs of a spiking tap and up to 32 events, 8 rounds of a channel's terms each;
+// 67 % of the issue slots of 128 CTAs). 40 filters 5 x 5 x 15 over 12 x 12, 128 samples: 2.65 -> 2.07 ms, the same
+// sums.
 struct ConvBwdShape {
     int Y, C, fx, fy, C_out, Xo, Yo, k_pre, k_post, n_pos;
 };
 
-constexpr int CONV_BWD_POS = 255;  // positions of a layer at most (the buckets of the sort)
+constexpr int CONV_BWD_POS = (255 + CONV_BWD_CLUSTER - 1) / CONV_BWD_CLUSTER;  // positions per rank
+constexpr int CONV_BWD_UNIT = 16;                                              // taps per unit: two units per tile
 
 // ROWS: K <= 32, a neuron's rows fit the lanes; TOP: the largest power of two <= K (at most 16), the search's first step.
 template <bool ROWS, int TOP, bool PRE, bool W_SMEM>
@@ -493,40 +496,34 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
                              const float* __restrict__ W, ConvBwdShape sh, const float* __restrict__ post_t,
                              const float2* __restrict__ tab, const int* __restrict__ nvalid, float tau_s, float tau,
                              long long pre_slots, float* __restrict__ grad, float* __restrict__ pre_err, int batch,
-                             int group, int batch_ev, int step) {
+                             int group, int batch_ev) {
     pdl_prologue();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) float4 cb_smem[];
-    __shared__ int s_beg[CONV_BWD_POS], s_len[CONV_BWD_POS];
+    __shared__ int s_beg[CONV_BWD_POS], s_len[CONV_BWD_POS], s_at[CONV_BWD_POS], s_next;
     const float inv_tau_s = 1.0f / tau_s, inv_tau = 1.0f / tau;  // the error terms' factors, as reciprocals
-    const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
+    const int rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarps = blockDim.x >> 5, red_ld = nwarps | 1;
+    const int nwarps = blockDim.x >> 5;
     const int C = sh.C, taps = sh.C_out * sh.fx * sh.fy, K = sh.k_post;
+    constexpr int UNIT = CONV_BWD_UNIT, UNITS = 32 / UNIT;
+    const int tiles = (taps + 31) / 32, units = tiles * UNITS, red_ld = units | 1;
     const int total = taps * C;
     const int n_post = sh.Xo * sh.Yo * sh.C_out;
-    float4* sE = cb_smem;                                      // staged events: (t, es, e, channel)
-    float* sred = reinterpret_cast<float*>(sE + batch_ev);     // [event][warp]
-    int* sslot = reinterpret_cast<int*>(sred + batch_ev * red_ld);
-    int* kcount = sslot + batch_ev;                            // per channel: a split position's earlier events
-    float* Gs = reinterpret_cast<float*>(kcount + C);          // [tap][channel]
-    const bool has_tap = tid < taps;
-    const int co = tid % sh.C_out, dxy = tid / sh.C_out;
-    const int dx = dxy / sh.fy, dy = dxy % sh.fy;
+    float4* sE = cb_smem;                                   // staged events: (t, es, e, channel)
+    int* sslot = reinterpret_cast<int*>(sE + batch_ev);     // their slots
+    int* schan = sslot + batch_ev;                          // channels in time order (staging)
+    int* kcount = schan + batch_ev;                         // per channel: a split position's earlier events
+    float* Gs = reinterpret_cast<float*>(kcount + C);       // [tap][channel]
+    float* sWf = Gs + total;                                // W_SMEM: the filters, [tap][channel] as they lie
+    float* sval = (W_SMEM ? sWf + total : sWf) + warp * 32;       // per warp: a chunk's gradient terms
+    float* sred = (W_SMEM ? sWf + total : sWf) + nwarps * 32;     // PRE: [event][unit], 0 where no tap takes part
     for (int q = tid; q < total; q += blockDim.x) Gs[q] = 0.0f;
-    const int wbase = ((co * sh.fx + dx) * sh.fy + dy) * C;  // the tap's place in the filters
-    const float* Wk = W;
-    if (W_SMEM) {
-        float* sWf = Gs + total;
-        if (has_tap)
-            for (int c = 0; c < C; ++c) sWf[tid * C + c] = W[wbase + c];
-        Wk = sWf;
-    }
-    // The rank's positions in a scattered order (step is coprime to n_pos), so that every batch holds positions from all
-    // over the input: at the border only some taps reach an output, and their warps would wait for the others.
-    auto position = [&](int i) { return (int)((unsigned)(rank + i * ranks) * (unsigned)step % (unsigned)sh.n_pos); };
-    const int n_mine = rank < sh.n_pos ? (sh.n_pos - 1 - rank) / ranks + 1 : 0;
+    if (W_SMEM)
+        for (int q = tid; q < total; q += blockDim.x) sWf[q] = W[q];
+    const float* Wk = W_SMEM ? sWf : W;
+    const int n_mine = rank < sh.n_pos ? (sh.n_pos - 1 - rank) / CONV_BWD_CLUSTER + 1 : 0;
     // The cluster's samples (one with group == 1: the per-sample gradient), accumulated in order.
     const int s_end = min(batch, ((int)blockIdx.y + 1) * group);
     for (int s = (int)blockIdx.y * group; s < s_end; ++s) {
@@ -537,7 +534,7 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
         const float2* tab_lane = tab + pn_s * (K + 1) + lane;
         __syncthreads();
         for (int i = tid; i < n_mine; i += blockDim.x) {
-            const int g = position(i);
+            const int g = rank + i * CONV_BWD_CLUSTER;
             s_beg[i] = bo[g];
             s_len[i] = bo[g + 1] - bo[g];
         }
@@ -553,92 +550,75 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
                 while (i1 < n_mine && cnt + s_len[i1] <= batch_ev) cnt += s_len[i1++];
             }
             if (cnt > 0) {
-                if (split && off0 == 0)
-                    for (int q = tid; q < C; q += blockDim.x) kcount[q] = 0;
-                // Stage the batch: a warp per position (a split one: 32 events per warp).
-                for (int w = warp; w < (split ? (cnt + 31) / 32 : i1 - i0); w += nwarps) {
-                    int at = 0, len = cnt, src = s_beg[i0] + off0;
-                    if (split) {
-                        at = w * 32;
-                        len = min(32, cnt - at);
-                        src += at;
-                    } else {
-                        for (int i = i0; i < i0 + w; ++i) at += s_len[i];
-                        len = s_len[i0 + w];
-                        src = s_beg[i0 + w];
+                // Stage the batch by (channel, time) per position: a warp per position (a split one: all warps).
+                auto channel = [&](int src) {
+                    return __ldg(reinterpret_cast<const int*>(evs + src) + 1) % C;
+                };
+                auto place = [&](int at, int q, int len, int src, int base) {
+                    const int c = schan[at + q];
+                    int less = 0, earlier = 0;
+                    for (int r = 0; r < len; ++r) {
+                        const int cr = schan[at + r];
+                        less += cr < c ? 1 : 0;
+                        earlier += cr == c && r < q ? 1 : 0;
                     }
-                    for (int q = lane; q < len; q += 32) {
-                        const float4 e = __ldg(reinterpret_cast<const float4*>(evs + src + q));  // (t, j, es, e)
-                        const int j = __float_as_int(e.y);
-                        sE[at + q] = make_float4(e.x, e.z, e.w, __int_as_float(j % C));
-                        sslot[at + q] = j * sh.k_pre;
-                    }
-                    if (PRE && !split) {
-                        __syncwarp();
-                        for (int q = lane; q < len; q += 32) {
-                            const int c = __float_as_int(sE[at + q].w);
-                            int earlier = 0;
-                            for (int r = 0; r < q; ++r) earlier += __float_as_int(sE[at + r].w) == c ? 1 : 0;
-                            sslot[at + q] += earlier;
-                        }
-                    }
-                }
-                __syncthreads();
-                if (PRE && split) {
-                    for (int q = tid; q < cnt; q += blockDim.x) {
-                        const int c = __float_as_int(sE[q].w);
-                        int earlier = kcount[c];
-                        for (int r = 0; r < q; ++r) earlier += __float_as_int(sE[r].w) == c ? 1 : 0;
-                        sslot[q] += earlier;
-                    }
+                    const float4 e = __ldg(reinterpret_cast<const float4*>(evs + src + q));  // (t, j, es, e)
+                    const int to = at + less + earlier;
+                    sE[to] = make_float4(e.x, e.z, e.w, __int_as_float(c));
+                    sslot[to] = __float_as_int(e.y) * sh.k_pre + base + earlier;
+                };
+                if (split) {
+                    const int src = s_beg[i0] + off0;
+                    if (off0 == 0)
+                        for (int q = tid; q < C; q += blockDim.x) kcount[q] = 0;
+                    for (int q = tid; q < cnt; q += blockDim.x) schan[q] = channel(src + q);
+                    __syncthreads();
+                    for (int q = tid; q < cnt; q += blockDim.x) place(0, q, cnt, src, kcount[schan[q]]);
                     __syncthreads();
                     for (int c = tid; c < C; c += blockDim.x) {
                         int more = 0;
-                        for (int r = 0; r < cnt; ++r) more += __float_as_int(sE[r].w) == c ? 1 : 0;
+                        for (int r = 0; r < cnt; ++r) more += schan[r] == c ? 1 : 0;
                         kcount[c] += more;
                     }
-                }
-                // Every warp through the batch's positions.
-                int at = 0;
-                for (int i = i0; i < i1; ++i) {
-                    const int len = split ? cnt : s_len[i];
-                    if (len == 0) continue;
-                    // Lane: one of the warp's taps, its post neuron (within the sample) and that neuron's spike count.
-                    const int g = position(i);
-                    const int xo = g / sh.Y - dx, yo = g % sh.Y - dy;
-                    const bool in = has_tap && xo >= 0 && yo >= 0 && xo < sh.Xo && yo < sh.Yo;
-                    const int pn_l = in ? (xo * sh.Yo + yo) * sh.C_out + co : 0;
-                    const int n_l = in ? __ldg(nvalid + pn_s + pn_l) : 0;
-                    const unsigned spiking = __ballot_sync(0xffffffffu, n_l > 0);
-                    if (!spiking) {  // no spike under the warp's taps
-                        if (PRE)
-                            for (int q = lane; q < len; q += 32) sred[(at + q) * red_ld + warp] = 0.0f;
-                        at += len;
-                        continue;
+                } else {
+                    for (int w = warp; w < i1 - i0; w += nwarps) {
+                        int at = 0;
+                        for (int i = i0; i < i0 + w; ++i) at += s_len[i];
+                        const int len = s_len[i0 + w], src = s_beg[i0 + w];
+                        if (lane == 0) s_at[i0 + w] = at;
+                        for (int q = lane; q < len; q += 32) schan[at + q] = channel(src + q);
+                        __syncwarp();
+                        for (int q = lane; q < len; q += 32) place(at, q, len, src, 0);
                     }
-                    for (int q0 = 0; q0 < len; q0 += 32) {
-                        const bool on = q0 + lane < len;
-                        const float4 e = on ? sE[at + q0 + lane] : make_float4(-BATS_INF, 0.0f, 0.0f, __int_as_float(-1));
-                        const int c = __float_as_int(e.w);
-                        const float f1 = e.y * inv_tau_s, f2 = e.z * inv_tau;
-                        // Lanes of the same channel, as links to the next lane, the 2nd, 4th, 8th and 16th after it
-                        // (32: none); head: the first lane of its channel.
-                        const unsigned peers = __match_any_sync(0xffffffffu, c);
-                        const unsigned after = peers & ~(2u * lanemask_lt() + 1u);
-                        const bool head = on && (peers & lanemask_lt()) == 0u;
-                        int link[5];
-                        link[0] = after ? __ffs(after) - 1 : 32;
-#pragma unroll
-                        for (int m = 1; m < 5; ++m) {
-                            const int far = __shfl_sync(0xffffffffu, link[m - 1], link[m - 1] & 31);
-                            link[m] = link[m - 1] < 32 ? far : 32;
-                        }
-                        const int longest = (int)__reduce_max_sync(0xffffffffu, on ? (unsigned)__popc(peers) : 0u);
-                        float* g_lane = Gs + warp * 32 * C + (on ? c : 0);       // + tap lane * C
-                        const float* w_lane = Wk + (W_SMEM ? warp * 32 * C : 0) + (on ? c : 0);
-                        float acc = 0.0f;
-                        // Rows of the neuron of tap lane b: K spike times and table entries on the lanes, +inf and 0
-                        // past its spikes.
+                }
+                if (PRE)
+                    for (int q = tid; q < cnt * red_ld; q += blockDim.x) sred[q] = 0.0f;
+                if (tid == 0) s_next = 0;
+                __syncthreads();
+                // Units of taps from the counter, each through the batch's positions.
+                for (;;) {
+                    int u = 0;
+                    if (lane == 0) u = atomicAdd(&s_next, 1);
+                    u = __shfl_sync(0xffffffffu, u, 0);
+                    if (u >= units) break;
+                    // Leaf i of the unit is tap `leaf_tap(i)` of the tile: the bits of its place in the tree reversed.
+                    const int tile0 = u / UNITS * 32, leaf0 = u % UNITS * UNIT;
+                    auto leaf_tap = [&](int i) { return tile0 + (int)(__brev((unsigned)(leaf0 + i)) >> 27); };
+                    const int tap = leaf_tap(lane % UNIT);
+                    const bool has_tap = tap < taps;
+                    const int co = tap / (sh.fx * sh.fy), dx = tap / sh.fy % sh.fx, dy = tap % sh.fy;
+                    for (int i4 = i0; i4 < i1; i4 += UNITS) {
+                        // Lane: one of the unit's taps (lane % UNIT) at one of 32 / UNIT positions, its post neuron
+                        // (within the sample) and that neuron's spike count.
+                        const int i = i4 + lane / UNIT, g = rank + i * CONV_BWD_CLUSTER;
+                        const int xo = g / sh.Y - dx, yo = g % sh.Y - dy;
+                        const bool in = has_tap && i < i1 && xo >= 0 && yo >= 0 && xo < sh.Xo && yo < sh.Yo &&
+                                        s_len[min(i, i1 - 1)] > 0;
+                        const int pn_l = in ? (xo * sh.Yo + yo) * sh.C_out + co : 0;
+                        const int n_l = in ? __ldg(nvalid + pn_s + pn_l) : 0;
+                        unsigned spiking = __ballot_sync(0xffffffffu, n_l > 0);
+                        // Rows of the neuron at lane b: K spike times and table entries on the lanes, +inf and 0 past its
+                        // spikes.
                         float t_row, a_row, b_row;
                         int n_row, pn_row;
                         auto load = [&](int b) {
@@ -653,63 +633,116 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
                                 b_row = ab.y;
                             }
                         };
-                        unsigned todo = spiking;
-                        load(__ffs(todo) - 1);
-                        while (todo) {
-                            const int b = __ffs(todo) - 1;
-                            todo &= todo - 1u;
-                            const float t_cur = t_row, a_cur = a_row, b_cur = b_row;
-                            const int n = n_row, pn = pn_row;
-                            if (todo) load(__ffs(todo) - 1);
-                            // The event's place among the spikes: p = #{k : t_k <= t}.
-                            float A, B;
-                            bool valid;
-                            if (ROWS) {
-                                int last = -1;  // p - 1
+                        while (spiking) {  // the positions with a spike under the unit's taps
+                            const int p = (__ffs(spiking) - 1) / UNIT;
+                            const unsigned mine = (spiking >> (UNIT * p)) & 0xffffu;
+                            spiking &= ~(0xffffu << (UNIT * p));
+                            const bool few = __popc(mine) <= 2;
+                            const int len = split ? cnt : s_len[i4 + p], at = split ? 0 : s_at[i4 + p];
+                            for (int q0 = 0; q0 < len; q0 += 32) {
+                                const bool on = q0 + lane < len;
+                                const float4 e = on ? sE[at + q0 + lane]
+                                                    : make_float4(-BATS_INF, 0.0f, 0.0f, __int_as_float(-1));
+                                const int c = __float_as_int(e.w);
+                                // A channel's events are neighbours: `run` of them from its first lane on.
+                                const int c_before = __shfl_up_sync(0xffffffffu, c, 1);
+                                const bool head = lane == 0 || c != c_before;
+                                const unsigned later = __ballot_sync(0xffffffffu, head) & ~(lanemask_lt() * 2u + 1u);
+                                const int run = head && on ? (later ? __ffs(later) - 1 : 32) - lane : 0;
+                                const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)run);
+                                const int row = on ? c : 0;
+                                float acc = 0.0f, open[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // open subtrees of 1, 2, 4 and 8 leaves
+                                unsigned todo = mine;
+                                int leaf = __ffs(todo) - 1;  // the leaf of acc
+                                load(UNIT * p + leaf);
+                                while (todo) {
+                                    const int i_leaf = __ffs(todo) - 1;
+                                    todo &= todo - 1u;
+                                    const float t_cur = t_row, a_cur = a_row, b_cur = b_row;
+                                    const int n = n_row, pn = pn_row, at_tap = leaf_tap(i_leaf) * C + row;
+                                    if (todo) load(UNIT * p + __ffs(todo) - 1);
+                                    // The event's place among the spikes: place = #{k : t_k <= t}.
+                                    float A, B;
+                                    bool valid;
+                                    if (ROWS) {
+                                        int last = -1;  // place - 1
 #pragma unroll
-                                for (int step = TOP; step > 0; step >>= 1) {
-                                    const float tk = __shfl_sync(0xffffffffu, t_cur, last + step);
-                                    if (tk <= e.x) last += step;
+                                        for (int step = TOP; step > 0; step >>= 1) {
+                                            if (step > 2 && n < step) continue;  // uniform
+                                            const float tk = __shfl_sync(0xffffffffu, t_cur, last + step);
+                                            if (tk <= e.x) last += step;
+                                        }
+                                        if (TOP == 16 && K == 32) {  // the 32nd spike
+                                            const float t31 = __shfl_sync(0xffffffffu, t_cur, 31);
+                                            last += last == 30 && t31 <= e.x ? 1 : 0;
+                                        }
+                                        A = __shfl_sync(0xffffffffu, a_cur, last + 1);
+                                        B = __shfl_sync(0xffffffffu, b_cur, last + 1);
+                                        valid = on && last + 1 < n;
+                                    } else {
+                                        const long long r = pn_s + pn;
+                                        const int place = post_position(post_t + r * K, n, e.x);
+                                        const float2 ab =
+                                            place < n ? __ldg(tab + r * (K + 1) + place) : make_float2(0.0f, 0.0f);
+                                        A = ab.x;
+                                        B = ab.y;
+                                        valid = on && place < n;
+                                    }
+                                    sval[lane] = valid ? fmaf(e.y, A, -(e.z * B)) : 0.0f;
+                                    if (PRE) {
+                                        const float term =
+                                            valid ? Wk[at_tap] * (A * e.y * inv_tau_s - B * e.z * inv_tau) : 0.0f;
+                                        if (few) {  // one or two leaves: no order
+                                            acc += term;
+                                        } else {    // close the subtrees that end before this leaf
+                                            const int up = 31 - __clz(leaf ^ i_leaf);
+                                            if (up <= 0) {
+                                                open[0] = acc;
+                                            } else {
+                                                acc += open[0];
+                                                open[0] = 0.0f;
+                                                if (up == 1) {
+                                                    open[1] = acc;
+                                                } else {
+                                                    acc += open[1];
+                                                    open[1] = 0.0f;
+                                                    if (up == 2) {
+                                                        open[2] = acc;
+                                                    } else {
+                                                        acc += open[2];
+                                                        open[2] = 0.0f;
+                                                        open[3] = acc;
+                                                    }
+                                                }
+                                            }
+                                            leaf = i_leaf;
+                                            acc = term;
+                                        }
+                                    }
+                                    __syncwarp();
+                                    // The channels' terms in time order.
+                                    float g_sum = run ? Gs[at_tap] : 0.0f;
+#pragma unroll 4
+                                    for (int r = 0; r < longest; ++r)
+                                        if (r < run) g_sum += sval[lane + r];
+                                    if (run) Gs[at_tap] = g_sum;
+                                    __syncwarp();
                                 }
-                                if (TOP == 16 && K == 32) {  // the 32nd spike
-                                    const float t31 = __shfl_sync(0xffffffffu, t_cur, 31);
-                                    last += last == 30 && t31 <= e.x ? 1 : 0;
-                                }
-                                A = __shfl_sync(0xffffffffu, a_cur, last + 1);
-                                B = __shfl_sync(0xffffffffu, b_cur, last + 1);
-                                valid = on && last + 1 < n;
-                            } else {
-                                const long long r = pn_s + pn;
-                                const int p = post_position(post_t + r * K, n, e.x);
-                                const float2 ab = p < n ? __ldg(tab + r * (K + 1) + p) : make_float2(0.0f, 0.0f);
-                                A = ab.x;
-                                B = ab.y;
-                                valid = on && p < n;
-                            }
-                            float v = valid ? fmaf(e.y, A, -(e.z * B)) : 0.0f;
-                            if (PRE) {
-                                const float w = w_lane[W_SMEM ? b * C : __shfl_sync(0xffffffffu, wbase, b)];
-                                const float term = A * f1 - B * f2;
-                                if (valid) acc = fmaf(w, term, acc);
-                            }
-                            // The channel's terms meet on its first lane.
+                                if (PRE && !few) {
 #pragma unroll
-                            for (int m = 0; m < 5; ++m) {
-                                if (longest <= (1 << m)) break;
-                                const float vn = __shfl_sync(0xffffffffu, v, link[m] & 31);
-                                if (link[m] < 32) v += vn;
+                                    for (int m = 0; m < 4; ++m) acc += open[m];
+                                }
+                                if (PRE && on) sred[(at + q0 + lane) * red_ld + u] = acc;
                             }
-                            if (head) g_lane[b * C] += v;
                         }
-                        if (PRE && on) sred[(at + q0 + lane) * red_ld + warp] = acc;
                     }
-                    at += len;
                 }
                 __syncthreads();
                 if (PRE)
                     for (int q = tid; q < cnt; q += blockDim.x) {
+                        const float* row = sred + q * red_ld;
                         float acc = 0.0f;
-                        for (int w = 0; w < nwarps; ++w) acc += sred[q * red_ld + w];
+                        for (int w = 0; w < tiles; ++w, row += UNITS) acc += row[0] + row[1];
                         pre_err[(long long)s * pre_slots + sslot[q]] = acc;
                     }
                 __syncthreads();  // the next batch's staging overwrites sE and sslot
@@ -723,14 +756,12 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
         }
     }
     cluster.sync();
-    const int per = (total + ranks - 1) / ranks;
+    const int per = (total + CONV_BWD_CLUSTER - 1) / CONV_BWD_CLUSTER;
     const int q_end = min(total, (rank + 1) * per);
     for (int q = rank * per + tid; q < q_end; q += blockDim.x) {
         float acc = 0.0f;
-        for (int r = 0; r < ranks; ++r) acc += cluster.map_shared_rank(Gs, r)[q];
-        const int tp = q / C, c = q - tp * C;
-        const int oc = tp % sh.C_out, od = tp / sh.C_out;
-        grad[(long long)blockIdx.y * total + ((long long)oc * sh.fx * sh.fy + od) * C + c] = acc;
+        for (int r = 0; r < CONV_BWD_CLUSTER; ++r) acc += cluster.map_shared_rank(Gs, r)[q];
+        grad[(long long)blockIdx.y * total + q] = acc;
     }
     cluster.sync();
 }
@@ -917,10 +948,10 @@ extern "C" int bats_conv_backward(const void* events, const int* ev_slot, const 
 
 // Shared memory of conv_backward_grouped_kernel: the gradient copy always, the filters where they fit beside it, and the
 // largest batch of events that the rest holds (at least 32).
-static size_t conv_grouped_smem(long long taps, int C, int batch_ev, bool w) {
-    const size_t warps = (size_t)(taps + 31) / 32;
-    return (size_t)batch_ev * (sizeof(float4) + sizeof(float) * (warps | 1) + sizeof(int)) + (size_t)C * sizeof(int) +
-           (size_t)taps * C * sizeof(float) * (w ? 2 : 1);
+static size_t conv_grouped_smem(long long taps, int C, int batch_ev, bool pre, bool w) {
+    const size_t units = (size_t)(taps + 31) / 32 * (32 / bats::CONV_BWD_UNIT);
+    return (size_t)batch_ev * (sizeof(float4) + 2 * sizeof(int) + (pre ? sizeof(float) * (units | 1) : 0)) +
+           std::min<size_t>(32, units) * 32 * sizeof(float) + (size_t)C * sizeof(int) + (size_t)taps * C * sizeof(float) * (w ? 2 : 1);
 }
 
 template <bool PRE, bool W_SMEM>
@@ -931,37 +962,6 @@ static auto* conv_grouped_kernel(int k_post) {
                           : bats::conv_backward_grouped_kernel<true, 4, PRE, W_SMEM>;
 }
 
-// A step coprime to n near n times the golden ratio's fraction: multiples of it visit 0 .. n - 1 in a scattered order.
-static int scatter_step(int n) {
-    for (int s = std::max(1, (int)(0.618 * n));; ++s) {
-        int a = s, b = n;
-        while (b) {
-            const int r = a % b;
-            a = b;
-            b = r;
-        }
-        if (a == 1) return s;
-    }
-}
-
-// CTAs per sample group (the cluster size, 1 to 8): the one that leaves the least of the GPU idle in its last wave, the
-// smaller of equals. per_sm: CTAs of this size an SM holds; clusters of 8 find room on about 128 of the 152 SMs (they
-// lie within one GPC). 64 groups of 1024 threads: 2 (128 CTAs in one wave; 512 CTAs of clusters of 8 took four).
-static int conv_bwd_ranks(int groups, int threads, size_t smem) {
-    const long long per_sm = std::max<long long>(1, std::min<long long>(1024 / threads, 228 * 1024 / (long long)(smem + 4096)));
-    int best = 1;
-    double best_use = 0.0;
-    for (int r = 1; r <= bats::CONV_BWD_CLUSTER; r *= 2) {
-        const long long ctas = (long long)groups * r, slots = per_sm * (r == 8 ? 128 : 152);
-        const double use = (double)ctas / (double)((ctas + slots - 1) / slots * slots) * (r == 8 ? 128.0 / 152 : 1.0);
-        if (use > best_use * 1.02) {
-            best_use = use;
-            best = r;
-        }
-    }
-    return best;
-}
-
 static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* bucket_offsets, long long ev_cap,
                                        const float* weights, const bats::ConvBwdShape& sh, const float* post_times,
                                        const void* tables, const int* nvalid, float tau_s, float tau,
@@ -969,32 +969,32 @@ static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* b
                                        cudaStream_t stream) {
     const long long taps = (long long)sh.C_out * sh.fx * sh.fy;
     constexpr size_t LIMIT = 224 * 1024;
-    const bool w = pre_errors && conv_grouped_smem(taps, sh.C, 64, true) <= LIMIT;
+    const bool pre = pre_errors != nullptr, w = pre && conv_grouped_smem(taps, sh.C, 64, pre, true) <= LIMIT;
     int batch_ev = 512;
-    while (batch_ev > 32 && conv_grouped_smem(taps, sh.C, batch_ev, w) > LIMIT) batch_ev /= 2;
-    const size_t smem = conv_grouped_smem(taps, sh.C, batch_ev, w);
+    while (batch_ev > 32 && conv_grouped_smem(taps, sh.C, batch_ev, pre, w) > LIMIT) batch_ev -= 32;
+    const size_t smem = conv_grouped_smem(taps, sh.C, batch_ev, pre, w);
     auto* kernel = !pre_errors ? conv_grouped_kernel<false, false>(sh.k_post)
                    : w         ? conv_grouped_kernel<true, true>(sh.k_post)
                                : conv_grouped_kernel<true, false>(sh.k_post);
     cudaError_t e = (cudaError_t)bats::max_dynamic_smem_set((const void*)kernel, (int)smem);
     if (e != cudaSuccess) return e;
-    const int groups = (batch + group - 1) / group, threads = (int)(((taps + 31) / 32) * 32);
-    const int ranks = conv_bwd_ranks(groups, threads, smem);
+    const int groups = (batch + group - 1) / group;
+    const int threads = (int)std::min<long long>(1024, (taps + 31) / 32 * (32 / bats::CONV_BWD_UNIT) * 32);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ranks, groups);
+    cfg.gridDim = dim3(bats::CONV_BWD_CLUSTER, groups);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ranks;
+    attr[0].val.clusterDim.x = bats::CONV_BWD_CLUSTER;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1 + (unsigned)bats::pdl_attribute(attr + 1);
     return cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const bats::Event*>(events_bucketed), bucket_offsets, ev_cap,
                               weights, sh, post_times, reinterpret_cast<const float2*>(tables), nvalid, tau_s, tau,
-                              pre_slots, grad, pre_errors, batch, group, batch_ev, scatter_step(sh.n_pos));
+                              pre_slots, grad, pre_errors, batch, group, batch_ev);
 }
 
 extern "C" int bats_conv_backward_grouped(const void* events_bucketed, const int* bucket_offsets, long long ev_cap,
