@@ -680,7 +680,8 @@ static int forward_fc_impl(const void* events, const int* ev_count, long long ev
     BATS_REQUIRE(((uintptr_t)weights_t & 15) == 0 && ((uintptr_t)events & 15) == 0, BATS_ERR_BAD_SHAPE,
                  "lif_forward_fc: weights_t and events must be 16-byte aligned");
     const bats::SolveConst sk = bats::make_solve_const(c, delta_theta_tau, tau, max_simulation);
-    if (algo == BATS_FWD_AUTO)
+    const bool pick = algo == BATS_FWD_AUTO;
+    if (pick)
         algo = bats_lif_forward_fc_default_algo(batch, n_post, (int)(ev_cap < (1LL << 30) ? ev_cap : (1LL << 30)));
     if (algo == BATS_FWD_LANES)
         return bats::launch_forward_lanes<4>(events, ev_count, ev_cap, weights_t, ld, batch, n_post, k_post, sk,
@@ -696,6 +697,13 @@ static int forward_fc_impl(const void* events, const int* ev_count, long long ev
     if (n_post <= 64)
         return bats::launch_tile<64, 16, 6>(screen, events, ev_count, ev_cap, weights_t, ld, batch, n_post, k_post, sk,
                                               n_spikes, a, x, times, post_exp_tau, status, pad, stream);
+    // 64-neuron tiles with 8-event stages where 128-neuron tiles would be filled less than 1 / 1.15 as well, up to about 20
+    // CTAs per SM (300 neurons, 256 samples, 150 / 800 events: 92 against 113 us, 237 against 279; 131 neurons, 128 samples, 3500
+    // events: 0.9 of the time; 131 neurons, 1024 samples, above the line: 135 / 144, 467 / 449).
+    const long long w64 = (n_post + 63) / 64, w128 = 2 * ((n_post + 127) / 128);
+    if (pick && 100 * w128 >= 115 * w64 && w64 * batch <= 152 * 20)
+        return bats::launch_tile<64, 8, 6>(screen, events, ev_count, ev_cap, weights_t, ld, batch, n_post, k_post, sk,
+                                             n_spikes, a, x, times, post_exp_tau, status, pad, stream);
     // 8-event stages: half the shared memory of 16-event stages, so 7 CTAs (28 consumer warps) fit on an SM
     // instead of 4, and a replay after a possible crossing covers fewer events.
     return bats::launch_tile<128, 8, 6>(screen, events, ev_count, ev_cap, weights_t, ld, batch, n_post, k_post, sk,
@@ -704,10 +712,17 @@ static int forward_fc_impl(const void* events, const int* ev_count, long long ev
 
 extern "C" int bats_lif_forward_fc_default_algo(int batch, int n_post, int ev_cap) {
     (void)ev_cap;
-    // Warp per (sample, neuron) when that gives fewer warps than about four per SM sub-partition of a
-    // 152-SM GPU, or the layer has so few neurons that the tile kernel would idle most of its lanes.
+    // Warp per (sample, neuron): its time grows with the number of warps, that of the tile kernel with the number of tiles
+    // and, below about a wave, with nothing. The lines are where both meet, per sub-partition of a 152-SM GPU; measured
+    // with input lists of 150 / 800 / 3500 events, lanes against tile in us:
+    //   at most 8 neurons (three quarters of a tile idle): always (4 neurons, 4096 samples: 199 / 343)
+    //   at most 16: 20 warps (12 neurons, 1024 samples 66 / 74, 168 / 164; 16 and 4096: 715 / 433, above the line)
+    //   at most 32: 16 warps (32 neurons, 256 samples: 50 / 87, 118 / 148, 259 / 363; 512 samples: 214 / 160, above)
+    //   wider: 8 warps (131 neurons, 32 samples: 31 / 64, 70 / 156, 136 / 388; silent layers 15 / 21, 44 / 58; twice as
+    //   many warps are still faster where the neurons spike, 52 / 70, 120 / 158, but not where they are silent, 79 / 58)
     const long long warps = (long long)batch * n_post;
-    return (n_post <= 16 || warps <= 152LL * 4 * 4) ? BATS_FWD_LANES : BATS_FWD_TILE;
+    const long long per_sub = n_post <= 8 ? warps : n_post <= 16 ? 20 : n_post <= 32 ? 16 : 8;
+    return warps <= 152LL * 4 * per_sub ? BATS_FWD_LANES : BATS_FWD_TILE;
 }
 
 extern "C" int bats_lif_forward_fc(const void* events, const int* ev_count, long long ev_cap, const float* weights_t,

@@ -118,7 +118,8 @@ int bats_intensity_to_spike_times(const unsigned char* pixels, int batch, int n_
  * producer warp streaming weight rows (throughput-oriented, large B * N_post); BATS_FWD_LANES runs one warp
  * per (sample, post neuron) with 32 events evaluated in parallel (latency-oriented: few neurons, small
  * batches, long event streams). Both give bit-identical results. BATS_FWD_AUTO picks by
- * bats_lif_forward_fc_default_algo. No counterpart in the reference (it has one kernel shape). */
+ * bats_lif_forward_fc_default_algo, and among the tile widths by how well N_post fills them. No counterpart in
+ * the reference (it has one kernel shape). */
 #define BATS_FWD_AUTO 0
 #define BATS_FWD_TILE 1
 #define BATS_FWD_LANES 2
