@@ -222,11 +222,16 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
 // Layer-path prep given the forward's spike counts: only each neuron's leading min(n_spikes, K) slots
 // are read (the forward writes +inf past them), so silent slots cost nothing. A warp handles 32 neurons
 // and stages their valid slots compactly in shared memory (at most PREPC_CAP per round; a round takes
-// the next lanes whose slots fit), then each lane runs bwd_prep_layer_kernel's arithmetic on its
-// neuron, so errors, tables and counts are identical to it (n = the first +inf time below the count,
-// or the count).
-constexpr int PREPC_WARPS = 4;
-constexpr int PREPC_CAP = 256;
+// the next lanes whose slots fit). The reset errors are a lane's serial chain over its neuron's spikes; the factors and the
+// suffix sums, which differ most in length between neurons, are one lane per slot. The arithmetic per neuron is
+// bwd_prep_layer_kernel's in its order, so errors, tables and counts are identical to it (n = the first +inf time below the
+// count, or the count).
+// What bounds it: the sectors of the scattered rows (a row of K slots per neuron and array, mostly one or two of them valid).
+// With whole neurons per lane 220 M warp instructions went into 1024 neurons x 4096 samples of 1642 spikes, at 9 of 32 lanes:
+// 365 -> 255 us (140 M); 800 neurons, 256 samples, 3510 spikes: 54 -> 40 us. Rounds of 128 slots (half the shared
+// memory, twice the warps) against 256: 255 / 335 and 41 / 40 us.
+constexpr int PREPC_WARPS = 8;
+constexpr int PREPC_CAP = 128;
 
 struct PrepCompact {
     float t[PREPC_CAP], z[PREPC_CAP], x[PREPC_CAP], a[PREPC_CAP], e[PREPC_CAP];
@@ -283,72 +288,59 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
         int n = 0;
         float h_t0 = BATS_INF, h_t1 = BATS_INF;  // the cursor head's spike times (read before the tables overwrite them)
         if (mine) {
-            float* rt = sm.t + off;
-            float* rz = sm.z + off;
-            float* rx = sm.x + off;
-            float* ra = sm.a + off;
-            float* re = sm.e + off;
             n = n_in;
             for (int k = 0; k < n_in; ++k)
-                if (isinf(rt[k])) {
+                if (isinf(sm.t[off + k])) {
                     n = k;
                     break;
                 }
-            h_t0 = n > 0 ? rt[0] : BATS_INF;
-            h_t1 = n > 1 ? rt[1] : BATS_INF;
+            h_t0 = n > 0 ? sm.t[off] : BATS_INF;
+            h_t1 = n > 1 ? sm.t[off + 1] : BATS_INF;
             float cum = 0.0f;
             for (int k = n - 1; k >= 0; --k) {
-                const float ek = re[k] + cum * rz[k];
-                re[k] = ek;
-                cum += ek * dtt / rx[k];
-            }
-            for (int k = 0; k < n; ++k) {
-                const float xk = rx[k];
-                ra[k] = tau / ra[k] * (1 + rz[k] * c / xk);
-                rz[k] = tau / xk;
-            }
-            for (int p0 = 0; p0 < n; p0 += 4) {
-                float sa[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                for (int k = p0; k < n; ++k) {
-                    const float ek = re[k], fa = ra[k], fb = rz[k];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if (k >= p0 + u) {
-                            sa[u] += ek * fa;
-                            sb[u] += ek * fb;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (p0 + u < n) {
-                        rt[p0 + u] = sa[u];
-                        rx[p0 + u] = sb[u];
-                    }
-                }
-            }
-        }
-        if (mine && lane < cnt) {
-            nvalid[nb + lane] = n;
-            if (head_t) {
-                // Cursor head: what PostCursor::init reads from this row, in one coalesced record per pair.
-                const float* ra = sm.t + off;
-                const float* rb = sm.x + off;
-                head_t[nb + lane] = make_float2(h_t0, h_t1);
-                head_ab[nb + lane] = make_float4(n > 0 ? ra[0] : 0.0f, n > 0 ? rb[0] : 0.0f, n > 1 ? ra[1] : 0.0f,
-                                                 n > 1 ? rb[1] : 0.0f);
+                const float ek = sm.e[off + k] + cum * sm.z[off + k];
+                sm.e[off + k] = ek;
+                cum += ek * dtt / sm.x[off + k];
             }
         }
         __syncwarp();
+        // Factors: a lane per slot (they replace a and z).
+        for (int q = lane; q < V; q += 32) {
+            const float xk = sm.x[q];
+            sm.a[q] = tau / sm.a[q] * (1 + sm.z[q] * c / xk);
+            sm.z[q] = tau / xk;
+        }
+        __syncwarp();
+        // Tables: a lane per entry p of a neuron, its sums upwards from k = p; the first two entries also into (t, x), for
+        // the head.
         for (int q0 = 0; q0 < V; q0 += 32) {
             const int q = q0 + lane;
             const int r = q < V ? sm.owner[q] : 0;
             const int ro = __shfl_sync(0xffffffffu, excl, r) - base;
             const int nr = __shfl_sync(0xffffffffu, n, r);
-            const int k = q - ro;
-            if (q < V && k < nr) {
-                err[(nb + r) * K + k] = sm.e[q];
-                tab[(nb + r) * K1 + k] = make_float2(sm.t[q], sm.x[q]);
+            const int p = q - ro;
+            if (q < V && p < nr) {
+                float sa = 0.0f, sb = 0.0f;
+                for (int k = q; k < ro + nr; ++k) {
+                    const float ek = sm.e[k];
+                    sa += ek * sm.a[k];
+                    sb += ek * sm.z[k];
+                }
+                err[(nb + r) * K + p] = sm.e[q];
+                tab[(nb + r) * K1 + p] = make_float2(sa, sb);
+                if (p < 2) {
+                    sm.t[q] = sa;
+                    sm.x[q] = sb;
+                }
+            }
+        }
+        __syncwarp();
+        if (mine && lane < cnt) {
+            nvalid[nb + lane] = n;
+            if (head_t) {
+                head_t[nb + lane] = make_float2(h_t0, h_t1);
+                head_ab[nb + lane] = make_float4(n > 0 ? sm.t[off] : 0.0f, n > 0 ? sm.x[off] : 0.0f,
+                                                 n > 1 ? sm.t[off + 1] : 0.0f, n > 1 ? sm.x[off + 1] : 0.0f);
             }
         }
         __syncwarp();
@@ -554,12 +546,12 @@ bwd_grad_narrow_kernel(const Event* __restrict__ ev_b, const int* __restrict__ b
     pdl_prologue();
     constexpr int JC = 32;
     __shared__ float G[JC][33];
-    __shared__ Event sev[GRAD_NARROW_WARPS][64];
+    extern __shared__ __align__(16) Event gn_events[];  // 64 per warp
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     const bool active = lane < n_post;
     const int bucket = blockIdx.y, J0 = bucket * JC, g = blockIdx.z;
     for (int jj = warp; jj < JC; jj += warps) G[jj][lane] = 0.0f;  // the warp's own rows: no other warp touches them
-    Event* wev = sev[warp];
+    Event* wev = gn_events + warp * 64;
     const int s_begin = g * group, s_end = min(batch, s_begin + group);
     bool worked = false;  // uniform over the CTA: some sample had events in the bucket and a spike
     for (int s0 = s_begin; s0 < s_end; s0 += 32) {
@@ -1065,7 +1057,7 @@ static cudaError_t launch_grad(const void* events, const int* ev_count, const vo
             // little (0.59 against 0.66 ms); two are slower in both (85 us, 0.77 ms).
             int warps = 1;
             while (warps < bats::GRAD_NARROW_WARPS && (long long)grid.y * grid.z * warps < 16 * 152) warps *= 2;
-            return bats::launch(bats::bwd_grad_narrow_kernel, grid, 32 * warps, 0, stream,
+            return bats::launch(bats::bwd_grad_narrow_kernel, grid, 32 * warps, warps * 64 * sizeof(bats::Event), stream,
                                 reinterpret_cast<const bats::Event*>(ev_b), boff, n_buckets, ev_cap, post_times,
                                 reinterpret_cast<const float2*>(tables), nvalid, n_post, k_post, n_pre, batch, group, out,
                                 flags, (const float2*)h.t, (const float4*)h.ab);
