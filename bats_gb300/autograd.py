@@ -38,8 +38,11 @@ class _LIFFunction(torch.autograd.Function):
         tau_s, tau, c, dtt = ctx.consts
         if grad_t is None:
             return None, None, None, None, None, None, None
-        errors = torch.where(torch.isinf(t), torch.zeros_like(grad_t), grad_t).contiguous().float().clone()
-        tabs = K.backward_prep(t, a, x, z, errors, c, tau, dtt)
+        if t.shape[2] <= 32:  # the gradient past the spikes is not read, and the reset errors are not written
+            tabs = K.backward_prep(t, a, x, z, grad_t.contiguous().float(), c, tau, dtt, keep_errors=True)
+        else:
+            errors = torch.where(torch.isinf(t), torch.zeros_like(grad_t), grad_t).contiguous().float().clone()
+            tabs = K.backward_prep(t, a, x, z, errors, c, tau, dtt)
         grad_w = None
         if ctx.needs_input_grad[1]:
             grad_w = K.weights_gradient(ctx.ev, t, tabs, ctx.n_pre, per_sample=False, reduce="sum")

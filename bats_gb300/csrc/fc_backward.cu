@@ -225,11 +225,13 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
 // the next lanes whose slots fit). The reset errors are a lane's serial chain over its neuron's spikes; the factors and the
 // suffix sums, which differ most in length between neurons, are one lane per slot. The arithmetic per neuron is
 // bwd_prep_layer_kernel's in its order, so errors, tables and counts are identical to it (n = the first +inf time below the
-// count, or the count).
+// count, or the count). Without n_spikes the count is the slots before a row's first +inf; without err_out the reset errors
+// stay in shared memory (err may be err_out).
 // What bounds it: the sectors of the scattered rows (a row of K slots per neuron and array, mostly one or two of them valid).
 // With whole neurons per lane 220 M warp instructions went into 1024 neurons x 4096 samples of 1642 spikes, at 9 of 32 lanes:
 // 365 -> 255 us (140 M); 800 neurons, 256 samples, 3510 spikes: 54 -> 40 us. Rounds of 128 slots (half the shared
 // memory, twice the warps) against 256: 255 / 335 and 41 / 40 us.
+// Without counts 475 k spikes of 300 neurons, 256 samples: 64 us with whole rows of K slots staged (ten warps an SM) -> 54 us.
 constexpr int PREPC_WARPS = 8;
 constexpr int PREPC_CAP = 128;
 
@@ -240,18 +242,27 @@ struct PrepCompact {
 
 __global__ void __launch_bounds__(PREPC_WARPS * 32)
 bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_spikes, const float* __restrict__ a,
-                        const float* __restrict__ x, const float* __restrict__ z, float* __restrict__ err,
+                        const float* __restrict__ x, const float* __restrict__ z, const float* err, float* err_out,
                         long long total, int K, float c, float tau, float dtt, float2* __restrict__ tab,
                         int* __restrict__ nvalid, float2* __restrict__ head_t, float4* __restrict__ head_ab) {
     pdl_prologue();
     __shared__ PrepCompact sm_all[PREPC_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     PrepCompact& sm = sm_all[warp];
-    const long long nb = ((long long)blockIdx.x * PREPC_WARPS + warp) * 32;
+    const long long nb = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * 32;
     if (nb >= total) return;
     const int cnt = (int)min(32LL, total - nb);
     const int K1 = K + 1;
-    const int n_in = lane < cnt ? min(max(n_spikes[nb + lane], 0), K) : 0;
+    int n_in = 0;
+    if (n_spikes) {
+        n_in = lane < cnt ? min(max(n_spikes[nb + lane], 0), K) : 0;
+    } else {  // the slots before the first +inf, a row on the lanes (K <= 32)
+#pragma unroll 16
+        for (int r = 0; r < cnt; ++r) {
+            const unsigned silent = __ballot_sync(0xffffffffu, lane >= K || isinf(t[(nb + r) * K + lane]));
+            if (lane == r) n_in = silent ? __ffs(silent) - 1 : 32;
+        }
+    }
     // Inclusive prefix of the counts over the warp's lanes.
     int incl = n_in;
 #pragma unroll
@@ -326,7 +337,7 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
                     sa += ek * sm.a[k];
                     sb += ek * sm.z[k];
                 }
-                err[(nb + r) * K + p] = sm.e[q];
+                if (err_out) err_out[(nb + r) * K + p] = sm.e[q];
                 tab[(nb + r) * K1 + p] = make_float2(sa, sb);
                 if (p < 2) {
                     sm.t[q] = sa;
@@ -951,6 +962,34 @@ extern "C" int bats_backward_prep(const float* post_times, const float* a, const
     return BATS_OK;
 }
 
+// Cursor heads of `pairs` (sample, neuron) pairs: the first two spike times (float2 per pair), then, from the
+// next 16-byte boundary, the first two suffix-table entries (float4 per pair).
+struct CursorHeads {
+    float2* t;
+    float4* ab;
+};
+static size_t heads_times_bytes(long long pairs) { return ((size_t)pairs * sizeof(float2) + 15) & ~(size_t)15; }
+static CursorHeads cursor_heads_of(const void* base, long long pairs) {
+    if (!base) return {nullptr, nullptr};
+    char* b = static_cast<char*>(const_cast<void*>(base));
+    return {reinterpret_cast<float2*>(b), reinterpret_cast<float4*>(b + heads_times_bytes(pairs))};
+}
+
+static int launch_prep_counted(const float* post_times, const int* n_spikes, const float* a, const float* x,
+                               const float* post_exp_tau, const float* errors, float* errors_out, long long total,
+                               int k_post, float c, float tau, float delta_theta_tau, void* tables, int* nvalid,
+                               void* cursor_heads, cudaStream_t stream) {
+    const long long warps = (total + 31) / 32;
+    const int per = warps < 152 * 8 ? 1 : bats::PREPC_WARPS;  // a layer of few warps goes to as many SMs as it can
+    const int blocks = (int)((warps + per - 1) / per);
+    const CursorHeads h = cursor_heads_of(cursor_heads, total);
+    BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel, blocks, per * 32, 0, stream, post_times,
+        n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
+        reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab));
+    BATS_CUDA(cudaGetLastError());
+    return BATS_OK;
+}
+
 extern "C" int bats_backward_prep_layer(const float* post_times, const float* a, const float* x,
                                         const float* post_exp_tau, float* errors, int batch, int n_post, int k_post,
                                         float c, float tau, float delta_theta_tau, float* f1, float* f2, void* tables,
@@ -966,6 +1005,9 @@ extern "C" int bats_backward_prep_layer(const float* post_times, const float* a,
         return bats_backward_prep(post_times, a, x, post_exp_tau, errors, batch, n_post, k_post, c, tau,
                                   delta_theta_tau, 1, 1, f1, f2, tables, nvalid, stream);
     }
+    if (!f1)
+        return launch_prep_counted(post_times, nullptr, a, x, post_exp_tau, errors, errors, total, k_post, c, tau,
+                                   delta_theta_tau, tables, nvalid, nullptr, stream);
     const long long warps = (total + 31) / 32;
     const int blocks = (int)((warps + bats::PREP_WARPS - 1) / bats::PREP_WARPS);
     const size_t smem = (size_t)bats::PREP_WARPS * 5 * 32 * bats::PREP_KS * sizeof(float);
@@ -977,18 +1019,6 @@ extern "C" int bats_backward_prep_layer(const float* post_times, const float* a,
     return BATS_OK;
 }
 
-// Cursor heads of `pairs` (sample, neuron) pairs: the first two spike times (float2 per pair), then, from the
-// next 16-byte boundary, the first two suffix-table entries (float4 per pair).
-struct CursorHeads {
-    float2* t;
-    float4* ab;
-};
-static size_t heads_times_bytes(long long pairs) { return ((size_t)pairs * sizeof(float2) + 15) & ~(size_t)15; }
-static CursorHeads cursor_heads_of(const void* base, long long pairs) {
-    if (!base) return {nullptr, nullptr};
-    char* b = static_cast<char*>(const_cast<void*>(base));
-    return {reinterpret_cast<float2*>(b), reinterpret_cast<float4*>(b + heads_times_bytes(pairs))};
-}
 extern "C" size_t bats_cursor_heads_bytes(int batch, int n_post) {
     const long long pairs = (long long)std::max(batch, 0) * std::max(n_post, 0);
     return heads_times_bytes(pairs) + (size_t)pairs * sizeof(float4);
@@ -1006,14 +1036,24 @@ extern "C" int bats_backward_prep_counted(const float* post_times, const int* n_
     if (total == 0) return BATS_OK;
     BATS_REQUIRE(post_times && n_spikes && a && x && post_exp_tau && errors && tables && nvalid, BATS_ERR_NULL,
                  "backward_prep_counted: null pointer");
-    const long long warps = (total + 31) / 32;
-    const int blocks = (int)((warps + bats::PREPC_WARPS - 1) / bats::PREPC_WARPS);
-    const CursorHeads h = cursor_heads_of(cursor_heads, total);
-    BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel, blocks, bats::PREPC_WARPS * 32, 0, stream, post_times,
-        n_spikes, a, x, post_exp_tau, errors, total, k_post, c, tau, delta_theta_tau, reinterpret_cast<float2*>(tables),
-        nvalid, h.t, h.ab));
-    BATS_CUDA(cudaGetLastError());
-    return BATS_OK;
+    return launch_prep_counted(post_times, n_spikes, a, x, post_exp_tau, errors, errors, total, k_post, c, tau,
+                               delta_theta_tau, tables, nvalid, cursor_heads, stream);
+}
+
+extern "C" int bats_backward_prep_readonly(const float* post_times, const float* a, const float* x,
+                                           const float* post_exp_tau, const float* errors, int batch, int n_post,
+                                           int k_post, float c, float tau, float delta_theta_tau, void* tables,
+                                           int* nvalid, void* cursor_heads, cudaStream_t stream) {
+    BATS_REQUIRE(batch >= 0 && n_post >= 0 && k_post > 0, BATS_ERR_BAD_SHAPE, "backward_prep_readonly: bad shape");
+    BATS_REQUIRE(((uintptr_t)cursor_heads & 15) == 0, BATS_ERR_BAD_SHAPE,
+                 "backward_prep_readonly: cursor_heads not 16-byte aligned");
+    BATS_REQUIRE(k_post <= 32, BATS_ERR_BAD_SHAPE, "backward_prep_readonly: k_post > 32 (use bats_backward_prep_layer)");
+    const long long total = (long long)batch * n_post;
+    if (total == 0) return BATS_OK;
+    BATS_REQUIRE(post_times && a && x && post_exp_tau && errors && tables && nvalid, BATS_ERR_NULL,
+                 "backward_prep_readonly: null pointer");
+    return launch_prep_counted(post_times, nullptr, a, x, post_exp_tau, errors, nullptr, total, k_post, c, tau,
+                               delta_theta_tau, tables, nvalid, cursor_heads, stream);
 }
 
 // Post neurons per gradient CTA: two independent warps (the same warps per SM as four, 2.6 % faster on an

@@ -350,15 +350,18 @@ def alloc_cursor_heads(batch: int, n_post: int, device="cuda") -> torch.Tensor:
 
 def backward_prep(post_times, a, x, post_exp_tau, errors, c: float, tau: float, delta_theta_tau: float,
                   recurrent: bool = True, out: BackwardTables | None = None, want_factors: bool = False,
-                  n_spikes=None) -> BackwardTables:
+                  n_spikes=None, keep_errors: bool = False) -> BackwardTables:
     """Reset errors in place + factors + suffix tables (replaces propagate_recurrent_errors and
     compute_factors, Wrappers/Backpropagation/propagate_recurrent_errors.py:9-16, compute_factors.py:11-22).
     For the forward kernels' outputs (the layer path); f1/f2 are only materialised if want_factors. With the
-    forward's spike counts `n_spikes` (B, N) only the slots below them are read."""
+    forward's spike counts `n_spikes` (B, N) only the slots below them are read. With `keep_errors` (K <= 32, no
+    factors) the errors, which may then be a gradient that belongs to the caller, are only read."""
     B, N, K = post_times.shape
     dev = post_times.device
     need_f = want_factors or K > 32 or not recurrent
-    counted = recurrent and n_spikes is not None and not need_f
+    if keep_errors and need_f:
+        raise ValueError("keep_errors: K <= 32, recurrent errors and no factors")
+    counted = recurrent and (n_spikes is not None or keep_errors) and not need_f
     if out is None:
         out = BackwardTables(torch.empty((B, N, K), dtype=F32, device=dev) if need_f else None,
                              torch.empty((B, N, K), dtype=F32, device=dev) if need_f else None,
@@ -367,7 +370,11 @@ def backward_prep(post_times, a, x, post_exp_tau, errors, c: float, tau: float, 
                              alloc_cursor_heads(B, N, dev) if counted else None)
     if not counted:
         out.heads = None  # only the counted prep writes the cursor heads
-    if counted:
+    if keep_errors:
+        call("bats_backward_prep_readonly", ptr(post_times), ptr(a), ptr(x), ptr(post_exp_tau), ptr(errors), B, N, K,
+             float(c), float(tau), float(delta_theta_tau), ptr(out.tables), ptr(out.nvalid), ptr(out.heads),
+             stream_ptr())
+    elif counted:
         call("bats_backward_prep_counted", ptr(post_times), ptr(_c(n_spikes, I32)), ptr(a), ptr(x),
              ptr(post_exp_tau), ptr(errors), B, N, K, float(c), float(tau), float(delta_theta_tau),
              ptr(out.tables), ptr(out.nvalid), ptr(out.heads), stream_ptr())

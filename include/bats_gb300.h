@@ -233,6 +233,12 @@ int bats_backward_prep_counted(const float* post_times, const int* n_spikes, con
                                const float* post_exp_tau, float* errors, int batch, int n_post, int k_post, float c,
                                float tau, float delta_theta_tau, void* tables, int* nvalid, void* cursor_heads,
                                cudaStream_t stream);
+/* The same without spike counts (a neuron's slots end at its first +inf time) and with the errors left as they are: only
+ * the tables, nvalid and cursor_heads are written. For gradients that belong to the caller. */
+int bats_backward_prep_readonly(const float* post_times, const float* a, const float* x, const float* post_exp_tau,
+                                const float* errors, int batch, int n_post, int k_post, float c, float tau,
+                                float delta_theta_tau, void* tables, int* nvalid, void* cursor_heads,
+                                cudaStream_t stream);
 
 /* Weight gradient of a fully-connected layer. group == 1: per-sample gradient (B, N_post, N_pre) like the
  * reference; group > 1: the batch mean (mean != 0) or sum (N_post, N_pre), accumulated per group of samples
