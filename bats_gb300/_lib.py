@@ -176,8 +176,13 @@ def ptr(t) -> int | None:
 
 
 def stream_ptr(stream=None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    """The raw handle of a stream, by default the current device's current one (asked for as a handle: the Stream object of
+    torch.cuda.current_stream() costs 5 us on each of a layer step's sixteen calls)."""
+    if stream is not None:
+        return stream.cuda_stream
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def require_cuda():
