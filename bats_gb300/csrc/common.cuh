@@ -425,9 +425,11 @@ struct PostCursor {
             ++p;
             tn = tn1;
             AB = AB1;
-            const bool more = p + 1 < n;
-            tn1 = more ? tp[p + 1] : BATS_INF;
-            AB1 = more ? tb[p + 1] : make_float2(0.0f, 0.0f);
+            tn1 = BATS_INF;
+            if (p + 1 < n) {
+                tn1 = tp[p + 1];
+                AB1 = tb[p + 1];
+            }
         }
     }
     __device__ __forceinline__ bool valid() const { return p < n; }
