@@ -462,14 +462,17 @@ __global__ void __launch_bounds__(1024) work_order_kernel(const int* __restrict_
 //      (a = fma(w, e^{t/tau_s}, a), b = fma(w, e^{t/tau}, b), event order), every lane running the
 //      same chain over the block's (w, exponentials) in warp-private shared memory and keeping the
 //      state after its own event;
-//   2. every lane evaluates the provable no-crossing test on its own state at once (one ballot);
+//   2. every lane evaluates the provable screen (may_cross, its event's constants formed once) on its own state (one ballot);
 //   3. candidates are taken in event order by their lane with the exact solver; a spike's reset
 //      changes b for the later events of the block, whose b chain is then re-run from the spiking
 //      event (a is unaffected by resets) and whose tests are re-evaluated.
 // The arithmetic per event is that of the reference's loop, so results are bit-identical to the
-// tile kernel's. The warp is latency-bound rather than issue-bound: a 32-event block costs about 230
-// instructions for one neuron, against the tile kernel's ~100 per 32 neurons and event, so the
-// variant pays off when B * N_post is small against the GPU's ~5000 resident warps.
+// tile kernel's. What bounds it: the latency of a block's chain of dependent steps where there are few warps (the loads,
+// hence two blocks ahead), instruction issue where there are many; a 32-event block costs about 230 instructions for one
+// neuron, against the tile kernel's ~100 per 32 neurons and event, so the variant pays off when B * N_post is small against
+// the GPU's ~5000 resident warps. With the event and its weight loaded together one block ahead (the second waiting for the
+// first) and the fuller test: 20 neurons, one sample of 2800 events 60 -> 46 us; 4096 warps of 3600 events 138 -> 117 us; 8192 of
+// 2400: 197 -> 173 us. (Copies into a ring in shared memory four blocks ahead: 50, 138 and 201 us, 20 % more instructions.)
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 lif_fc_forward_lanes_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_count, long long ev_cap,
@@ -477,7 +480,7 @@ lif_fc_forward_lanes_kernel(const Event* __restrict__ ev, const int* __restrict_
                             int* __restrict__ n_spikes, float* __restrict__ a_out, float* __restrict__ x_out,
                             float* __restrict__ t_out, float* __restrict__ z_out, int pad) {
     pdl_prologue();
-    __shared__ float4 blk[WARPS][32];  // (w, es, e, -) of the block's events
+    __shared__ float4 blk[WARPS][32];  // the block's events as (t, w, es, e)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = blockIdx.y;
     const int i = blockIdx.x * WARPS + warp;
@@ -489,44 +492,39 @@ lif_fc_forward_lanes_kernel(const Event* __restrict__ ev, const int* __restrict_
     float* xo = x_out + obase;
     float* to = t_out + obase;
     float* zo = z_out + obase;
-    float4* my = blk[warp];
     float a = 0.0f, b = 0.0f;
     int n = 0;
     bool done = false;
-    // The next block's event and weight are loaded one block ahead, so that the gather latency overlaps
-    // the current block's chain and tests.
-    float4 e4_nx = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float w_nx = 0.0f;
-    if (lane < E) {
-        e4_nx = __ldg(reinterpret_cast<const float4*>(evs + lane));
-        w_nx = __ldg(wt + (long long)__float_as_int(e4_nx.y) * ld + i);
-    }
+    float4* my = blk[warp];
+    // Events in registers two blocks ahead and their weights, whose addresses they hold, one: neither load waits on the other.
+    const Event* ev_from = evs + lane;
+    const float* w_from = wt + i;
+    auto event_at = [&](int m) {
+        return m + lane < E ? __ldg(reinterpret_cast<const float4*>(ev_from + m)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    auto weight_of = [&](const float4& e, int m) {
+        return m + lane < E ? __ldg(w_from + (long long)__float_as_int(e.y) * ld) : 0.0f;
+    };
+    float4 e4_nx = event_at(0), e4_nx2 = event_at(32);
+    float w_nx = weight_of(e4_nx, 0);
     for (int m0 = 0; m0 < E && !done; m0 += 32) {
         const int m = m0 + lane;
         const int cnt = min(32, E - m0);
         const bool in = lane < cnt;
         const float4 e4 = e4_nx;  // (t, j, es, e); zeros past the end
-        const float w = w_nx;
-        e4_nx = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        w_nx = 0.0f;
-        if (m + 32 < E) {
-            e4_nx = __ldg(reinterpret_cast<const float4*>(evs + m + 32));
-            w_nx = __ldg(wt + (long long)__float_as_int(e4_nx.y) * ld + i);
-        }
+        my[lane] = make_float4(e4.x, w_nx, e4.z, e4.w);
+        e4_nx = e4_nx2;
+        w_nx = weight_of(e4_nx, m0 + 32);
+        e4_nx2 = event_at(m0 + 64);
         // Window end: the next event's time and exponential (+inf after the last event).
-        float t_nx = __shfl_down_sync(0xffffffffu, e4.x, 1);
-        float e_nx = __shfl_down_sync(0xffffffffu, e4.w, 1);
-        if (lane == 31 && m0 + 32 < E) {
-            const float4 nx = __ldg(reinterpret_cast<const float4*>(evs + m0 + 32));
-            t_nx = nx.x;
-            e_nx = nx.w;
-        }
+        float t_nx = __shfl_sync(0xffffffffu, lane == 0 ? e4_nx.x : e4.x, lane + 1);
+        float e_nx = __shfl_sync(0xffffffffu, lane == 0 ? e4_nx.w : e4.w, lane + 1);
         if (m + 1 >= E) {
             t_nx = BATS_INF;
             e_nx = BATS_INF;
         }
-        // 1. sequential chain; lanes past the block's end carry w = 0, which leaves a and b unchanged.
-        my[lane] = make_float4(w, e4.z, e4.w, 0.0f);
+        const CrossWindow win = cross_window(e4.z, e4.w, e4.w, e_nx, sk);
+        // 1. sequential chain.
         __syncwarp();
         // Lane l stops after event l: its state is the chain's l-th prefix, with no select per step.
         float am = a, bm = b;
@@ -534,12 +532,12 @@ lif_fc_forward_lanes_kernel(const Event* __restrict__ ev, const int* __restrict_
         for (int k = 0; k < 32; ++k) {
             const float4 q = my[k];
             if (k <= lane) {
-                am = fmaf(q.x, q.y, am);
-                bm = fmaf(q.x, q.z, bm);
+                am = fmaf(q.y, q.z, am);
+                bm = fmaf(q.y, q.w, bm);
             }
         }
         // 2. provable no-crossing tests of all lanes at once.
-        unsigned cand = __ballot_sync(0xffffffffu, in && !no_crossing<false>(am, bm, e4.w, e_nx, sk));
+        unsigned cand = __ballot_sync(0xffffffffu, in && may_cross(am, bm, win, sk));
         // 3. candidates in event order.
         while (cand) {
             const int u = __ffs(cand) - 1;
@@ -547,7 +545,7 @@ lif_fc_forward_lanes_kernel(const Event* __restrict__ ev, const int* __restrict_
             int full = 0;
             if (lane == u) {
                 const int n0 = n;
-                full = solve_crossings<false>(am, bm, e4.x, t_nx, e4.w, e_nx, sk, n, k_post, ao, xo, to, zo) ? 1 : 0;
+                full = solve_candidate<false>(am, bm, e4.x, t_nx, win, sk, n, k_post, 0, ao, xo, to, zo) ? 1 : 0;
                 spiked = n - n0;
             }
             n = __shfl_sync(0xffffffffu, n, u);
@@ -558,12 +556,13 @@ lif_fc_forward_lanes_kernel(const Event* __restrict__ ev, const int* __restrict_
             }
             if (spiked) {
                 float cb2 = __shfl_sync(0xffffffffu, bm, u);
+#pragma unroll 4
                 for (int k = u + 1; k < cnt; ++k) {
                     const float4 q = my[k];
-                    cb2 = fmaf(q.x, q.z, cb2);
-                    bm = (lane == k) ? cb2 : bm;
+                    if (k <= lane) cb2 = fmaf(q.y, q.w, cb2);
                 }
-                cand = __ballot_sync(0xffffffffu, in && lane > u && !no_crossing<false>(am, bm, e4.w, e_nx, sk));
+                bm = lane > u ? cb2 : bm;
+                cand = __ballot_sync(0xffffffffu, in && lane > u && may_cross(am, bm, win, sk));
             } else {
                 cand &= cand - 1u;
             }
