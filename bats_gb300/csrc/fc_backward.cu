@@ -862,8 +862,8 @@ bwd_pre_err_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_coun
 // With few post neurons, one thread per post neuron leaves most lanes idle and the per-sample CTA
 // serial over all events; here lanes take events instead, and every lane runs over the (few) post
 // neurons. The sample's post-spike times, suffix tables and counts are staged in shared memory.
-// (The weight gradient of narrow layers keeps the thread-per-neuron merge of bwd_grad_warp_kernel,
-// which costs a few instructions per event for all neurons at once, with more sample groups instead.)
+// (The weight gradient of narrow layers keeps the thread-per-neuron merge, which costs a few instructions per event for
+// all neurons at once: bwd_grad_narrow_kernel.)
 
 // Shared-memory copy of one sample's post-neuron data: times (N_post, K), tables (N_post, K + 1),
 // counts (N_post), issued as asynchronous copies (cp.async, no register round trip, all in flight at
@@ -879,7 +879,12 @@ __device__ __forceinline__ void stage_post(const float* __restrict__ post_t, con
 }
 
 // Pre-spike errors, thread per event: sum over post neurons i (in order) of w_ij * SA_i(p) and
-// w_ij * SB_i(p), then * e^{t/tau_s}/tau_s and * e^{t/tau}/tau, written to the event's slot.
+// w_ij * SB_i(p), then * e^{t/tau_s}/tau_s and * e^{t/tau}/tau, written to the event's slot. A warp's 32 events are
+// neighbours in time: a lane per neuron looks up its places for the first and the last, and only the neurons that spiked in between
+// are searched per event. Weights are read four neurons at a time.
+// What bounds it: the latency of its loads (a warp of 20 neurons has few instructions left), and setting the slots without an
+// event to 0 before it. With a search per (event, neuron) and a weight per load: 32 neurons, 256 samples 172 -> 72 us; 20 neurons,
+// 4096 samples 298 -> 252 us.
 __global__ void __launch_bounds__(128)
 bwd_pre_err_narrow_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_slot,
                           const int* __restrict__ ev_count, long long ev_cap, const float* __restrict__ wt, int ld,
@@ -897,23 +902,48 @@ bwd_pre_err_narrow_kernel(const Event* __restrict__ ev, const int* __restrict__ 
     stage_post(post_t, tab, nvalid, s, n_post, k_post, st, stab, snv);
     cp_async_wait_all();
     __syncthreads();
-    // The sample's events, strided over the CTAs of its row of the grid.
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < E; m += gridDim.x * blockDim.x) {
-        const long long em = (long long)s * ev_cap + m;
+    // The sample's events, 32 to a warp, strided over the CTAs of its row of the grid.
+    const int lane = threadIdx.x & 31;
+    const int n_l = lane < n_post ? snv[lane] : 0;
+    const float* row_l = st + (lane < n_post ? lane : 0) * k_post;
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m - lane < E; m += gridDim.x * blockDim.x) {
+        const bool on = m < E;
+        const long long em = (long long)s * ev_cap + (on ? m : E - 1);
         const Event e = ev[em];
         const float* wrow = wt + (long long)e.j * ld;
+        // Lane i: neuron i's places for the first and the last of the 32 event times (its whole range if they are not in
+        // order); where they agree, all events share the place.
+        const float t_before = __shfl_up_sync(0xffffffffu, e.t, 1);
+        const bool ordered = __all_sync(0xffffffffu, lane == 0 || t_before <= e.t);
+        const float t_first = __shfl_sync(0xffffffffu, e.t, 0), t_last = __shfl_sync(0xffffffffu, e.t, 31);
+        const int from_l = ordered ? post_position(row_l, n_l, t_first) : 0;
+        const int to_l = ordered ? post_position(row_l, n_l, t_last) : n_l;
+        const unsigned mixed = __ballot_sync(0xffffffffu, from_l != to_l);
+        const unsigned todo = mixed | __ballot_sync(0xffffffffu, from_l < n_l);
         float sa = 0.0f, sb = 0.0f;
-        for (int i = 0; i < n_post; ++i) {
-            const int n = snv[i];
-            const int p = post_position(st + i * k_post, n, e.t);
-            if (p < n) {
-                const float w = __ldg(wrow + i);
-                const float2 AB = stab[i * (k_post + 1) + p];
-                sa += w * AB.x;
-                sb += w * AB.y;
+        for (int i4 = 0; i4 < n_post; i4 += 4) {
+            if (!((todo >> i4) & 15u)) continue;  // no spike after these events in four neurons
+            const float4 w4 = __ldg(reinterpret_cast<const float4*>(wrow + i4));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i4 + u;
+                if (!((todo >> i) & 1u)) continue;
+                const float w = u == 0 ? w4.x : u == 1 ? w4.y : u == 2 ? w4.z : w4.w;
+                int p = __shfl_sync(0xffffffffu, from_l, i);
+                bool live = true;
+                if ((mixed >> i) & 1u) {
+                    const int to = __shfl_sync(0xffffffffu, to_l, i);
+                    p += post_position(st + i * k_post + p, to - p, e.t);
+                    live = p < __shfl_sync(0xffffffffu, n_l, i);
+                }
+                if (live) {
+                    const float2 AB = stab[i * (k_post + 1) + p];
+                    sa += w * AB.x;
+                    sb += w * AB.y;
+                }
             }
         }
-        pre_err[(long long)s * slots_per_sample + ev_slot[em]] = sa * e.es / tau_s - sb * e.e / tau;
+        if (on) pre_err[(long long)s * slots_per_sample + ev_slot[em]] = sa * e.es / tau_s - sb * e.e / tau;
     }
 }
 
