@@ -81,6 +81,8 @@ SIGNATURES = {
     "bats_pre_errors_workspace_bytes": (c_size, [c_int, c_ll, c_int]),
     "bats_pre_errors": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp, c_int, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int,
                                 c_int, c_float, c_float, c_vp, c_vp, c_size, c_vp]),
+    "bats_pre_errors_slots": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp, c_int, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int,
+                                c_int, c_float, c_float, c_vp, c_vp, c_size, c_vp]),
     "bats_conv_backward": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                    c_int, c_vp, c_vp, c_vp, c_int, c_float, c_float, c_vp, c_vp, c_vp]),
     "bats_pool_backward": (c_int, [c_vp, c_vp, c_ll, c_vp, c_ll, c_vp]),

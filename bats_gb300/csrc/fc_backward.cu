@@ -1274,17 +1274,17 @@ static int launch_pre_err(const void* events, const int* ev_count, long long ev_
     return BATS_OK;
 }
 
-extern "C" int bats_pre_errors(const void* events, const int* ev_slot, const int* ev_count, long long ev_cap,
-                               const float* weights_t, int ld, const float* post_times, const void* tables,
+static int pre_errors_impl(const void* events, const int* ev_slot, const int* ev_count, long long ev_cap,
+                           const float* weights_t, int ld, const float* post_times, const void* tables,
                                const int* nvalid, int batch, int n_post, int k_post, int n_pre, int k_pre,
                                float tau_s, float tau, float* pre_errors, void* workspace, size_t workspace_bytes,
-                               cudaStream_t stream) {
+                               bool zero, cudaStream_t stream) {
     BATS_REQUIRE(batch >= 0 && n_post >= 0 && n_pre >= 0 && k_post > 0 && k_pre > 0 && ld >= n_post && ld % 4 == 0,
                  BATS_ERR_BAD_SHAPE, "pre_errors: bad shape");
     if (batch == 0 || n_pre == 0) return BATS_OK;
     BATS_REQUIRE(events && ev_slot && ev_count && pre_errors, BATS_ERR_NULL, "pre_errors: null pointer");
     const long long slots = (long long)n_pre * k_pre;
-    BATS_CUDA(cudaMemsetAsync(pre_errors, 0, (size_t)batch * slots * sizeof(float), stream));
+    if (zero) BATS_CUDA(cudaMemsetAsync(pre_errors, 0, (size_t)batch * slots * sizeof(float), stream));
     if (n_post == 0) return BATS_OK;
     BATS_REQUIRE(weights_t && post_times && tables && nvalid, BATS_ERR_NULL, "pre_errors: null pointer");
     BATS_REQUIRE(((uintptr_t)weights_t & 15) == 0 && ((uintptr_t)events & 15) == 0, BATS_ERR_BAD_SHAPE,
@@ -1329,6 +1329,26 @@ extern "C" int bats_pre_errors(const void* events, const int* ev_slot, const int
         reinterpret_cast<const bats::Event*>(events), ev_slot, ev_count, ev_cap, tiles, slots, tau_s, tau, pre_errors));
     BATS_CUDA(cudaGetLastError());
     return BATS_OK;
+}
+
+extern "C" int bats_pre_errors(const void* events, const int* ev_slot, const int* ev_count, long long ev_cap,
+                               const float* weights_t, int ld, const float* post_times, const void* tables,
+                               const int* nvalid, int batch, int n_post, int k_post, int n_pre, int k_pre,
+                               float tau_s, float tau, float* pre_errors, void* workspace, size_t workspace_bytes,
+                               cudaStream_t stream) {
+    return pre_errors_impl(events, ev_slot, ev_count, ev_cap, weights_t, ld, post_times, tables, nvalid, batch, n_post, k_post,
+                           n_pre, k_pre, tau_s, tau, pre_errors, workspace, workspace_bytes,
+                           true, stream);
+}
+
+extern "C" int bats_pre_errors_slots(const void* events, const int* ev_slot, const int* ev_count, long long ev_cap,
+                                     const float* weights_t, int ld, const float* post_times, const void* tables,
+                                     const int* nvalid, int batch, int n_post, int k_post, int n_pre, int k_pre,
+                                     float tau_s, float tau, float* pre_errors, void* workspace, size_t workspace_bytes,
+                                     cudaStream_t stream) {
+    return pre_errors_impl(events, ev_slot, ev_count, ev_cap, weights_t, ld, post_times, tables, nvalid, batch, n_post, k_post,
+                           n_pre, k_pre, tau_s, tau, pre_errors, workspace, workspace_bytes,
+                           false, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

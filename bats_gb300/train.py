@@ -71,7 +71,8 @@ class FCTrainStep:
                                               torch.empty((B, N), dtype=i32, device=dev),
                                               K.alloc_cursor_heads(B, N, dev) if not need_f else None))
             self.grad.append(torch.empty((N, n_prev), dtype=f32, device=dev))
-            self.pre_err.append(torch.empty((B, n_prev, k_prev), dtype=f32, device=dev))
+            # Only the slots of spikes are written and read; the others stay as they are.
+            self.pre_err.append(torch.zeros((B, n_prev, k_prev), dtype=f32, device=dev))
             n_prev, k_prev = N, Kp
         self.loss = torch.empty((B,), dtype=f32, device=dev)
         self.errors = torch.empty((B, n_prev, k_prev), dtype=f32, device=dev)
@@ -185,7 +186,7 @@ class FCTrainStep:
             if li > 0:
                 pe = self.pre_err[li]
                 L.append((f"{tag}.pre_err", lambda s, ev=ev, t=t, tb=tb, spec=spec, li=li, pe=pe, tau32=tau32: call(
-                    "bats_pre_errors", ptr(ev.events), ptr(ev.slots), ptr(ev.counts), ev.cap, ptr(self.Wt[li]),
+                    "bats_pre_errors_slots", ptr(ev.events), ptr(ev.slots), ptr(ev.counts), ev.cap, ptr(self.Wt[li]),
                     self.Wt[li].shape[1], ptr(t), ptr(tb.tables), ptr(tb.nvalid), B, spec.n_neurons,
                     spec.max_n_spike, ev.n_neurons, ev.k, float(np.float32(spec.tau_s)), float(tau32), ptr(pe), ws,
                     wsb, s)))

@@ -300,6 +300,11 @@ int bats_pre_errors(const void* events, const int* ev_slot, const int* ev_count,
                     const float* weights_t, int ld, const float* post_times, const void* tables, const int* nvalid,
                     int batch, int n_post, int k_post, int n_pre, int k_pre, float tau_s, float tau,
                     float* pre_errors, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+/* The same, writing only the slots of events: a layer's counted backward prep reads no other. */
+int bats_pre_errors_slots(const void* events, const int* ev_slot, const int* ev_count, long long ev_cap,
+                    const float* weights_t, int ld, const float* post_times, const void* tables, const int* nvalid,
+                    int batch, int n_post, int k_post, int n_pre, int k_pre, float tau_s, float tau,
+                    float* pre_errors, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
 /* Convolutional backward: per-sample filter gradient (B, C_out, fx, fy, C) and, if pre_errors is not
  * NULL, the pre-spike errors (B, X*Y*C, k_pre). Replaces compute_weights_gradient_conv and
