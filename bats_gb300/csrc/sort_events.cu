@@ -8,9 +8,9 @@
 //  bats/Layers/LIFLayer.py:66-84, bats/CudaKernels/CuFiles/Inference/compute_pre_exps.cu:2-22).
 // The reference sorts every (neuron, slot) of the batch on the device with argpartition after a
 // host sync on the largest spike count; here every sample's valid slots (time < +inf) are
-// compacted and sorted by a stable LSD radix sort in shared memory (8-bit digits, warp ranks
-// from nine ballots per digit), so the event list needs no host sync and no padding to the
-// batch maximum. Ties keep slot order, which makes the order deterministic.
+// gathered into shared memory, dealt into equal spans of the sample's time and ranked inside their span by
+// (time, slot) (crowded or very large samples by an LSD radix sort), so the event list needs no host sync and no
+// padding to the batch maximum. Ties keep slot order, which makes the order deterministic.
 //
 // CTA b sorts sample b, or sample sample_order[b] when an order is given (the samples longest first: on a
 // batch of uneven samples wider than the resident CTAs, the long samples then start in the first wave
@@ -25,9 +25,9 @@ namespace bats {
 
 constexpr int SORT_BINS = 256;  // digit values of a counting pass; threads tid < SORT_BINS own one bin each
 constexpr int SORT_MAX_BUCKETS = 255;
-// Threads per CTA: 512 for layers of more than SORT_WIDE_CAP slots (each round of a counting pass ranks 512
-// items: 0.88 -> 0.71 ms on the 4096-sample uneven batch's second sort, 0.093 -> 0.081 ms on 800 x 30 slots
-// at batch 256), 256 below (samples of a few hundred items, which a larger block only spreads thinner).
+// Threads per CTA: 512 for layers of more than SORT_WIDE_CAP slots, 256 below (samples of a few hundred items, which a
+// larger block only spreads thinner; the line was drawn with a radix sort: 0.88 -> 0.71 ms on the 4096-sample uneven
+// batch's second sort, 0.093 -> 0.081 ms on 800 x 30 slots at batch 256).
 constexpr int SORT_WIDE_CAP = 1024;
 // Items held in shared memory (two key buffers and two value buffers): slot values are 16-bit when the
 // layer has at most 65536 slots (cap = n_pre * k_pre), else 32-bit. Batches of at most SORT_SMALL_BATCH

@@ -526,9 +526,9 @@ def enqueue_launches(launches, side, main, aux=None, join=()) -> None:
     """Enqueue a step's launch list on the torch stream `main`. With `aux`, the launches named in `side`
     ({launch: the launch it waits for}) run on `aux`, each after its dependency has been enqueued on `main`,
     and `main` waits for `aux` before the first `.wt_copy` launch (which copies the staged transposed weights
-    that those launches wrote), before the launches named in `join`, or at the end. The launches on `aux` read only what their dependency and the
-    launches before it wrote, and write nothing that `main` reads before the join, so the results are those
-    of the list run in order on one stream."""
+    that those launches wrote), before the launches named in `join`, or at the end. The launches on `aux` read
+    only what their dependency and the launches before it wrote, and write nothing that `main` reads before the
+    join, so the results are those of the list run in order on one stream."""
     sm = main.cuda_stream
     if aux is None:
         for _, fn in launches:
