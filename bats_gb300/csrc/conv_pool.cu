@@ -462,9 +462,172 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
 }
 
 // Conv backward over events grouped by input position (the bucketed copy of the sort with
-// bucket_width = C: one bucket per (x, y), time order inside), on a cluster of CONV_BWD_CLUSTER CTAs per
-// sample (position groups dealt to the ranks). Within a position group every filter tap sees one and the same post
-// neuron (x - dx, y - dy, co). A warp's lanes are the group's events, 32 at a time, and it goes through those taps whose
+// bucket_width = C: one bucket per (x, y), time order inside), on a cluster of CONV_BWD_CLUSTER CTAs per sample group
+// (position groups dealt to the ranks). Within a position group every filter tap sees one and the same post neuron
+// (x - dx, y - dy, co). Two kernels, whose results are the same bit for bit, run one after the other, and each cluster's samples
+// are taken by the one that its own count of spiking neurons makes the cheaper (ConvForm): no host knows it.
+struct ConvBwdShape {
+    int Y, C, fx, fy, C_out, Xo, Yo, k_pre, k_post, n_pos;
+};
+
+// TAPS: the taps form alone; CHOOSE: both are launched, and each cluster picks.
+enum class ConvForm { TAPS, CHOOSE };
+
+// Whether the cluster's samples s0 .. s_end - 1 go to the events form: the pairs of a spiking tap and up to 32 events,
+// ~200 warp instructions each there, against ~20 per event and 32 taps in the taps form, whatever spikes. The line is drawn by
+// 40 filters 5 x 5 x 15, 128 samples, K 10 (taps / events form): at 0.19 pairs per event and tile 2.65 / 2.07 ms, at 0.77 1.43 /
+// 2.26; without pre-errors at 0.77 1.19 / 1.32; 64 filters 3 x 3 x 64 at 0.53 291 / 312 us. Uniform over the cluster; ends
+// with a barrier.
+template <bool PRE>
+__device__ __forceinline__ bool conv_events_form(const int* __restrict__ boff, const int* __restrict__ nvalid,
+                                                 const ConvBwdShape& sh, int s0, int s_end) {
+    __shared__ int s_spiking, s_events;
+    if (threadIdx.x == 0) s_spiking = s_events = 0;
+    __syncthreads();
+    const int n_post = sh.Xo * sh.Yo * sh.C_out;
+    const long long n = (long long)(s_end - s0) * n_post;
+    const int* nv = nvalid + (long long)s0 * n_post;
+    int spiking = 0, events = 0;
+#pragma unroll 4
+    for (long long q = threadIdx.x; q < n; q += blockDim.x) spiking += __ldg(nv + q) > 0 ? 1 : 0;
+    for (int s = s0 + threadIdx.x; s < s_end; s += blockDim.x)
+        events += __ldg(boff + (long long)s * (sh.n_pos + 1) + sh.n_pos);
+    spiking = __reduce_add_sync(0xffffffffu, spiking);
+    events = __reduce_add_sync(0xffffffffu, events);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_spiking, spiking);
+        atomicAdd(&s_events, events);
+    }
+    __syncthreads();
+    const float ev = (float)s_events, tiles = (float)((sh.C_out * sh.fx * sh.fy + 31) / 32);
+    const float chunks = ev / (32.0f * (float)sh.n_pos * (float)(s_end - s0)) + 0.5f;  // of 32 events, per position
+    return (float)s_spiking * (float)(sh.fx * sh.fy) * chunks <= (PRE ? 0.4f : 0.6f) * ev * tiles;
+}
+
+// The taps form: a thread per filter tap. A tap's post neuron has its spike data set up once per position and is followed by
+// a forward-only cursor over the position's events. A spike's slot (neuron j, k-th spike of j) follows from the order of
+// appearance of j in the group. The per-sample gradient copies are combined over the cluster as in
+// conv_backward_cluster_kernel; pre errors are reduced over the taps in the CTA that owns the group.
+template <bool PRE, bool W_SMEM>
+__global__ void __launch_bounds__(1024)
+conv_backward_taps_kernel(const Event* __restrict__ ev_b, const int* __restrict__ boff, long long ev_cap,
+                          const float* __restrict__ W, ConvBwdShape sh, const float* __restrict__ post_t,
+                          const float2* __restrict__ tab, const int* __restrict__ nvalid, float tau_s, float tau,
+                          long long pre_slots, float* __restrict__ grad, float* __restrict__ pre_err, int batch,
+                          int group, ConvForm form) {
+    pdl_prologue();
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) float4 cb_smem[];
+    __shared__ Event sev[32];
+    __shared__ float sred[32][33];
+    __shared__ int sslot[32], scc[32];
+    const int s0 = (int)blockIdx.y * group, s_end = min(batch, s0 + group);
+    if (form == ConvForm::CHOOSE && conv_events_form<PRE>(boff, nvalid, sh, s0, s_end)) return;
+    const float inv_tau_s = 1.0f / tau_s, inv_tau = 1.0f / tau;  // the error terms' factors, as reciprocals
+    const int rank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nwarps = blockDim.x >> 5;
+    const int C = sh.C, taps = sh.C_out * sh.fx * sh.fy;
+    const int total = taps * C;
+    const int n_post = sh.Xo * sh.Yo * sh.C_out;
+    float* Gs = reinterpret_cast<float*>(cb_smem);          // [tap][channel]
+    int* kcount = reinterpret_cast<int*>(Gs + total);       // per channel: earlier events of the position
+    for (int q = tid; q < total; q += blockDim.x) Gs[q] = 0.0f;
+    // The filters, for the pre-spike error terms: in shared memory when they fit (a thread's weight reads are C floats
+    // apart, one cache sector per lane from global memory).
+    const float* Wk = W;
+    if (W_SMEM) {
+        float* sWf = reinterpret_cast<float*>(kcount + C);
+        for (int q = tid; q < total; q += blockDim.x) sWf[q] = W[q];
+        Wk = sWf;
+    }
+    const bool has_tap = tid < taps;
+    const int co = has_tap ? tid / (sh.fx * sh.fy) : 0, dx = has_tap ? tid / sh.fy % sh.fx : 0;
+    const int dy = has_tap ? tid % sh.fy : 0;
+    __syncthreads();
+    // The cluster's samples (one with group == 1: the per-sample gradient), accumulated in order.
+    for (int s = s0; s < s_end; ++s) {
+        const int* bo = boff + (long long)s * (sh.n_pos + 1);
+        const Event* evs = ev_b + (long long)s * ev_cap;
+        for (int g = rank; g < sh.n_pos; g += CONV_BWD_CLUSTER) {
+            const int beg = bo[g], end = bo[g + 1];
+            if (beg >= end) continue;  // uniform over the CTA
+            const int xo = g / sh.Y - dx, yo = g % sh.Y - dy;
+            const bool in = has_tap && xo >= 0 && yo >= 0 && xo < sh.Xo && yo < sh.Yo;
+            PostCursor cur;
+            const long long pn = in ? (long long)s * n_post + (xo * sh.Yo + yo) * sh.C_out + co : 0;
+            cur.init(post_t + pn * sh.k_post, tab + pn * (sh.k_post + 1), in ? nvalid[pn] : 0);
+            // Two barriers per chunk: after warp 0 stages it (every thread reads it), and after the error terms are in
+            // sred (every thread is done with the chunk's records; the chunk's events then sum the terms). The next
+            // chunk's first barrier orders those sums' reads of sred and sslot before anything overwrites them (warp 0
+            // sums, then stages; the other warps write sred only after that barrier).
+            for (int m0 = beg; m0 < end; m0 += 32) {
+                const int cnt = min(32, end - m0);
+                if (warp == 0) {
+                    if (m0 == beg) {  // the position's spike counters per channel: warp 0's alone
+                        for (int q = lane; q < C; q += 32) kcount[q] = 0;
+                        __syncwarp();
+                    }
+                    // Stage the chunk; the spikes' slots: j * k_pre + the order of appearance of j in the group (all
+                    // events of a position share x and y, so j is fixed by the channel: earlier chunks' counts plus
+                    // the rank among this chunk's events of the same channel).
+                    Event e;
+                    int c = -1;
+                    if (lane < cnt) {
+                        e = evs[m0 + lane];
+                        c = e.j % C;
+                        sev[lane] = e;
+                        scc[lane] = c;
+                    }
+                    const unsigned peers = __match_any_sync(0xffffffffu, c);
+                    const int before = __popc(peers & lanemask_lt());
+                    int base = 0;
+                    if (lane < cnt) base = kcount[c];
+                    __syncwarp();
+                    if (lane < cnt) {
+                        sslot[lane] = e.j * sh.k_pre + base + before;
+                        if (before == __popc(peers) - 1) kcount[c] = base + __popc(peers);
+                    }
+                }
+                __syncthreads();
+                float term[32];
+#pragma unroll
+                for (int q = 0; q < 32; ++q) {
+                    term[q] = 0.0f;
+                    if (q < cnt && in) {
+                        const Event e = sev[q];
+                        cur.advance_past(e.t);
+                        if (cur.valid()) {
+                            const int at = tid * C + scc[q];
+                            Gs[at] += fmaf(e.es, cur.AB.x, -(e.e * cur.AB.y));
+                            if (PRE) term[q] = Wk[at] * (cur.AB.x * e.es * inv_tau_s - cur.AB.y * e.e * inv_tau);
+                        }
+                    }
+                }
+                // The chunk's 32 error terms summed over the warp at once (lane q: event q), then over the warps.
+                if (PRE) sred[lane][warp] = warp_transpose_reduce<32>(term);
+                __syncthreads();  // every thread is done with the chunk's records (warp 0 may restage them next)
+                if (PRE && tid < cnt) {
+                    float acc = 0.0f;
+                    for (int w = 0; w < nwarps; ++w) acc += sred[tid][w];
+                    pre_err[(long long)s * pre_slots + sslot[tid]] = acc;
+                }
+            }
+        }
+    }
+    cluster.sync();
+    const int per = (total + CONV_BWD_CLUSTER - 1) / CONV_BWD_CLUSTER;
+    const int q_end = min(total, (rank + 1) * per);
+    for (int q = rank * per + tid; q < q_end; q += blockDim.x) {
+        float acc = 0.0f;
+        for (int r = 0; r < CONV_BWD_CLUSTER; ++r) acc += cluster.map_shared_rank(Gs, r)[q];
+        grad[(long long)blockIdx.y * total + q] = acc;
+    }
+    cluster.sync();
+}
+
+// The events form: a warp's lanes are a position's events, 32 at a time, and it goes through those taps whose
 // post neuron lies inside the output and spiked: the neuron's spike times and table rows lie on the lanes (K <= 32;
 // loaded one neuron ahead), every lane finds its event's place among them by a binary search over shuffles and leaves its
 // gradient term in shared memory. The events of a group are staged by (channel, time), so that a channel's terms are
@@ -482,10 +645,6 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
 // What bounds it: instruction issue (4.7 M pairs of a spiking tap and up to 32 events, 8 rounds of a channel's terms each;
 // 67 % of the issue slots of 128 CTAs). 40 filters 5 x 5 x 15 over 12 x 12, 128 samples: 2.65 -> 2.07 ms, the same
 // sums.
-struct ConvBwdShape {
-    int Y, C, fx, fy, C_out, Xo, Yo, k_pre, k_post, n_pos;
-};
-
 constexpr int CONV_BWD_POS = (255 + CONV_BWD_CLUSTER - 1) / CONV_BWD_CLUSTER;  // positions per rank
 constexpr int CONV_BWD_UNIT = 16;                                              // taps per unit: two units per tile
 
@@ -502,6 +661,8 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) float4 cb_smem[];
     __shared__ int s_beg[CONV_BWD_POS], s_len[CONV_BWD_POS], s_at[CONV_BWD_POS], s_next;
+    const int s0 = (int)blockIdx.y * group, s_end = min(batch, s0 + group);
+    if (!conv_events_form<PRE>(boff, nvalid, sh, s0, s_end)) return;
     const float inv_tau_s = 1.0f / tau_s, inv_tau = 1.0f / tau;  // the error terms' factors, as reciprocals
     const int rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -525,8 +686,7 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
     const float* Wk = W_SMEM ? sWf : W;
     const int n_mine = rank < sh.n_pos ? (sh.n_pos - 1 - rank) / CONV_BWD_CLUSTER + 1 : 0;
     // The cluster's samples (one with group == 1: the per-sample gradient), accumulated in order.
-    const int s_end = min(batch, ((int)blockIdx.y + 1) * group);
-    for (int s = (int)blockIdx.y * group; s < s_end; ++s) {
+    for (int s = s0; s < s_end; ++s) {
         const int* bo = boff + (long long)s * (sh.n_pos + 1);
         const Event* evs = ev_b + (long long)s * ev_cap;
         const long long pn_s = (long long)s * n_post;
@@ -1088,28 +1248,20 @@ static auto* conv_grouped_kernel(int k_post) {
                           : bats::conv_backward_grouped_kernel<true, 4, PRE, W_SMEM>;
 }
 
+// From so many filter taps on the events form is worth a second launch (its clusters that do not take part cost a few us):
+// 216 taps, 21 samples, few spiking 120 -> 62 us; 72 taps all spiking 44 us, and 81 in the events form.
+constexpr long long CONV_EVENTS_TAPS = 192;
+
 static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* bucket_offsets, long long ev_cap,
                                        const float* weights, const bats::ConvBwdShape& sh, const float* post_times,
                                        const void* tables, const int* nvalid, float tau_s, float tau,
                                        long long pre_slots, float* grad, float* pre_errors, int batch, int group,
                                        cudaStream_t stream) {
     const long long taps = (long long)sh.C_out * sh.fx * sh.fy;
-    constexpr size_t LIMIT = 224 * 1024;
-    const bool pre = pre_errors != nullptr, w = pre && conv_grouped_smem(taps, sh.C, 64, pre, true) <= LIMIT;
-    int batch_ev = 512;
-    while (batch_ev > 32 && conv_grouped_smem(taps, sh.C, batch_ev, pre, w) > LIMIT) batch_ev -= 32;
-    const size_t smem = conv_grouped_smem(taps, sh.C, batch_ev, pre, w);
-    auto* kernel = !pre_errors ? conv_grouped_kernel<false, false>(sh.k_post)
-                   : w         ? conv_grouped_kernel<true, true>(sh.k_post)
-                               : conv_grouped_kernel<true, false>(sh.k_post);
-    cudaError_t e = (cudaError_t)bats::max_dynamic_smem_set((const void*)kernel, (int)smem);
-    if (e != cudaSuccess) return e;
+    const bool pre = pre_errors != nullptr, choose = taps >= CONV_EVENTS_TAPS;
     const int groups = (batch + group - 1) / group;
-    const int threads = (int)std::min<long long>(1024, (taps + 31) / 32 * (32 / bats::CONV_BWD_UNIT) * 32);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(bats::CONV_BWD_CLUSTER, groups);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1118,8 +1270,37 @@ static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* b
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1 + (unsigned)bats::pdl_attribute(attr + 1);
-    return cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const bats::Event*>(events_bucketed), bucket_offsets, ev_cap,
-                              weights, sh, post_times, reinterpret_cast<const float2*>(tables), nvalid, tau_s, tau,
+    const auto* ev = reinterpret_cast<const bats::Event*>(events_bucketed);
+    const auto* tab = reinterpret_cast<const float2*>(tables);
+    {
+        const size_t grad_bytes = (size_t)taps * sh.C * sizeof(float), small = grad_bytes + (size_t)sh.C * sizeof(int);
+        const bool w = pre && small + grad_bytes <= 200 * 1024;
+        const size_t smem = small + (w ? grad_bytes : 0);
+        auto* kernel = !pre ? bats::conv_backward_taps_kernel<false, false>
+                       : w  ? bats::conv_backward_taps_kernel<true, true>
+                            : bats::conv_backward_taps_kernel<true, false>;
+        cudaError_t e = (cudaError_t)bats::max_dynamic_smem_set((const void*)kernel, (int)smem);
+        if (e != cudaSuccess) return e;
+        cfg.blockDim = dim3((unsigned)((taps + 31) / 32 * 32));
+        cfg.dynamicSmemBytes = smem;
+        e = cudaLaunchKernelEx(&cfg, kernel, ev, bucket_offsets, ev_cap, weights, sh, post_times, tab, nvalid, tau_s, tau,
+                               pre_slots, grad, pre_errors, batch, group,
+                               choose ? bats::ConvForm::CHOOSE : bats::ConvForm::TAPS);
+        if (e != cudaSuccess || !choose) return e;
+    }
+    constexpr size_t LIMIT = 224 * 1024;
+    const bool w = pre && conv_grouped_smem(taps, sh.C, 64, pre, true) <= LIMIT;
+    int batch_ev = 512;
+    while (batch_ev > 32 && conv_grouped_smem(taps, sh.C, batch_ev, pre, w) > LIMIT) batch_ev -= 32;
+    const size_t smem = conv_grouped_smem(taps, sh.C, batch_ev, pre, w);
+    auto* kernel = !pre ? conv_grouped_kernel<false, false>(sh.k_post)
+                   : w  ? conv_grouped_kernel<true, true>(sh.k_post)
+                        : conv_grouped_kernel<true, false>(sh.k_post);
+    cudaError_t e = (cudaError_t)bats::max_dynamic_smem_set((const void*)kernel, (int)smem);
+    if (e != cudaSuccess) return e;
+    cfg.blockDim = dim3((unsigned)std::min<long long>(1024, (taps + 31) / 32 * (32 / bats::CONV_BWD_UNIT) * 32));
+    cfg.dynamicSmemBytes = smem;
+    return cudaLaunchKernelEx(&cfg, kernel, ev, bucket_offsets, ev_cap, weights, sh, post_times, tab, nvalid, tau_s, tau,
                               pre_slots, grad, pre_errors, batch, group, batch_ev);
 }
 
