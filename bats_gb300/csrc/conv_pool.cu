@@ -40,7 +40,7 @@ struct __align__(16) ConvEvent {
 constexpr int CONV_SUB = 64;               // kept events per round of the lists
 constexpr int CONV_GROUP = 8;              // list entries per pass of the screen
 constexpr int CONV_LIST = CONV_SUB + CONV_GROUP;
-constexpr int CONV_POSITIONS = 32;         // positions per CTA at most (2.9 KB of list each)
+constexpr int CONV_POSITIONS = 16;         // positions per CTA at most (2.9 KB of list each)
 
 // One position's list of relevant events, in time order: window constants (the window ends at the next relevant
 // event), times and filter rows ((dx fy + dy) C + c, or -1: weight 0).
@@ -1130,7 +1130,9 @@ static void conv_tile(int C_out, int threads, int& TX, int& TY) {
     TY = P / TX;
 }
 
-// Larger tiles read the sample's events fewer times and share more of each receptive field; smaller ones give more CTAs
+// A CTA has at least eight warps, which make the lists where few output channels use them, and at most 16 positions, whose lists
+// leave room for other CTAs (2 filters 5 x 5 over 28 x 28, 128 samples: 117 us with two warps and 32 positions, 57 so; 42
+// without lists; 3 filters 3 x 3 x 6 over 12 x 12: 115, 64 and 220). Larger tiles read the sample's events fewer times and share more of each receptive field; smaller ones give more CTAs
 // and shorter waits at the barriers. 512 threads pay only where a sample can carry many events (12 x 12 x 15 x 40 slots,
 // 768 CTAs: 0.76 ms, 256 threads 0.87; 28 x 28 x 1 slots: 0.099 ms, 256 threads 0.087) and the grid still fills two
 // CTAs on each of the 152 SMs; below that the tile is halved (42 CTAs of 512 threads: 0.142 ms, 168 of 128: 0.095).
@@ -1163,7 +1165,7 @@ extern "C" int bats_conv_forward(const void* events, const int* ev_count, long l
     const int Xo = X - fx + 1, Yo = Y - fy + 1;
     int TX, TY;
     conv_plan(batch, Xo, Yo, C_out, ev_cap, TX, TY);
-    const int threads = ((TX * TY * C_out + 31) / 32) * 32;
+    const int threads = std::max((TX * TY * C_out + 31) / 32 * 32, 32 * std::min(TX * TY, 8));  // (eight warps make lists)
     const int tiles_x = (Xo + TX - 1) / TX, tiles_y = (Yo + TY - 1) / TY;
     const size_t base_smem = TX * TY * sizeof(bats::ConvList) + (bats::CONV_SUB + threads) * sizeof(bats::ConvEvent);
     const size_t w_smem = (size_t)C_out * ((fx * fy * C) | 1) * sizeof(float);
