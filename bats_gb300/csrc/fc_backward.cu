@@ -100,9 +100,9 @@ constexpr int PREP_KS = 33;  // padded row stride (conflict-free)
 
 __global__ void __launch_bounds__(PREP_WARPS * 32)
 bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, const float* __restrict__ x,
-                      const float* __restrict__ z, float* __restrict__ err, long long total, int K, float c, float tau,
-                      float dtt, float* __restrict__ f1, float* __restrict__ f2, float2* __restrict__ tab,
-                      int* __restrict__ nvalid) {
+                      const float* __restrict__ z, const float* err, float* err_out, long long total, int K, float c,
+                      float tau, float dtt, float* __restrict__ f1, float* __restrict__ f2, float2* __restrict__ tab,
+                      int* __restrict__ nvalid, float2* __restrict__ head_t, float4* __restrict__ head_ab) {
     pdl_prologue();
     extern __shared__ float prep_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -133,7 +133,11 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
     __shared__ int sN[PREP_WARPS][32];
     sN[warp][lane] = n;
     if (!__any_sync(0xffffffffu, n > 0)) {
-        // Silent neurons: nothing to read or write but zero factors (no table entry is ever read past n).
+        // Silent neurons: nothing to read or write but zero factors (no table entry is ever read past n) and empty heads.
+        if (head_t && lane < cnt) {
+            head_t[nb + lane] = make_float2(BATS_INF, BATS_INF);
+            head_ab[nb + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
         if (f1)
             for (int q = lane; q < nk; q += 32) {
                 f1[base + q] = 0.0f;
@@ -160,6 +164,7 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
         float* rx = sX + lane * PREP_KS;
         float* ra = sA + lane * PREP_KS;
         float* re = sE + lane * PREP_KS;
+        const float h_t0 = n > 0 ? rt[0] : BATS_INF, h_t1 = n > 1 ? rt[1] : BATS_INF;  // before the sums overwrite them
         // Reset errors, last spike first (propagate_recurrent_errors.cu:17-22).
         float cum = 0.0f;
         for (int k = n - 1; k >= 0; --k) {
@@ -200,12 +205,17 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
                 }
             }
         }
+        if (head_t) {
+            head_t[nb + lane] = make_float2(h_t0, h_t1);
+            head_ab[nb + lane] = make_float4(n > 0 ? rt[0] : 0.0f, n > 0 ? rx[0] : 0.0f, n > 1 ? rt[1] : 0.0f,
+                                             n > 1 ? rx[1] : 0.0f);
+        }
     }
     __syncwarp();
     for (int q = lane; q < nk; q += 32) {
         const int r = q / K, k = q % K;
         const int o = r * PREP_KS + k;
-        if (k < sN[warp][r]) err[base + q] = sE[o];
+        if (err_out && k < sN[warp][r]) err_out[base + q] = sE[o];
         if (f1) {
             f1[base + q] = sA[o];
             f2[base + q] = sZ[o];
@@ -221,7 +231,7 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
 
 // Layer-path prep given the forward's spike counts: only each neuron's leading min(n_spikes, K) slots
 // are read (the forward writes +inf past them), so silent slots cost nothing. A warp handles 32 neurons
-// and stages their valid slots compactly in shared memory (at most PREPC_CAP per round; a round takes
+// and stages their valid slots compactly in shared memory (at most CAP per round; a round takes
 // the next lanes whose slots fit). The reset errors are a lane's serial chain over its neuron's spikes; the factors and the
 // suffix sums, which differ most in length between neurons, are one lane per slot. The arithmetic per neuron is
 // bwd_prep_layer_kernel's in its order, so errors, tables and counts are identical to it (n = the first +inf time below the
@@ -232,24 +242,24 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
 // 365 -> 255 us (140 M); 800 neurons, 256 samples, 3510 spikes: 54 -> 40 us. Rounds of 128 slots (half the shared
 // memory, twice the warps) against 256: 255 / 335 and 41 / 40 us.
 // Without counts 475 k spikes of 300 neurons, 256 samples: 64 us with whole rows of K slots staged (ten warps an SM) -> 54 us.
-constexpr int PREPC_WARPS = 8;
-constexpr int PREPC_CAP = 128;
-
+template <int CAP>
 struct PrepCompact {
-    float t[PREPC_CAP], z[PREPC_CAP], x[PREPC_CAP], a[PREPC_CAP], e[PREPC_CAP];
-    unsigned char owner[PREPC_CAP];
+    float t[CAP], z[CAP], x[CAP], a[CAP], e[CAP];
+    unsigned char owner[CAP];
 };
 
-__global__ void __launch_bounds__(PREPC_WARPS * 32)
+// CAP: slots per round; WARPS: per CTA.
+template <int CAP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_spikes, const float* __restrict__ a,
                         const float* __restrict__ x, const float* __restrict__ z, const float* err, float* err_out,
                         long long total, int K, float c, float tau, float dtt, float2* __restrict__ tab,
                         int* __restrict__ nvalid, float2* __restrict__ head_t, float4* __restrict__ head_ab) {
     pdl_prologue();
-    __shared__ PrepCompact sm_all[PREPC_WARPS];
+    __shared__ PrepCompact<CAP> sm_all[WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    PrepCompact& sm = sm_all[warp];
-    const long long nb = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * 32;
+    PrepCompact<CAP>& sm = sm_all[warp];
+    const long long nb = ((long long)blockIdx.x * WARPS + warp) * 32;
     if (nb >= total) return;
     const int cnt = (int)min(32LL, total - nb);
     const int K1 = K + 1;
@@ -273,7 +283,7 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
     const int excl = incl - n_in;
     int r0 = 0, base = 0;
     while (r0 < 32) {
-        const unsigned in_round = __ballot_sync(0xffffffffu, lane >= r0 && incl - base <= PREPC_CAP);
+        const unsigned in_round = __ballot_sync(0xffffffffu, lane >= r0 && incl - base <= CAP);
         const int r1 = 32 - __clz(in_round);
         const int V = __shfl_sync(0xffffffffu, incl, r1 - 1) - base;
         const bool mine = lane >= r0 && lane < r1;
@@ -1005,17 +1015,45 @@ static CursorHeads cursor_heads_of(const void* base, long long pairs) {
     return {reinterpret_cast<float2*>(b), reinterpret_cast<float4*>(b + heads_times_bytes(pairs))};
 }
 
-static int launch_prep_counted(const float* post_times, const int* n_spikes, const float* a, const float* x,
-                               const float* post_exp_tau, const float* errors, float* errors_out, long long total,
-                               int k_post, float c, float tau, float delta_theta_tau, void* tables, int* nvalid,
-                               void* cursor_heads, cudaStream_t stream) {
+static int launch_prep_layer(const float* post_times, const float* a, const float* x, const float* post_exp_tau,
+                             const float* errors, float* errors_out, long long total, int k_post, float c, float tau,
+                             float delta_theta_tau, float* f1, float* f2, void* tables, int* nvalid, void* cursor_heads,
+                             cudaStream_t stream) {
     const long long warps = (total + 31) / 32;
-    const int per = warps < 152 * 8 ? 1 : bats::PREPC_WARPS;  // a layer of few warps goes to as many SMs as it can
-    const int blocks = (int)((warps + per - 1) / per);
+    const int blocks = (int)((warps + bats::PREP_WARPS - 1) / bats::PREP_WARPS);
+    const size_t smem = (size_t)bats::PREP_WARPS * 5 * 32 * bats::PREP_KS * sizeof(float);
     const CursorHeads h = cursor_heads_of(cursor_heads, total);
-    BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel, blocks, per * 32, 0, stream, post_times,
-        n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
-        reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab));
+    BATS_CUDA((cudaError_t)bats::max_dynamic_smem_set((const void*)bats::bwd_prep_layer_kernel, (int)smem));
+    BATS_CUDA(bats::launch(bats::bwd_prep_layer_kernel, blocks, bats::PREP_WARPS * 32, smem, stream, post_times, a, x,
+        post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau, f1, f2, reinterpret_cast<float2*>(tables),
+        nvalid, h.t, h.ab));
+    BATS_CUDA(cudaGetLastError());
+    return BATS_OK;
+}
+
+// The prep without factors (K <= 32), by the number of warps of 32 neurons. Up to twenty per SM: without counts the layer
+// kernel (no rounds and no search for the counts: 300 neurons, 256 samples, all 30 slots valid 46 us, 83 in the counted kernel; 10
+// neurons 21 / 40), with counts one warp per CTA, so that they spread over the SMs, and all 32 x 32 slots in one round (10
+// neurons, all valid 31 us, 56 in rounds of 128 slots; 800 neurons, 64 samples, 8.9 valid 29 / 40). Beyond, where the shared
+// memory of whole rows leaves ten warps on an SM, the counted kernel with rounds of 128 slots, eight warps per CTA (800
+// neurons, 256 samples: 42 us, 46 in one round; without counts 54 / 64 in the layer kernel).
+static int launch_prep(const float* post_times, const int* n_spikes, const float* a, const float* x,
+                       const float* post_exp_tau, const float* errors, float* errors_out, long long total, int k_post,
+                       float c, float tau, float delta_theta_tau, void* tables, int* nvalid, void* cursor_heads,
+                       cudaStream_t stream) {
+    const long long warps = (total + 31) / 32;
+    const CursorHeads h = cursor_heads_of(cursor_heads, total);
+    if (warps > 20 * 152)
+        BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<128, 8>, (unsigned)((warps + 7) / 8), 256, 0, stream, post_times,
+            n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
+            reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab));
+    else if (n_spikes)
+        BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<1024, 1>, (unsigned)warps, 32, 0, stream, post_times,
+            n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
+            reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab));
+    else
+        return launch_prep_layer(post_times, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau,
+                                 delta_theta_tau, nullptr, nullptr, tables, nvalid, cursor_heads, stream);
     BATS_CUDA(cudaGetLastError());
     return BATS_OK;
 }
@@ -1036,17 +1074,10 @@ extern "C" int bats_backward_prep_layer(const float* post_times, const float* a,
                                   delta_theta_tau, 1, 1, f1, f2, tables, nvalid, stream);
     }
     if (!f1)
-        return launch_prep_counted(post_times, nullptr, a, x, post_exp_tau, errors, errors, total, k_post, c, tau,
-                                   delta_theta_tau, tables, nvalid, nullptr, stream);
-    const long long warps = (total + 31) / 32;
-    const int blocks = (int)((warps + bats::PREP_WARPS - 1) / bats::PREP_WARPS);
-    const size_t smem = (size_t)bats::PREP_WARPS * 5 * 32 * bats::PREP_KS * sizeof(float);
-    BATS_CUDA((cudaError_t)bats::max_dynamic_smem_set((const void*)bats::bwd_prep_layer_kernel, (int)smem));
-    BATS_CUDA(bats::launch(bats::bwd_prep_layer_kernel, blocks, bats::PREP_WARPS * 32, smem, stream, post_times, a, x,
-        post_exp_tau, errors, total, k_post, c, tau, delta_theta_tau, f1, f2, reinterpret_cast<float2*>(tables),
-        nvalid));
-    BATS_CUDA(cudaGetLastError());
-    return BATS_OK;
+        return launch_prep(post_times, nullptr, a, x, post_exp_tau, errors, errors, total, k_post, c, tau,
+                           delta_theta_tau, tables, nvalid, nullptr, stream);
+    return launch_prep_layer(post_times, a, x, post_exp_tau, errors, errors, total, k_post, c, tau, delta_theta_tau, f1, f2,
+                             tables, nvalid, nullptr, stream);
 }
 
 extern "C" size_t bats_cursor_heads_bytes(int batch, int n_post) {
@@ -1066,8 +1097,8 @@ extern "C" int bats_backward_prep_counted(const float* post_times, const int* n_
     if (total == 0) return BATS_OK;
     BATS_REQUIRE(post_times && n_spikes && a && x && post_exp_tau && errors && tables && nvalid, BATS_ERR_NULL,
                  "backward_prep_counted: null pointer");
-    return launch_prep_counted(post_times, n_spikes, a, x, post_exp_tau, errors, errors, total, k_post, c, tau,
-                               delta_theta_tau, tables, nvalid, cursor_heads, stream);
+    return launch_prep(post_times, n_spikes, a, x, post_exp_tau, errors, errors, total, k_post, c, tau, delta_theta_tau,
+                       tables, nvalid, cursor_heads, stream);
 }
 
 extern "C" int bats_backward_prep_readonly(const float* post_times, const float* a, const float* x,
@@ -1082,8 +1113,8 @@ extern "C" int bats_backward_prep_readonly(const float* post_times, const float*
     if (total == 0) return BATS_OK;
     BATS_REQUIRE(post_times && a && x && post_exp_tau && errors && tables && nvalid, BATS_ERR_NULL,
                  "backward_prep_readonly: null pointer");
-    return launch_prep_counted(post_times, nullptr, a, x, post_exp_tau, errors, nullptr, total, k_post, c, tau,
-                               delta_theta_tau, tables, nvalid, cursor_heads, stream);
+    return launch_prep(post_times, nullptr, a, x, post_exp_tau, errors, nullptr, total, k_post, c, tau, delta_theta_tau,
+                       tables, nvalid, cursor_heads, stream);
 }
 
 // Post neurons per gradient CTA: two independent warps (the same warps per SM as four, 2.6 % faster on an

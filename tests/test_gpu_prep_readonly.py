@@ -1,6 +1,7 @@
-"""The backward prep that leaves the errors alone and finds the counts itself, against the thread-per-neuron prep over the same state: counts
-and every table entry below them equal bit for bit, the errors untouched, the cursor heads those of the rows. One slot, full buffers of
-32, a last warp partly filled, silent neurons, +inf before the end of a train; and a gradient that is an expanded scalar."""
+"""The backward prep that leaves the errors alone and finds the counts itself, and the one that is given the counts, against the
+thread-per-neuron prep over the same state: counts and every table entry below them equal bit for bit, the errors untouched or the same,
+the cursor heads those of the rows. One slot, full buffers of 32, a last warp partly filled, silent neurons, +inf before the end of a
+train, both sides of the line between the kernels (3040 warps); and a gradient that is an expanded scalar."""
 import numpy as np
 import pytest
 import torch
@@ -12,8 +13,9 @@ from bats_gb300.autograd import lif_fc
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B,N,k", [(1, 1, 1), (3, 33, 32), (7, 70, 30), (64, 5, 2)])
-def test_readonly_prep(cuda, B, N, k):
+@pytest.mark.parametrize("counted", [False, True])
+@pytest.mark.parametrize("B,N,k", [(1, 1, 1), (3, 33, 32), (7, 70, 30), (64, 5, 2), (2947, 33, 3), (2948, 33, 3), (3100, 32, 32)])
+def test_readonly_prep(cuda, B, N, k, counted):
     rng = np.random.default_rng(B + k)
     n = rng.integers(0, k + 1, (B, N))
     n[0, 0] = k
@@ -25,9 +27,12 @@ def test_readonly_prep(cuda, B, N, k):
     err = torch.as_tensor(np.where(slot, rng.normal(size=(B, N, k)), np.nan).astype(np.float32)).cuda()
     t = torch.as_tensor(t).cuda()
     kept = err.clone()
-    got = K.backward_prep(t, a, x, z, err, 0.4, 0.26, 0.7, keep_errors=True)
-    assert torch.equal(err.view(torch.int32), kept.view(torch.int32))
     first = torch.where(torch.isinf(t), torch.arange(k, device="cuda"), k).amin(-1).int()
+    if counted:
+        got = K.backward_prep(t, a, x, z, kept, 0.4, 0.26, 0.7, n_spikes=first)
+    else:
+        got = K.backward_prep(t, a, x, z, err, 0.4, 0.26, 0.7, keep_errors=True)
+        assert torch.equal(err.view(torch.int32), kept.view(torch.int32))
     assert torch.equal(got.nvalid, first)
     z_inf = torch.where(torch.arange(k, device="cuda") < first[..., None], z, torch.full_like(z, float("inf")))
     f1, f2, tab, nv = torch.empty_like(t), torch.empty_like(t), torch.empty((B, N, k + 1, 2), device="cuda"), torch.empty((B, N), dtype=torch.int32, device="cuda")
@@ -35,6 +40,8 @@ def test_readonly_prep(cuda, B, N, k):
          ptr(tab), ptr(nv), stream_ptr())
     valid = torch.arange(k + 1, device="cuda") < first[..., None]
     assert torch.equal(got.tables[valid], tab[valid])
+    if counted:  # the reset errors below the counts
+        assert torch.equal(kept[valid[..., :k]], err[valid[..., :k]])
     pairs = B * N
     heads = got.heads.cpu().numpy()
     ht = heads[:8 * pairs].view(np.float32).reshape(B, N, 2)
