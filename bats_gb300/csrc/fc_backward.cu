@@ -232,8 +232,9 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
 // Layer-path prep given the forward's spike counts: only each neuron's leading min(n_spikes, K) slots
 // are read (the forward writes +inf past them), so silent slots cost nothing. A warp handles 32 neurons
 // and stages their valid slots compactly in shared memory (at most CAP per round; a round takes
-// the next lanes whose slots fit). The reset errors are a lane's serial chain over its neuron's spikes; the factors and the
-// suffix sums, which differ most in length between neurons, are one lane per slot. The arithmetic per neuron is
+// the next lanes whose slots fit). The reset errors are a lane's serial chain over its neuron's spikes; the factors are one
+// lane per slot, the suffix sums one lane per four consecutive entries (one lane per entry reads four times as much where
+// buffers are full: 800 neurons, 256 samples, 30 valid slots 171 -> 144 us; few valid slots alike). The arithmetic per neuron is
 // bwd_prep_layer_kernel's in its order, so errors, tables and counts are identical to it (n = the first +inf time below the
 // count, or the count). Without n_spikes the count is the slots before a row's first +inf; without err_out the reset errors
 // stay in shared memory (err may be err_out).
@@ -325,33 +326,61 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
             }
         }
         __syncwarp();
-        // Factors: a lane per slot (they replace a and z).
-        for (int q = lane; q < V; q += 32) {
-            const float xk = sm.x[q];
-            sm.a[q] = tau / sm.a[q] * (1 + sm.z[q] * c / xk);
-            sm.z[q] = tau / xk;
-        }
-        __syncwarp();
-        // Tables: a lane per entry p of a neuron, its sums upwards from k = p; the first two entries also into (t, x), for
-        // the head.
+        // Factors: a lane per slot (they replace a and z); the reset errors go out.
         for (int q0 = 0; q0 < V; q0 += 32) {
             const int q = q0 + lane;
             const int r = q < V ? sm.owner[q] : 0;
             const int ro = __shfl_sync(0xffffffffu, excl, r) - base;
             const int nr = __shfl_sync(0xffffffffu, n, r);
-            const int p = q - ro;
-            if (q < V && p < nr) {
-                float sa = 0.0f, sb = 0.0f;
-                for (int k = q; k < ro + nr; ++k) {
-                    const float ek = sm.e[k];
-                    sa += ek * sm.a[k];
-                    sb += ek * sm.z[k];
+            if (q < V) {
+                const float xk = sm.x[q];
+                sm.a[q] = tau / sm.a[q] * (1 + sm.z[q] * c / xk);
+                sm.z[q] = tau / xk;
+                if (err_out && q - ro < nr) err_out[(nb + r) * K + q - ro] = sm.e[q];
+            }
+        }
+        // Tables: a lane per four consecutive entries of a neuron, each entry's sums upwards from its own spike, the four
+        // chains side by side; the first two entries also into (t, x), for the head.
+        const int fours = (n + 3) >> 2;
+        int fours_incl = fours;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, fours_incl, o);
+            if (lane >= o) fours_incl += y;
+        }
+        const int fours_all = __shfl_sync(0xffffffffu, fours_incl, 31), fours_from = fours_incl - fours;
+        __syncwarp();
+        for (int g = 0; g < fours; ++g) sm.owner[fours_from + g] = (unsigned char)lane;
+        __syncwarp();
+        for (int i0 = 0; i0 < fours_all; i0 += 32) {
+            const int i = i0 + lane;
+            const int r = i < fours_all ? sm.owner[i] : 0;
+            const int ro = __shfl_sync(0xffffffffu, excl, r) - base;
+            const int nr = __shfl_sync(0xffffffffu, n, r);
+            const int p0 = 4 * (i - __shfl_sync(0xffffffffu, fours_from, r));
+            if (i < fours_all) {
+                float sa[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                for (int k = p0; k < nr; ++k) {
+                    const float ek = sm.e[ro + k], fa = sm.a[ro + k], fb = sm.z[ro + k];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (k >= p0 + u) {
+                            sa[u] += ek * fa;
+                            sb[u] += ek * fb;
+                        }
+                    }
                 }
-                if (err_out) err_out[(nb + r) * K + p] = sm.e[q];
-                tab[(nb + r) * K1 + p] = make_float2(sa, sb);
-                if (p < 2) {
-                    sm.t[q] = sa;
-                    sm.x[q] = sb;
+                float2* out = tab + (nb + r) * K1 + p0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (p0 + u < nr) out[u] = make_float2(sa[u], sb[u]);
+                if (p0 == 0) {
+                    sm.t[ro] = sa[0];
+                    sm.x[ro] = sb[0];
+                    if (nr > 1) {
+                        sm.t[ro + 1] = sa[1];
+                        sm.x[ro + 1] = sb[1];
+                    }
                 }
             }
         }
@@ -1034,7 +1063,7 @@ static int launch_prep_layer(const float* post_times, const float* a, const floa
 // The prep without factors (K <= 32), by the number of warps of 32 neurons. Up to twenty per SM: without counts the layer
 // kernel (no rounds and no search for the counts: 300 neurons, 256 samples, all 30 slots valid 46 us, 83 in the counted kernel; 10
 // neurons 21 / 40), with counts one warp per CTA, so that they spread over the SMs, and all 32 x 32 slots in one round (10
-// neurons, all valid 31 us, 56 in rounds of 128 slots; 800 neurons, 64 samples, 8.9 valid 29 / 40). Beyond, where the shared
+// neurons, all valid 25 us, 56 in rounds of 128 slots; 800 neurons, 64 samples, 8.9 valid 28 / 40). Beyond, where the shared
 // memory of whole rows leaves ten warps on an SM, the counted kernel with rounds of 128 slots, eight warps per CTA (800
 // neurons, 256 samples: 42 us, 46 in one round; without counts 54 / 64 in the layer kernel).
 static int launch_prep(const float* post_times, const int* n_spikes, const float* a, const float* x,
