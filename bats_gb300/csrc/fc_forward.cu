@@ -738,6 +738,7 @@ extern "C" int bats_lif_forward_fc_default_algo(int batch, int n_post, int ev_ca
     //   at most 8 neurons (three quarters of a tile idle): always (4 neurons, 4096 samples: 199 / 343)
     //   at most 16: 20 warps (12 neurons, 1024 samples 66 / 74, 168 / 164; 16 and 4096: 715 / 433, above the line)
     //   at most 32: 16 warps (32 neurons, 256 samples: 50 / 87, 118 / 148, 259 / 363; 512 samples: 214 / 160, above)
+    //     (output layers, which spike; silent ones pay: 24 neurons, 256 samples of 718 events 56 / 42)
     //   wider: 8 warps (131 neurons, 32 samples: 31 / 64, 70 / 156, 136 / 388; silent layers 15 / 21, 44 / 58; twice as
     //   many warps are still faster where the neurons spike, 52 / 70, 120 / 158, but not where they are silent, 79 / 58)
     const long long warps = (long long)batch * n_post;
