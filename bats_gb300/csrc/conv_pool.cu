@@ -1130,12 +1130,13 @@ static void conv_tile(int C_out, int threads, int& TX, int& TY) {
     TY = P / TX;
 }
 
-// A CTA has at least eight warps, which make the lists where few output channels use them, and at most 16 positions, whose lists
-// leave room for other CTAs (2 filters 5 x 5 over 28 x 28, 128 samples: 117 us with two warps and 32 positions, 57 so; 42
-// without lists; 3 filters 3 x 3 x 6 over 12 x 12: 115, 64 and 220). Larger tiles read the sample's events fewer times and share more of each receptive field; smaller ones give more CTAs
-// and shorter waits at the barriers. 512 threads pay only where a sample can carry many events (12 x 12 x 15 x 40 slots,
-// 768 CTAs: 0.76 ms, 256 threads 0.87; 28 x 28 x 1 slots: 0.099 ms, 256 threads 0.087) and the grid still fills two
-// CTAs on each of the 152 SMs; below that the tile is halved (42 CTAs of 512 threads: 0.142 ms, 168 of 128: 0.095).
+// A CTA has at least eight warps, which make the lists where few output channels use them, and at most 16 positions,
+// whose lists leave room for other CTAs (2 filters 5 x 5 over 28 x 28, 128 samples: 117 us with two warps and 32
+// positions, 57 so; 42 without lists; 3 filters 3 x 3 x 6 over 12 x 12: 115, 64 and 220). Larger tiles read the sample's
+// events fewer times and share more of each receptive field; smaller ones give more CTAs and shorter waits at the
+// barriers. 512 threads pay only where a sample can carry many events (12 x 12 x 15 x 40 slots, 768 CTAs: 0.76 ms, 256
+// threads 0.87; 28 x 28 x 1 slots: 0.099 ms, 256 threads 0.087) and the grid still fills two CTAs on each of the 152 SMs;
+// below that the tile is halved (42 CTAs of 512 threads: 0.142 ms, 168 of 128: 0.095).
 static void conv_plan(int batch, int Xo, int Yo, int C_out, long long ev_cap, int& TX, int& TY) {
     for (int threads = ev_cap >= 8192 ? 512 : 256;; threads /= 2) {
         conv_tile(C_out, threads, TX, TY);
