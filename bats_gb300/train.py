@@ -536,19 +536,20 @@ def enqueue_launches(launches, side, main, aux=None, join=()) -> None:
         return
     forks = set(side.values())
     events = {}
-    joined = False
+    apart = False  # launches on `aux` that `main` has not waited for (nothing to wait for: no work of a capture)
     for name, fn in launches:
         if name in side:
             aux.wait_event(events[side[name]])
             fn(aux.cuda_stream)
+            apart = True
             continue
-        if (name.endswith(".wt_copy") or name in join) and not joined:
+        if (name.endswith(".wt_copy") or name in join) and apart:
             main.wait_stream(aux)
-            joined = True
+            apart = False
         fn(sm)
         if name in forks:
             e = torch.cuda.Event()
             e.record(main)
             events[name] = e
-    if not joined:
+    if apart:
         main.wait_stream(aux)
