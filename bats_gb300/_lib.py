@@ -65,6 +65,8 @@ SIGNATURES = {
     "bats_cursor_heads_bytes": (c_size, [c_int, c_int]),
     "bats_backward_prep_counted": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_float, c_float,
                                            c_float, c_vp, c_vp, c_vp, c_vp]),
+    "bats_backward_prep_counted_clear": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_float, c_float,
+                                                 c_float, c_vp, c_vp, c_vp, c_vp]),
     "bats_backward_prep_readonly": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_float, c_float,
                                             c_float, c_vp, c_vp, c_vp, c_vp]),
     "bats_backward_prep_layer": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_float, c_float, c_float,

@@ -243,6 +243,8 @@ bwd_prep_layer_kernel(const float* __restrict__ t, const float* __restrict__ a, 
 // 365 -> 255 us (140 M); 800 neurons, 256 samples, 3510 spikes: 54 -> 40 us. Rounds of 128 slots (half the shared
 // memory, twice the warps) against 256: 255 / 335 and 41 / 40 us.
 // Without counts 475 k spikes of 300 neurons, 256 samples: 64 us with whole rows of K slots staged (ten warps an SM) -> 54 us.
+// clear: nvalid still holds the counts of the call before on the same buffers, and the errors from there down to the new
+// counts are set to 0 (the slots that lost their spike since; a fill of the whole array instead takes 7 us per 25 MB).
 template <int CAP>
 struct PrepCompact {
     float t[CAP], z[CAP], x[CAP], a[CAP], e[CAP];
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_spikes, const float* __restrict__ a,
                         const float* __restrict__ x, const float* __restrict__ z, const float* err, float* err_out,
                         long long total, int K, float c, float tau, float dtt, float2* __restrict__ tab,
-                        int* __restrict__ nvalid, float2* __restrict__ head_t, float4* __restrict__ head_ab) {
+                        int* __restrict__ nvalid, float2* __restrict__ head_t, float4* __restrict__ head_ab, bool clear) {
     pdl_prologue();
     __shared__ PrepCompact<CAP> sm_all[WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -264,6 +266,7 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
     if (nb >= total) return;
     const int cnt = (int)min(32LL, total - nb);
     const int K1 = K + 1;
+    const int n_before = clear && lane < cnt ? min(nvalid[nb + lane], K) : 0;
     int n_in = 0;
     if (n_spikes) {
         n_in = lane < cnt ? min(max(n_spikes[nb + lane], 0), K) : 0;
@@ -386,6 +389,7 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
         }
         __syncwarp();
         if (mine && lane < cnt) {
+            for (int k = n; k < n_before; ++k) err_out[(nb + lane) * K + k] = 0.0f;
             nvalid[nb + lane] = n;
             if (head_t) {
                 head_t[nb + lane] = make_float2(h_t0, h_t1);
@@ -1069,17 +1073,17 @@ static int launch_prep_layer(const float* post_times, const float* a, const floa
 static int launch_prep(const float* post_times, const int* n_spikes, const float* a, const float* x,
                        const float* post_exp_tau, const float* errors, float* errors_out, long long total, int k_post,
                        float c, float tau, float delta_theta_tau, void* tables, int* nvalid, void* cursor_heads,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, bool clear = false) {
     const long long warps = (total + 31) / 32;
     const CursorHeads h = cursor_heads_of(cursor_heads, total);
     if (warps > 20 * 152)
         BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<128, 8>, (unsigned)((warps + 7) / 8), 256, 0, stream, post_times,
             n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
-            reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab));
+            reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab, clear));
     else if (n_spikes)
         BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<1024, 1>, (unsigned)warps, 32, 0, stream, post_times,
             n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
-            reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab));
+            reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab, clear));
     else
         return launch_prep_layer(post_times, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau,
                                  delta_theta_tau, nullptr, nullptr, tables, nvalid, cursor_heads, stream);
@@ -1114,10 +1118,10 @@ extern "C" size_t bats_cursor_heads_bytes(int batch, int n_post) {
     return heads_times_bytes(pairs) + (size_t)pairs * sizeof(float4);
 }
 
-extern "C" int bats_backward_prep_counted(const float* post_times, const int* n_spikes, const float* a, const float* x,
-                                          const float* post_exp_tau, float* errors, int batch, int n_post, int k_post,
-                                          float c, float tau, float delta_theta_tau, void* tables, int* nvalid,
-                                          void* cursor_heads, cudaStream_t stream) {
+static int prep_counted_impl(const float* post_times, const int* n_spikes, const float* a, const float* x,
+                             const float* post_exp_tau, float* errors, int batch, int n_post, int k_post, float c,
+                             float tau, float delta_theta_tau, void* tables, int* nvalid, void* cursor_heads, bool clear,
+                             cudaStream_t stream) {
     BATS_REQUIRE(batch >= 0 && n_post >= 0 && k_post > 0, BATS_ERR_BAD_SHAPE, "backward_prep_counted: bad shape");
     BATS_REQUIRE(((uintptr_t)cursor_heads & 15) == 0, BATS_ERR_BAD_SHAPE,
                  "backward_prep_counted: cursor_heads not 16-byte aligned");
@@ -1127,7 +1131,23 @@ extern "C" int bats_backward_prep_counted(const float* post_times, const int* n_
     BATS_REQUIRE(post_times && n_spikes && a && x && post_exp_tau && errors && tables && nvalid, BATS_ERR_NULL,
                  "backward_prep_counted: null pointer");
     return launch_prep(post_times, n_spikes, a, x, post_exp_tau, errors, errors, total, k_post, c, tau, delta_theta_tau,
-                       tables, nvalid, cursor_heads, stream);
+                       tables, nvalid, cursor_heads, stream, clear);
+}
+
+extern "C" int bats_backward_prep_counted(const float* post_times, const int* n_spikes, const float* a,
+                                          const float* x, const float* post_exp_tau, float* errors, int batch,
+                                          int n_post, int k_post, float c, float tau, float delta_theta_tau,
+                                          void* tables, int* nvalid, void* cursor_heads, cudaStream_t stream) {
+    return prep_counted_impl(post_times, n_spikes, a, x, post_exp_tau, errors, batch, n_post, k_post, c, tau,
+                             delta_theta_tau, tables, nvalid, cursor_heads, false, stream);
+}
+
+extern "C" int bats_backward_prep_counted_clear(const float* post_times, const int* n_spikes, const float* a,
+                                                const float* x, const float* post_exp_tau, float* errors, int batch,
+                                                int n_post, int k_post, float c, float tau, float delta_theta_tau,
+                                                void* tables, int* nvalid, void* cursor_heads, cudaStream_t stream) {
+    return prep_counted_impl(post_times, n_spikes, a, x, post_exp_tau, errors, batch, n_post, k_post, c, tau,
+                             delta_theta_tau, tables, nvalid, cursor_heads, true, stream);
 }
 
 extern "C" int bats_backward_prep_readonly(const float* post_times, const float* a, const float* x,

@@ -68,10 +68,11 @@ class FCTrainStep:
             self.tabs.append(K.BackwardTables(torch.empty((B, N, Kp), dtype=f32, device=dev) if need_f else None,
                                               torch.empty((B, N, Kp), dtype=f32, device=dev) if need_f else None,
                                               torch.empty((B, N, Kp + 1, 2), dtype=f32, device=dev),
-                                              torch.empty((B, N), dtype=i32, device=dev),
+                                              torch.zeros((B, N), dtype=i32, device=dev),
                                               K.alloc_cursor_heads(B, N, dev) if not need_f else None))
             self.grad.append(torch.empty((N, n_prev), dtype=f32, device=dev))
-            # Only the slots of spikes are written and read; the others stay as they are.
+            # 0 at every slot without a spike: the pre-error launch writes the spikes' slots and the prep that reads them
+            # clears those that had a spike a step before (self.tabs' counts).
             self.pre_err.append(torch.zeros((B, n_prev, k_prev), dtype=f32, device=dev))
             n_prev, k_prev = N, Kp
         self.loss = torch.empty((B,), dtype=f32, device=dev)
@@ -175,7 +176,8 @@ class FCTrainStep:
             tag = f"L{li + 1}"
             if spec.max_n_spike <= 32:  # only the slots below the forward's spike counts are read
                 L.append((f"{tag}.prep", lambda s, o=self.out[li], e=errors, spec=spec, c=c, tau32=tau32, dtt=dtt,
-                          tb=tb: call("bats_backward_prep_counted", ptr(o[3]), ptr(o[0]), ptr(o[1]), ptr(o[2]),
+                          tb=tb, clear="_clear" if li + 1 < len(self.specs) else "":
+                          call("bats_backward_prep_counted" + clear, ptr(o[3]), ptr(o[0]), ptr(o[1]), ptr(o[2]),
                                       ptr(o[4]), ptr(e), B, spec.n_neurons, spec.max_n_spike, float(c),
                                       float(tau32), float(dtt), ptr(tb.tables), ptr(tb.nvalid), ptr(tb.heads), s)))
             else:
@@ -186,10 +188,11 @@ class FCTrainStep:
             if li > 0:
                 pe = self.pre_err[li]
                 L.append((f"{tag}.pre_err", lambda s, ev=ev, t=t, tb=tb, spec=spec, li=li, pe=pe, tau32=tau32: call(
-                    "bats_pre_errors_slots", ptr(ev.events), ptr(ev.slots), ptr(ev.counts), ev.cap, ptr(self.Wt[li]),
-                    self.Wt[li].shape[1], ptr(t), ptr(tb.tables), ptr(tb.nvalid), B, spec.n_neurons,
-                    spec.max_n_spike, ev.n_neurons, ev.k, float(np.float32(spec.tau_s)), float(tau32), ptr(pe), ws,
-                    wsb, s)))
+                    # (a layer of K > 32 has another prep, which clears nothing)
+                    "bats_pre_errors_slots" if ev.k <= 32 else "bats_pre_errors", ptr(ev.events), ptr(ev.slots),
+                    ptr(ev.counts), ev.cap, ptr(self.Wt[li]), self.Wt[li].shape[1], ptr(t), ptr(tb.tables),
+                    ptr(tb.nvalid), B, spec.n_neurons, spec.max_n_spike, ev.n_neurons, ev.k,
+                    float(np.float32(spec.tau_s)), float(tau32), ptr(pe), ws, wsb, s)))
                 errors = pe
             # Above the first layer: the staging copy of Wt and the second workspace (see __init__).
             wt_out = self.Wt_next[li] if li > 0 else self.Wt[li]

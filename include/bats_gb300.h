@@ -233,6 +233,13 @@ int bats_backward_prep_counted(const float* post_times, const int* n_spikes, con
                                const float* post_exp_tau, float* errors, int batch, int n_post, int k_post, float c,
                                float tau, float delta_theta_tau, void* tables, int* nvalid, void* cursor_heads,
                                cudaStream_t stream);
+/* The same for errors that bats_pre_errors_slots wrote: errors and nvalid are those that the call before left (both 0 before
+ * the first), and the errors between the new and the former nvalid are set to 0, so that the errors stay 0 at every slot
+ * past a neuron's spikes. */
+int bats_backward_prep_counted_clear(const float* post_times, const int* n_spikes, const float* a, const float* x,
+                                     const float* post_exp_tau, float* errors, int batch, int n_post, int k_post,
+                                     float c, float tau, float delta_theta_tau, void* tables, int* nvalid,
+                                     void* cursor_heads, cudaStream_t stream);
 /* The same without spike counts (a neuron's slots end at its first +inf time) and with the errors left as they are: only
  * the tables, nvalid and cursor_heads are written. For gradients that belong to the caller. */
 int bats_backward_prep_readonly(const float* post_times, const float* a, const float* x, const float* post_exp_tau,
@@ -300,7 +307,7 @@ int bats_pre_errors(const void* events, const int* ev_slot, const int* ev_count,
                     const float* weights_t, int ld, const float* post_times, const void* tables, const int* nvalid,
                     int batch, int n_post, int k_post, int n_pre, int k_pre, float tau_s, float tau,
                     float* pre_errors, void* workspace, size_t workspace_bytes, cudaStream_t stream);
-/* The same, writing only the slots of events: a layer's counted backward prep reads no other. */
+/* The same, writing only the slots of events; the others stay as they are (bats_backward_prep_counted_clear keeps them 0). */
 int bats_pre_errors_slots(const void* events, const int* ev_slot, const int* ev_count, long long ev_cap,
                     const float* weights_t, int ld, const float* post_times, const void* tables, const int* nvalid,
                     int batch, int n_post, int k_post, int n_pre, int k_pre, float tau_s, float tau,
