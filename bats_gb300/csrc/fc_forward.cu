@@ -212,6 +212,7 @@ __device__ __forceinline__ bool forward_tile_item(FwdSmem<TILE, SEV, STAGES>& sm
             if (!__all_sync(0xffffffffu, quiet)) break;
             a = aa;
             b = bb;
+            __syncwarp();  // every lane's reads of the slot come before its release
             if (lane == 0) mbar_arrive(&sm.empty[pos.slot]);
             pos.next();
         }
