@@ -163,7 +163,8 @@ constexpr int STOP_EVERY = 8;  // stages between two looks at whether every neur
 // crossing after any of the stage's events (784 -> 800 silent neurons, 256 samples: 46 -> 33 us). SCREEN: every full stage
 // is tried so first; otherwise it is evaluated as without SCREEN. The FMA sequence is the same either way, so results are
 // bit-identical. (Tries at growing distances all through the loop made active layers 2.5 % slower.)
-// A neuron with k_post spikes is done; a warp whose neurons are all done only passes stages on (see forward_produce).
+// A neuron with k_post spikes is done; a warp whose neurons are all done, or that has none, only passes stages on (see
+// forward_produce).
 //
 // What bounds it: instruction issue (76 % of the issue slots), 590 warp instructions per warp and 8-event stage of an
 // active 800 x 800 layer (batch 256, 652 events a sample, 1.4 spikes per warp and stage), 884 with a screen per
@@ -179,6 +180,19 @@ __device__ __forceinline__ bool forward_tile_item(FwdSmem<TILE, SEV, STAGES>& sm
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
     const int n_stages = (E + SEV - 1) / SEV;
+    if (tile0 + warp * 32 >= n_post) {  // no neuron (the last tile's warps): only passes stages on
+        if (lane == 0) *(volatile int*)&sm.finished[warp] = it;
+        for (int k = 0; k < n_stages; ++k) {
+            const bool ok = mbar_wait(&sm.full[pos.slot], pos.phase, &sm.abort, status);
+            if (!__all_sync(0xffffffffu, ok)) return false;
+            const bool stop = *(volatile int*)&sm.stop_at == pos.k;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.empty[pos.slot]);
+            pos.next();
+            if (stop) break;
+        }
+        return true;
+    }
     const int i = tile0 + tid;
     const bool active = i < n_post;
     const long long obase = ((long long)s * n_post + (active ? i : 0)) * k_post;
