@@ -26,7 +26,9 @@
 // Wrappers/Inference/aggregate_spikes_conv.py:10-28; backward bats/Layers/PoolingLayer.py:55-66):
 // a stable 4-way merge of the children's sorted spike lists, inf slots last in concatenation order.
 #include <cooperative_groups.h>
+#include <numeric>
 #include "common.cuh"
+#include "conv_form.cuh"
 #include "abi_util.h"
 
 namespace bats {
@@ -464,44 +466,61 @@ conv_backward_cluster_kernel(const Event* __restrict__ ev, const int* __restrict
 // Conv backward over events grouped by input position (the bucketed copy of the sort with
 // bucket_width = C: one bucket per (x, y), time order inside), on a cluster of CONV_BWD_CLUSTER CTAs per sample group
 // (position groups dealt to the ranks). Within a position group every filter tap sees one and the same post neuron
-// (x - dx, y - dy, co). Two kernels, whose results are the same bit for bit, run one after the other, and each cluster's samples
-// are taken by the one that its own count of spiking neurons makes the cheaper (ConvForm): no host knows it.
+// (x - dx, y - dy, co). Two kernels, whose results are the same bit for bit, run one after the other: the first, the taps form,
+// leaves the batch to the second, the events form, where few enough neurons spike (no host knows it).
 struct ConvBwdShape {
     int Y, C, fx, fy, C_out, Xo, Yo, k_pre, k_post, n_pos;
 };
 
-// TAPS: the taps form alone; CHOOSE: both are launched, and each cluster picks.
+// TAPS: the taps form alone; CHOOSE: both are launched, and the first decides.
 enum class ConvForm { TAPS, CHOOSE };
 
-// Whether the cluster's samples s0 .. s_end - 1 go to the events form: the pairs of a spiking tap and up to 32 events,
-// ~200 warp instructions each there, against ~20 per event and 32 taps in the taps form, whatever spikes. The line is drawn by
-// 40 filters 5 x 5 x 15, 128 samples, K 10 (taps / events form): at 0.19 pairs per event and tile 2.65 / 2.07 ms, at 0.77 1.43 /
-// 2.26; without pre-errors at 0.77 1.19 / 1.32; 64 filters 3 x 3 x 64 at 0.53 291 / 312 us. Uniform over the cluster; ends
-// with a barrier.
-template <bool PRE>
-__device__ __forceinline__ bool conv_events_form(const int* __restrict__ boff, const int* __restrict__ nvalid,
-                                                 const ConvBwdShape& sh, int s0, int s_end) {
-    __shared__ int s_spiking, s_events;
-    if (threadIdx.x == 0) s_spiking = s_events = 0;
-    __syncthreads();
-    const int n_post = sh.Xo * sh.Yo * sh.C_out;
-    const long long n = (long long)(s_end - s0) * n_post;
-    const int* nv = nvalid + (long long)s0 * n_post;
-    int spiking = 0, events = 0;
-#pragma unroll 4
-    for (long long q = threadIdx.x; q < n; q += blockDim.x) spiking += __ldg(nv + q) > 0 ? 1 : 0;
-    for (int s = s0 + threadIdx.x; s < s_end; s += blockDim.x)
-        events += __ldg(boff + (long long)s * (sh.n_pos + 1) + sh.n_pos);
+// Where the events form takes the batch, the taps form leaves this in the first word of every group's gradient, which the events
+// form overwrites: the decision is made in one kernel and read in the other. No gradient can look so: it is the result of an
+// addition, whose NaN is 0x7fffffff.
+constexpr unsigned CONV_LEFT = 0x7fc0b175u;
+
+// The decision (conv_events_pays) is the batch's, so that the kernels do not run their longest samples one after the other
+// (with pre-errors a choice per group took 0.917 of the taps form's time, one for the batch 0.885, mean of 2150 layers). Every CTA forms it from
+// the same sample of the batch, with no word between them: every nv_step-th neuron and every s_step-th sample.
+struct ConvVoteShape {
+    int nv_step, nv_count, s_step, s_count;
+};
+constexpr int CONV_VOTE = 1024;  // neurons and samples looked at, at most
+
+// In two halves around a barrier of the caller's, which the loads overlap with what else comes before it: the warps' counts,
+// then their sum. The same in every thread of the grid.
+struct ConvVote {
+    int spiking[32];
+    unsigned long long events[32];
+};
+__device__ __forceinline__ void conv_vote_count(ConvVote& v, const ConvVoteShape& vs, const int* __restrict__ boff,
+                                                const int* __restrict__ nvalid, const ConvBwdShape& sh) {
+    int spiking = 0;
+    unsigned long long events = 0;
+    for (int q = threadIdx.x; q < vs.s_count; q += blockDim.x)
+        events += (unsigned)__ldg(boff + (long long)q * vs.s_step * (sh.n_pos + 1) + sh.n_pos);
+#pragma unroll 8
+    for (int q = threadIdx.x; q < vs.nv_count; q += blockDim.x)
+        spiking += __ldg(nvalid + (long long)q * vs.nv_step) > 0 ? 1 : 0;
     spiking = __reduce_add_sync(0xffffffffu, spiking);
-    events = __reduce_add_sync(0xffffffffu, events);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) events += __shfl_xor_sync(0xffffffffu, events, o);
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&s_spiking, spiking);
-        atomicAdd(&s_events, events);
+        v.spiking[threadIdx.x >> 5] = spiking;
+        v.events[threadIdx.x >> 5] = events;
     }
-    __syncthreads();
-    const float ev = (float)s_events, tiles = (float)((sh.C_out * sh.fx * sh.fy + 31) / 32);
-    const float chunks = ev / (32.0f * (float)sh.n_pos * (float)(s_end - s0)) + 0.5f;  // of 32 events, per position
-    return (float)s_spiking * (float)(sh.fx * sh.fy) * chunks <= (PRE ? 0.4f : 0.6f) * ev * tiles;
+}
+__device__ __forceinline__ bool conv_events_form(const ConvVote& v, const ConvVoteShape& vs, const ConvBwdShape& sh,
+                                                 int batch, bool pre) {
+    const int lane = threadIdx.x & 31;
+    const bool on = lane < (int)(blockDim.x >> 5);
+    const unsigned spiking = __reduce_add_sync(0xffffffffu, on ? (unsigned)v.spiking[lane] : 0u);
+    unsigned long long events = on ? v.events[lane] : 0;
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) events += __shfl_xor_sync(0xffffffffu, events, o);
+    return conv_events_pays((unsigned long long)spiking * (unsigned)vs.nv_step, events * (unsigned)vs.s_step, batch, sh.n_pos,
+                            sh.C_out * sh.fx * sh.fy, sh.fx * sh.fy, pre);
 }
 
 // The taps form: a thread per filter tap. A tap's post neuron has its spike data set up once per position and is followed by
@@ -514,7 +533,7 @@ conv_backward_taps_kernel(const Event* __restrict__ ev_b, const int* __restrict_
                           const float* __restrict__ W, ConvBwdShape sh, const float* __restrict__ post_t,
                           const float2* __restrict__ tab, const int* __restrict__ nvalid, float tau_s, float tau,
                           long long pre_slots, float* __restrict__ grad, float* __restrict__ pre_err, int batch,
-                          int group, ConvForm form) {
+                          int group, ConvForm form, ConvVoteShape vs) {
     pdl_prologue();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -522,8 +541,9 @@ conv_backward_taps_kernel(const Event* __restrict__ ev_b, const int* __restrict_
     __shared__ Event sev[32];
     __shared__ float sred[32][33];
     __shared__ int sslot[32], scc[32];
+    __shared__ ConvVote vote;
     const int s0 = (int)blockIdx.y * group, s_end = min(batch, s0 + group);
-    if (form == ConvForm::CHOOSE && conv_events_form<PRE>(boff, nvalid, sh, s0, s_end)) return;
+    if (form == ConvForm::CHOOSE) conv_vote_count(vote, vs, boff, nvalid, sh);
     const float inv_tau_s = 1.0f / tau_s, inv_tau = 1.0f / tau;  // the error terms' factors, as reciprocals
     const int rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -546,6 +566,10 @@ conv_backward_taps_kernel(const Event* __restrict__ ev_b, const int* __restrict_
     const int co = has_tap ? tid / (sh.fx * sh.fy) : 0, dx = has_tap ? tid / sh.fy % sh.fx : 0;
     const int dy = has_tap ? tid % sh.fy : 0;
     __syncthreads();
+    if (form == ConvForm::CHOOSE && conv_events_form(vote, vs, sh, batch, PRE)) {  // uniform over the grid
+        if (rank == 0 && tid == 0) grad[(long long)blockIdx.y * total] = __uint_as_float(CONV_LEFT);
+        return;
+    }
     // The cluster's samples (one with group == 1: the per-sample gradient), accumulated in order.
     for (int s = s0; s < s_end; ++s) {
         const int* bo = boff + (long long)s * (sh.n_pos + 1);
@@ -662,7 +686,8 @@ conv_backward_grouped_kernel(const Event* __restrict__ ev_b, const int* __restri
     extern __shared__ __align__(16) float4 cb_smem[];
     __shared__ int s_beg[CONV_BWD_POS], s_len[CONV_BWD_POS], s_at[CONV_BWD_POS], s_next;
     const int s0 = (int)blockIdx.y * group, s_end = min(batch, s0 + group);
-    if (!conv_events_form<PRE>(boff, nvalid, sh, s0, s_end)) return;
+    // Every CTA reads the word before its first barrier of the cluster, and the gradient is written after it.
+    if (__float_as_uint(grad[(long long)blockIdx.y * sh.C_out * sh.fx * sh.fy * sh.C]) != CONV_LEFT) return;
     const float inv_tau_s = 1.0f / tau_s, inv_tau = 1.0f / tau;  // the error terms' factors, as reciprocals
     const int rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1251,9 +1276,10 @@ static auto* conv_grouped_kernel(int k_post) {
                           : bats::conv_backward_grouped_kernel<true, 4, PRE, W_SMEM>;
 }
 
-// From so many filter taps on the events form is worth a second launch (its clusters that do not take part cost a few us):
-// 216 taps, 21 samples, few spiking 120 -> 62 us; 72 taps all spiking 44 us, and 81 in the events form.
-constexpr long long CONV_EVENTS_TAPS = 192;
+// From so many filter taps, and slots x tiles of 32 taps, on the events form is worth a second launch (a few us where no group
+// takes it): 216 taps, 21 samples, few spiking 120 -> 62 us; 72 taps all spiking 44 us, and 81 in the events form. Below 10^4
+// slots x tiles the times with it are 1.04 of those without (mean of 420 layers, 0.91 above).
+constexpr long long CONV_EVENTS_TAPS = 192, CONV_EVENTS_WORK = 10000;
 
 static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* bucket_offsets, long long ev_cap,
                                        const float* weights, const bats::ConvBwdShape& sh, const float* post_times,
@@ -1261,7 +1287,8 @@ static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* b
                                        long long pre_slots, float* grad, float* pre_errors, int batch, int group,
                                        cudaStream_t stream) {
     const long long taps = (long long)sh.C_out * sh.fx * sh.fy;
-    const bool pre = pre_errors != nullptr, choose = taps >= CONV_EVENTS_TAPS;
+    const bool pre = pre_errors != nullptr;
+    const bool choose = taps >= CONV_EVENTS_TAPS && ev_cap * ((taps + 31) / 32) >= CONV_EVENTS_WORK;
     const int groups = (batch + group - 1) / group;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(bats::CONV_BWD_CLUSTER, groups);
@@ -1286,9 +1313,17 @@ static cudaError_t launch_conv_grouped(const void* events_bucketed, const int* b
         if (e != cudaSuccess) return e;
         cfg.blockDim = dim3((unsigned)((taps + 31) / 32 * 32));
         cfg.dynamicSmemBytes = smem;
+        // Steps that share no factor with the neurons of a sample, so that every channel and position comes up.
+        const long long neurons = (long long)batch * sh.Xo * sh.Yo * sh.C_out;
+        bats::ConvVoteShape vs;
+        vs.nv_step = (int)((neurons + bats::CONV_VOTE - 1) / bats::CONV_VOTE);
+        while (std::gcd(vs.nv_step, sh.Xo * sh.Yo * sh.C_out) != 1) ++vs.nv_step;
+        vs.nv_count = (int)((neurons + vs.nv_step - 1) / vs.nv_step);
+        vs.s_step = (batch + bats::CONV_VOTE - 1) / bats::CONV_VOTE;
+        vs.s_count = (batch + vs.s_step - 1) / vs.s_step;
         e = cudaLaunchKernelEx(&cfg, kernel, ev, bucket_offsets, ev_cap, weights, sh, post_times, tab, nvalid, tau_s, tau,
                                pre_slots, grad, pre_errors, batch, group,
-                               choose ? bats::ConvForm::CHOOSE : bats::ConvForm::TAPS);
+                               choose ? bats::ConvForm::CHOOSE : bats::ConvForm::TAPS, vs);
         if (e != cudaSuccess || !choose) return e;
     }
     constexpr size_t LIMIT = 224 * 1024;
