@@ -22,8 +22,9 @@ import numpy as np
 import torch
 
 from . import kernels as K
+from ._gc import no_collection
 from ._lib import call, ptr, stream_ptr
-from .train import FCLayerSpec, enqueue_launches, no_collection
+from .train import FCLayerSpec, enqueue_launches
 
 
 @dataclass

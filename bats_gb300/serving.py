@@ -20,9 +20,7 @@ tests/test_gpu_serving.py checks bit for bit.
 from __future__ import annotations
 
 import collections
-import contextlib
 import ctypes
-import gc
 import time
 from dataclasses import dataclass, field
 from typing import Deque, Dict, List, Optional, Sequence
@@ -31,22 +29,9 @@ import numpy as np
 import torch
 
 from . import kernels as K
+from ._gc import no_collection as no_gc_pauses
 from ._lib import BatsFcLayer, call, ptr
 from .autotune import Autotuner, get_tuner
-
-
-@contextlib.contextmanager
-def no_gc_pauses():
-    """Automatic garbage collection off while serving (restored afterwards): a generation-2 collection
-    over the tens of thousands of request and result objects of a busy loop stops the host for about
-    30 ms, which shows up directly in the latency tail. The serving objects hold no reference cycles."""
-    was = gc.isenabled()
-    gc.disable()
-    try:
-        yield
-    finally:
-        if was:
-            gc.enable()
 
 
 @dataclass

@@ -10,8 +10,6 @@ its hidden layers (self.out) hold valid times only below their spike counts (no 
 """
 from __future__ import annotations
 
-import contextlib
-import gc
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
@@ -19,6 +17,7 @@ import numpy as np
 import torch
 
 from . import kernels as K
+from ._gc import no_collection
 from ._lib import call, ptr, stream_ptr
 from .autotune import Autotuner, get_tuner
 
@@ -509,20 +508,6 @@ class FCTrainStep:
     @property
     def d2h_bytes(self) -> int:
         return self.h_loss.numel() * 4
-
-
-@contextlib.contextmanager
-def no_collection():
-    """Automatic garbage collection off (restored afterwards): a collection during a graph capture may free an older
-    step (its launch list holds it in a reference cycle) with its CUDA graph, and the calls that frees it with
-    invalidate the capture."""
-    was = gc.isenabled()
-    gc.disable()
-    try:
-        yield
-    finally:
-        if was:
-            gc.enable()
 
 
 def enqueue_launches(launches, side, main, aux=None, join=()) -> None:
