@@ -2,9 +2,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
-#include <utility>
 #include "abi_util.h"
 
 namespace bats {
@@ -25,13 +23,29 @@ int max_dynamic_smem_set(const void* func, int bytes) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     static std::mutex mu;
-    static std::map<std::pair<const void*, int>, int> largest;
+    struct Entry {
+        const void* f;
+        int dev, bytes;
+    };
+    static Entry kept[512];  // no allocation: nothing to throw through a C entry
+    static int used = 0;
     std::lock_guard<std::mutex> lock(mu);
-    int& have = largest[{func, dev}];
-    if (have >= bytes) return (int)cudaSuccess;
+    Entry* k = kept;
+    while (k < kept + used && !(k->f == func && k->dev == dev)) ++k;
+    if (k < kept + used && k->bytes >= bytes) return (int)cudaSuccess;
+    if (k == kept + used && used == 512) {
+        // Not remembered: never below the limit that another call may have set.
+        cudaFuncAttributes a;
+        e = cudaFuncGetAttributes(&a, func);
+        if (e != cudaSuccess) return (int)e;
+        if (a.maxDynamicSharedSizeBytes >= bytes) return (int)cudaSuccess;
+        return (int)cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    }
     e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) have = bytes;
-    return (int)e;
+    if (e != cudaSuccess) return (int)e;
+    if (k == kept + used) *k = Entry{func, dev, 0}, ++used;
+    k->bytes = bytes;
+    return (int)cudaSuccess;
 }
 
 bool pdl_enabled() {
