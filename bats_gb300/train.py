@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from . import kernels as K
-from ._gc import no_collection
+from ._gc import free_outside_captures, no_collection
 from ._lib import call, ptr, stream_ptr
 from .autotune import Autotuner, get_tuner
 
@@ -375,6 +375,7 @@ class FCTrainStep:
             torch.cuda.current_stream().wait_stream(side)
             torch.cuda.synchronize()
             self.graph = g
+            free_outside_captures(self, g)
             return True
         except Exception as exc:  # pragma: no cover - reported by the caller
             self.graph = None
