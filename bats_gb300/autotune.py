@@ -1,7 +1,8 @@
 """Autotuner for the kernel variants: picks, per shape and GPU, the variant that runs fastest on the
 caller's own buffers, and caches the choice.
 
-Tuned today: the FC forward kernel (tile: CTA per post-neuron tile and sample, producer warp streaming
+Tuned today: the FC forward kernel (auto: what the library takes by itself for the shape, which may be a tile that no other
+name stands for; tile: CTA per post-neuron tile and sample, producer warp streaming
 weight rows; lanes: warp per post neuron and sample, 32 events evaluated at once; queue: persistent CTAs
 over a longest-first work queue; the tile and queue kinds with or without the per-stage no-crossing
 screen) and the number of
@@ -10,17 +11,21 @@ results (the forward variants bit for bit, the gradient up to the order of the p
 choice only changes speed.
 
 The cache is a JSON file (BATS_GB300_AUTOTUNE, default ~/.cache/bats_gb300/autotune.json) keyed by the
-kind of kernel, the shape and the GPU (name and SM count); set BATS_GB300_AUTOTUNE=off to keep it in
-memory only.
+kind of kernel, the library build (a choice timed on other kernels says nothing), the shape and the GPU
+(name and SM count); set BATS_GB300_AUTOTUNE=off to keep it in memory only.
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 import threading
 from typing import Callable, Dict, Optional
 
 import torch
+
+from . import _lib
 
 _LOCK = threading.Lock()
 
@@ -30,6 +35,21 @@ def _default_path() -> Optional[str]:
     if p == "off":
         return None
     return p or os.path.join(os.path.expanduser("~"), ".cache", "bats_gb300", "autotune.json")
+
+
+@functools.lru_cache(maxsize=None)
+def _digest(path: str, mtime_ns: int, size: int) -> str:
+    with open(path, "rb") as f:
+        return hashlib.sha256(f.read()).hexdigest()[:12]
+
+
+def build_tag() -> str:
+    """Of the library's file: its contents, read once per process and file."""
+    try:
+        st = os.stat(_lib.LIB_PATH)
+        return "lib" + _digest(_lib.LIB_PATH, st.st_mtime_ns, st.st_size)
+    except OSError:
+        return "lib-"
 
 
 class Autotuner:
@@ -51,7 +71,7 @@ class Autotuner:
         return f"{p.name}|sm{p.multi_processor_count}"
 
     def key(self, kind: str, *shape) -> str:
-        return "|".join([kind, self.device_tag()] + [str(int(v)) for v in shape])
+        return "|".join([kind, build_tag(), self.device_tag()] + [str(int(v)) for v in shape])
 
     def _save(self) -> None:
         if not self.path:
