@@ -56,52 +56,9 @@ struct SortShared {
     int warp_tot[T / 32];
     int appended;         // items found (gather_items)
     unsigned kmin, kmax;  // their smallest and largest key
-    int pad_;             // the items behind are read as uint4
+    unsigned pairs;       // sum of the squares of the bucket sizes (bucket_sort); the items behind are read as uint4
 };
 static_assert(sizeof(SortShared<256>) % 16 == 0 && sizeof(SortShared<512>) % 16 == 0, "uint4 reads of the items");
-
-template <int T>
-__device__ __forceinline__ int block_exclusive_flag_scan(bool f, SortShared<T>& sh, int& block_total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned bal = __ballot_sync(0xffffffffu, f);
-    const int in_warp = __popc(bal & lanemask_lt());
-    if (lane == 0) sh.warp_tot[warp] = __popc(bal);
-    __syncthreads();
-    int off = 0, tot = 0;
-#pragma unroll
-    for (int w = 0; w < T / 32; ++w) {
-        const int c = sh.warp_tot[w];
-        off += (w < warp) ? c : 0;
-        tot += c;
-    }
-    __syncthreads();
-    block_total = tot;
-    return off + in_warp;
-}
-
-// Block-wide exclusive scan of one int per thread (in thread order); block_total gets the sum.
-template <int T>
-__device__ __forceinline__ int block_exclusive_scan(int v, SortShared<T>& sh, int& block_total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) sh.warp_tot[warp] = incl;
-    __syncthreads();
-    int off = 0, tot = 0;
-#pragma unroll
-    for (int w = 0; w < T / 32; ++w) {
-        const int c = sh.warp_tot[w];
-        off += (w < warp) ? c : 0;
-        tot += c;
-    }
-    __syncthreads();
-    block_total = tot;
-    return off + incl - v;
-}
 
 // Exclusive scan of sh.hist (SORT_BINS bins, one per thread tid < SORT_BINS) into sh.base; clears sh.wcnt.
 template <int T>
@@ -174,22 +131,6 @@ __device__ __forceinline__ void stable_pass(const uint32_t* ka, const V* va, uin
         }
     }
     __syncthreads();
-}
-
-// Valid (finite) times among the first pre_counts[j] slots of pre neuron j (loads eight at a time, so that a
-// thread's scattered loads are in flight together).
-__device__ __forceinline__ int leading_valid(const int* cnt_src, const float* tsrc, int j, int k_pre) {
-    const int c = min(max(cnt_src[j], 0), k_pre);
-    const float* tj = tsrc + (long long)j * k_pre;
-    int v = 0;
-    for (int q0 = 0; q0 < c; q0 += 8) {
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int q = q0 + u;
-            if (q < c) v += tj[q] < BATS_INF;
-        }
-    }
-    return v;
 }
 
 __device__ __forceinline__ Event make_event(uint32_t key, uint32_t slot, int k_pre, long long sample_off,
@@ -320,12 +261,16 @@ __device__ __forceinline__ int time_bucket(uint32_t key, float t_min, float scal
     return (int)fminf((key_to_float(key) - t_min) * scale, (float)(buckets - 1));
 }
 
-constexpr int SORT_BUCKET_LIMIT = 384;  // items of one bucket up to which ranking them by comparison is taken
+// Comparisons per item up to which ranking inside the buckets is taken, against a radix sort of a second list in slot order. 54
+// samples of 5500 items, times on a grid of 200 / 100 / 50 steps (27, 55 and 110 comparisons): 43, 58 and 86 us by
+// comparison, 53 by radix; 8 samples of 11200 on 500 / 200 steps: 74 and 107, 104; 256 of 2400 on 50 / 20: 44 and 68, 58. (With up
+// to 384 items in any bucket: 238 us on 20 steps, where the radix sort alone takes 72.)
+constexpr unsigned SORT_COMPARISONS = 48;
 
 // Sorts the n gathered items (ka, va) by (key, slot) with (kb, vb) as the second buffer, leaving them in (ka, va):
 // the items are dealt into buckets of equal time spans, and each finds its place inside its bucket by counting the
 // smaller ones. Six barriers whatever n, against three per 512 items and pass of a radix sort. False (nothing sorted)
-// when one bucket holds more than SORT_BUCKET_LIMIT items or the times span no finite range.
+// when that takes more than SORT_COMPARISONS comparisons per item (times on a coarse grid, or crowded by an outlier).
 template <int T, typename V>
 __device__ __forceinline__ bool bucket_sort(uint32_t* ka, V* va, uint32_t* kb, V* vb, int n, SortShared<T>& sh) {
     constexpr int NB = T / 32 * SORT_BINS;  // as many buckets as the counters of the counting passes hold
@@ -334,30 +279,35 @@ __device__ __forceinline__ bool bucket_sort(uint32_t* ka, V* va, uint32_t* kb, V
     int* count = &sh.wcnt[0][0];
     int* start = &sh.wofs[0][0];
     const float t_min = key_to_float(sh.kmin), span = key_to_float(sh.kmax) - t_min;
-    const bool usable = span > 0.0f && span <= 3.0e38f;  // uniform
+    const bool usable = span > 0.0f && span <= 3.0e38f;  // uniform; else all items are in one bucket
     const float scale = usable ? fminf((float)NB / span, 3.0e38f) : 0.0f;
     for (int q = tid; q < NB; q += T) count[q] = 0;
+    if (tid == 0) sh.pairs = 0u;
     __syncthreads();
-    if (!usable && n > SORT_BUCKET_LIMIT) return false;
     for (int i = tid; i < n; i += T) atomicAdd(&count[time_bucket(ka[i], t_min, scale, NB)], 1);
     __syncthreads();
     // Exclusive scan: thread tid owns buckets PER * tid ..
     int own[PER], sum = 0;
-    bool over = false;
+    unsigned pairs = 0u;  // n^2 at most, below 2^32 for what fits in shared memory
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
         own[u] = count[PER * tid + u];
-        over |= own[u] > SORT_BUCKET_LIMIT;
+        pairs += (unsigned)(own[u] * own[u]);
         sum += own[u];
     }
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
     }
-    if (lane == 31) sh.warp_tot[warp] = incl;
-    if (__syncthreads_or(over)) return false;
+    if (lane == 31) {
+        sh.warp_tot[warp] = incl;
+        atomicAdd(&sh.pairs, pairs);
+    }
+    __syncthreads();
+    if (sh.pairs > SORT_COMPARISONS * (unsigned)n) return false;
     int base = incl - sum;
     for (int w = 0; w < warp; ++w) base += sh.warp_tot[w];
 #pragma unroll
@@ -391,38 +341,103 @@ __device__ __forceinline__ bool bucket_sort(uint32_t* ka, V* va, uint32_t* kb, V
     return true;
 }
 
-struct SlotDigit {
-    int shift;
-    __device__ int operator()(uint32_t, uint32_t slot) const { return (int)((slot >> shift) & 255u); }
-};
+// The sample's valid slots as a list in slot order: a contiguous range of slots per warp, counted, then written. With the
+// pre layer's spike counts the lanes are neurons and read the slots below their counts, else the lanes are slots; eight
+// loads in flight per lane.
+template <int T, typename V>
+__device__ __forceinline__ void compact_slots(const float* __restrict__ tsrc, const int* __restrict__ cnt_src, int n_slots,
+                                              int k_pre, uint32_t* keys, V* vals, SortShared<T>& sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rows = cnt_src ? n_slots / k_pre : n_slots;
+    const int per = ((rows + 31) / 32 + T / 32 - 1) / (T / 32) * 32;
+    const int lo = min(rows, warp * per), hi = min(rows, lo + per);
+    auto put = [&](int pos, float t, int slot) {
+        keys[pos] = float_to_key(t);
+        vals[pos] = (V)slot;
+    };
+    // f(time, slot) for the valid slots of neuron j in order.
+    auto each = [&](int j, auto f) {
+        const int c = j < hi ? min(cnt_src[j], k_pre) : 0;
+        for (int q0 = 0; q0 < c; q0 += 8) {
+            float t[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) t[u] = q0 + u < c ? tsrc[j * k_pre + q0 + u] : BATS_INF;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (t[u] < BATS_INF) f(t[u], j * k_pre + q0 + u);
+        }
+    };
+    int c = 0;
+    if (cnt_src) {
+        for (int r = lo; r < hi; r += 32) each(r + lane, [&](float, int) { ++c; });
+    } else {
+#pragma unroll 8
+        for (int q = lo + lane; q < hi; q += 32) c += tsrc[q] < BATS_INF ? 1 : 0;
+    }
+    c = (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
+    if (lane == 0) sh.warp_tot[warp] = c;
+    __syncthreads();
+    int base = 0;
+    for (int w = 0; w < warp; ++w) base += sh.warp_tot[w];
+    if (cnt_src) {
+        for (int r = lo; r < hi; r += 32) {
+            int mine = 0;
+            each(r + lane, [&](float, int) { ++mine; });
+            int incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            int pos = base + incl - mine;
+            each(r + lane, [&](float t, int slot) { put(pos++, t, slot); });
+            base += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    } else {
+        for (int q0 = lo; q0 < hi; q0 += 8 * 32) {
+            float t[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int q = q0 + 32 * u + lane;
+                t[u] = q < hi ? tsrc[q] : BATS_INF;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const unsigned valid = __ballot_sync(0xffffffffu, t[u] < BATS_INF);
+                if (t[u] < BATS_INF) put(base + __popc(valid & lanemask_lt()), t[u], q0 + 32 * u + lane);
+                base += __popc(valid);
+            }
+        }
+    }
+    __syncthreads();
+}
 
-// LSD radix sort of the items by (digits of the slot, if SLOTS, then) the time key, 8 bits a pass; passes whose digit is
-// uniform are skipped. With SLOTS the result does not depend on the order the items came in; without, ties keep it.
-template <int T, typename V, bool SLOTS>
+// LSD radix sort of the items by the time key, 8 bits a pass; passes whose digit is uniform are skipped. Ties keep their order.
+template <int T, typename V>
 __device__ __forceinline__ void radix_sort(uint32_t*& ka, V*& va, uint32_t*& kb, V*& vb, int n, SortShared<T>& sh) {
     const int tid = threadIdx.x;
-    for (int pass = SLOTS ? -(int)sizeof(V) : 0; pass < 4; ++pass) {
-        const int shift = pass < 0 ? (pass + (int)sizeof(V)) * 8 : pass * 8;
+    for (int shift = 0; shift < 32; shift += 8) {
         if (tid < SORT_BINS) sh.hist[tid] = 0;
         __syncthreads();
-        for (int i = tid; i < n; i += T)
-            atomicAdd(&sh.hist[((pass < 0 ? (uint32_t)va[i] : ka[i]) >> shift) & 255u], 1);
+        for (int i = tid; i < n; i += T) atomicAdd(&sh.hist[(ka[i] >> shift) & 255u], 1);
         __syncthreads();
         if (__syncthreads_or(tid < SORT_BINS && sh.hist[tid] == n)) continue;
         scan_bins<T>(sh);
-        if (pass < 0)
-            stable_pass<T>(ka, va, kb, vb, n, sh, SlotDigit{shift});
-        else
-            stable_pass<T>(ka, va, kb, vb, n, sh, TimeDigit{shift});
+        stable_pass<T>(ka, va, kb, vb, n, sh, TimeDigit{shift});
         uint32_t* t0 = ka; ka = kb; kb = t0;
         V* t1 = va; va = vb; vb = t1;
     }
 }
 
 // V: type of the slot values (uint16_t when n_slots <= 65536). smem_cap: items held in shared memory.
-// Samples of up to smem_cap valid slots: gathered into shared memory in any order, then bucket_sort (or, where the times
-// crowd too much, radix_sort over slot and time). Larger ones: compacted in slot order into the global scratch and
-// sorted there by radix_sort over the time alone. The order is by time, ties by slot, either way.
+// Samples of up to smem_cap valid slots: gathered into shared memory in any order, then bucket_sort. Where the times crowd too
+// much for it, or in the global scratch where the sample is larger: compacted in slot order, then radix_sort. The order is by
+// time, ties by slot, either way.
+template <typename V>
+struct __align__(4 * sizeof(V)) Quad {
+    V x, y, z, w;
+};
+
 template <typename V, int T>
 __global__ void __launch_bounds__(T)
 sort_events_kernel(const float* __restrict__ times, const int* __restrict__ pre_counts, int n_slots, int k_pre,
@@ -474,73 +489,33 @@ sort_events_kernel(const float* __restrict__ times, const int* __restrict__ pre_
         const uint32_t key = tid < n ? ka[tid] : 0u;
         const V val = tid < n ? va[tid] : V(0);
         if (tid < n) {
-            int rank = 0, same = 0;
+            // By time and slot as one 64-bit number (the keys past n are larger than any time's).
+            const unsigned long long mine = (unsigned long long)key << 32 | val;
+            auto before = [&](uint32_t k, V v) { return ((unsigned long long)k << 32 | v) < mine ? 1 : 0; };
+            int rank = 0;
             const uint4* k4 = reinterpret_cast<const uint4*>(ka);
+            const Quad<V>* v4 = reinterpret_cast<const Quad<V>*>(va);
 #pragma unroll 2
             for (int q = 0; q < (n + 3) >> 2; ++q) {
                 const uint4 k = k4[q];
-                rank += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
-                same += (k.x == key) + (k.y == key) + (k.z == key) + (k.w == key);
+                const Quad<V> v = v4[q];
+                rank += before(k.x, v.x) + before(k.y, v.y) + before(k.z, v.z) + before(k.w, v.w);
             }
-            if (same > 1)  // equal times: by slot
-                for (int q = 0; q < n; ++q) rank += (ka[q] == key && va[q] < val) ? 1 : 0;
             kb[rank] = key;
             vb[rank] = val;
         }
         __syncthreads();
         uint32_t* t0 = ka; ka = kb; kb = t0;
         V* t1 = va; va = vb; vb = t1;
-    } else if (n <= smem_cap) {
-        if (!bucket_sort<T, V>(ka, va, kb, vb, n, sh)) radix_sort<T, V, true>(ka, va, kb, vb, n, sh);
-    } else {
-        // Two key and two value buffers in this sample's part of the global scratch (cap items each); compaction in
-        // slot order (stable).
-        ka = reinterpret_cast<uint32_t*>(scratch + (long long)s * cap * (8 + 2 * sizeof(V)));
-        kb = ka + cap;
-        va = reinterpret_cast<V*>(kb + cap);
-        vb = va + cap;
-        int base = 0;
-        if (cnt_src) {
-            // Thread per pre neuron, rounds of SORT_THREADS neurons; each copies its leading valid slots.
-            for (int r0 = 0; r0 < n_pre; r0 += SORT_THREADS) {
-                const int j = r0 + tid;
-                const int c = j < n_pre ? leading_valid(cnt_src, tsrc, j, k_pre) : 0;
-                int tot;
-                int pos = base + block_exclusive_scan(c, sh, tot);
-                const int slot0 = j * k_pre;
-                const int lim = c > 0 ? min(max(cnt_src[j], 0), k_pre) : 0;
-                for (int q0 = 0; q0 < lim; q0 += 8) {
-                    float tv[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) tv[u] = q0 + u < lim ? tsrc[slot0 + q0 + u] : BATS_INF;
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        if (tv[u] < BATS_INF) {
-                            ka[pos] = float_to_key(tv[u]);
-                            va[pos] = (V)(slot0 + q0 + u);
-                            ++pos;
-                        }
-                    }
-                }
-                base += tot;
-            }
-        } else {
-            for (int r0 = 0; r0 < n_slots; r0 += SORT_THREADS) {
-                const int slot = r0 + tid;
-                float t = BATS_INF;
-                if (slot < n_slots) t = tsrc[slot];
-                const bool f = t < BATS_INF;
-                int tot;
-                const int pos = block_exclusive_flag_scan(f, sh, tot);
-                if (f) {
-                    ka[base + pos] = float_to_key(t);
-                    va[base + pos] = (V)slot;
-                }
-                base += tot;
-            }
+    } else if (n > smem_cap || !bucket_sort<T, V>(ka, va, kb, vb, n, sh)) {
+        if (n > smem_cap) {  // two key and two value buffers in this sample's part of the global scratch (cap items each)
+            ka = reinterpret_cast<uint32_t*>(scratch + (long long)s * cap * (8 + 2 * sizeof(V)));
+            kb = ka + cap;
+            va = reinterpret_cast<V*>(kb + cap);
+            vb = va + cap;
         }
-        __syncthreads();
-        radix_sort<T, V, false>(ka, va, kb, vb, n, sh);
+        compact_slots<T, V>(tsrc, cnt_src, n_slots, k_pre, ka, va, sh);
+        radix_sort<T, V>(ka, va, kb, vb, n, sh);
     }
 
     Event* eo = ev_out + (long long)s * cap;
