@@ -512,7 +512,7 @@ __device__ __forceinline__ void conv_vote_count(ConvVote& v, const ConvVoteShape
     }
 }
 __device__ __forceinline__ bool conv_events_form(const ConvVote& v, const ConvVoteShape& vs, const ConvBwdShape& sh,
-                                                 int batch, bool pre) {
+                                                 int batch) {
     const int lane = threadIdx.x & 31;
     const bool on = lane < (int)(blockDim.x >> 5);
     const unsigned spiking = __reduce_add_sync(0xffffffffu, on ? (unsigned)v.spiking[lane] : 0u);
@@ -520,7 +520,7 @@ __device__ __forceinline__ bool conv_events_form(const ConvVote& v, const ConvVo
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) events += __shfl_xor_sync(0xffffffffu, events, o);
     return conv_events_pays((unsigned long long)spiking * (unsigned)vs.nv_step, events * (unsigned)vs.s_step, batch, sh.n_pos,
-                            sh.C_out * sh.fx * sh.fy, sh.fx * sh.fy, pre);
+                            sh.C_out * sh.fx * sh.fy, sh.fx * sh.fy);
 }
 
 // The taps form: a thread per filter tap. A tap's post neuron has its spike data set up once per position and is followed by
@@ -566,7 +566,7 @@ conv_backward_taps_kernel(const Event* __restrict__ ev_b, const int* __restrict_
     const int co = has_tap ? tid / (sh.fx * sh.fy) : 0, dx = has_tap ? tid / sh.fy % sh.fx : 0;
     const int dy = has_tap ? tid % sh.fy : 0;
     __syncthreads();
-    if (form == ConvForm::CHOOSE && conv_events_form(vote, vs, sh, batch, PRE)) {  // uniform over the grid
+    if (form == ConvForm::CHOOSE && conv_events_form(vote, vs, sh, batch)) {  // uniform over the grid
         if (rank == 0 && tid == 0) grad[(long long)blockIdx.y * total] = __uint_as_float(CONV_LEFT);
         return;
     }

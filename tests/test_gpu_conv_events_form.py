@@ -53,7 +53,7 @@ def test_events_form_equals_taps_form(cuda, rule, X, Y, C, C_out, k, K_post, the
     taps, spiking = C_out * FX * FY, int((tabs.nvalid > 0).sum())
     assert taps >= 192 and ev.cap * (taps // 32) >= 10000
     for room in (0.6, 1.6):
-        form = rule(int(spiking * room), int(ev.counts.sum()), B, X * Y, taps, FX * FY, want_pre)
+        form = rule(int(spiking * room), int(ev.counts.sum()), B, X * Y, taps, FX * FY)
         if few:
             assert form
         elif X > 3 and room < 1:  # (the small layer is nearly all edge: its line lies past all neurons)
