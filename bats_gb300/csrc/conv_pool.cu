@@ -27,7 +27,9 @@
 // a stable 4-way merge of the children's sorted spike lists, inf slots last in concatenation order.
 #include <cooperative_groups.h>
 #include <numeric>
+#include <type_traits>
 #include "common.cuh"
+#include "async_copy.cuh"
 #include "conv_form.cuh"
 #include "abi_util.h"
 
@@ -39,17 +41,16 @@ struct __align__(16) ConvEvent {
     int xyc;  // x | y << 10 | c << 20; bit 31: an exponential is not finite (relevant to every neuron)
 };
 
-constexpr int CONV_SUB = 64;               // kept events per round of the lists
 constexpr int CONV_GROUP = 8;              // list entries per pass of the screen
-constexpr int CONV_LIST = CONV_SUB + CONV_GROUP;
 constexpr int CONV_POSITIONS = 16;         // positions per CTA at most (2.9 KB of list each)
 
 // One position's list of relevant events, in time order: window constants (the window ends at the next relevant
-// event), times and filter rows ((dx fy + dy) C + c, or -1: weight 0).
+// event), times and filter rows ((dx fy + dy) C + c, or -1: weight 0). SUB: kept events per round of the lists.
+template <int SUB>
 struct ConvList {
-    CrossWindow win[CONV_LIST];
-    float t[CONV_LIST + 1];
-    int row[CONV_LIST];
+    CrossWindow win[SUB + CONV_GROUP];
+    float t[SUB + CONV_GROUP + 1];
+    int row[SUB + CONV_GROUP];
     int n;       // entries
     int groups;  // groups of CONV_GROUP entries that may be processed (the last entry waits for its window's end)
     int pad_[5];
@@ -58,7 +59,8 @@ struct ConvList {
 // Appends the kept events sev[0 .. cnt) that are relevant to position (xo, yo) to its list (one warp): the entries not
 // processed yet move to the front, the new ones follow, and the window constants are formed. last: no event follows,
 // so the last window ends at +inf and the last group may be short.
-__device__ __forceinline__ void conv_list_append(ConvList& l, const ConvEvent* sev, int cnt, bool last, int xo, int yo,
+template <int SUB>
+__device__ __forceinline__ void conv_list_append(ConvList<SUB>& l, const ConvEvent* sev, int cnt, bool last, int xo, int yo,
                                                  int fx, int fy, int C, const SolveConst& sk, int lane) {
     int n = l.n;
     const int from = l.groups * CONV_GROUP;
@@ -124,15 +126,15 @@ __device__ __forceinline__ void conv_list_append(ConvList& l, const ConvEvent* s
 }
 
 // CTA per (tile of TX x TY positions, sample), thread = (position, output channel). The sample's events inside the
-// tile's receptive field are compacted into shared memory; CONV_SUB of them at a time, a warp per position builds the
+// tile's receptive field are compacted into shared memory; SUB of them at a time, a warp per position builds the
 // position's own list of relevant events, which its C_out threads then run through in groups of CONV_GROUP, as the
 // fully-connected tile kernel runs through a stage: a branch-free pass with the screen of every event, and the exact
 // loop from the first event after which a crossing cannot be ruled out. A warp's lanes may belong to two positions:
 // they step through their own lists side by side.
 // What bounds it: instruction issue. 12 x 12 x 15 -> 5 x 5 x 40, batch 128: 1.78 -> 0.76 ms; before, every thread tested
 // every event of the tile for its own field and ran the screen one event at a time, lanes of two positions after one
-// another. CONV_SUB 32: 0.90 ms (more barriers).
-template <bool W_SMEM>
+// another. SUB 32: 0.90 ms (more barriers); it takes half the shared memory, see conv_narrow.
+template <bool W_SMEM, int SUB>
 __global__ void __launch_bounds__(1024)
 conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_count, long long ev_cap,
                     const float* __restrict__ W, int X, int Y, int C, int fx, int fy, int C_out, int Xo, int Yo,
@@ -145,15 +147,15 @@ conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_cou
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nwarps = blockDim.x >> 5;
     const int P = TX * TY;
-    ConvList* lists = reinterpret_cast<ConvList*>(smem_raw);
-    ConvEvent* sev = reinterpret_cast<ConvEvent*>(lists + P);  // CONV_SUB + blockDim entries
-    float* sW = reinterpret_cast<float*>(sev + CONV_SUB + blockDim.x);
+    ConvList<SUB>* lists = reinterpret_cast<ConvList<SUB>*>(smem_raw);
+    ConvEvent* sev = reinterpret_cast<ConvEvent*>(lists + P);  // SUB + blockDim entries
+    float* sW = reinterpret_cast<float*>(sev + SUB + blockDim.x);
     const int s = blockIdx.y;
     const int tx0 = (blockIdx.x / tiles_y) * TX, ty0 = (blockIdx.x % tiles_y) * TY;
     const int R = fx * fy * C, ldw = W_SMEM ? (R | 1) : R;  // odd: a row's channels lie in different banks
     if (W_SMEM)
         for (int co = warp; co < C_out; co += nwarps)
-            for (int q = lane; q < R; q += 32) sW[co * ldw + q] = W[co * R + q];
+            for (int q = lane; q < R; q += 32) cp_async4(sW + co * ldw + q, W + co * R + q);
     for (int p = tid; p < P; p += blockDim.x) lists[p].n = lists[p].groups = 0;
     const int co = tid % C_out, pl = tid / C_out;
     const int xo = tx0 + pl / TY, yo = ty0 + pl % TY;
@@ -161,7 +163,7 @@ conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_cou
     const int n_post = Xo * Yo * C_out;
     const int post = (xo * Yo + yo) * C_out + co;
     const long long obase = ((long long)s * n_post + (active ? post : 0)) * k_post;
-    const ConvList& l = lists[active ? pl : 0];
+    const ConvList<SUB>& l = lists[active ? pl : 0];
     const float* wrow = (W_SMEM ? sW : W) + (active ? co * ldw : 0);
     auto weight = [&](int row) { return row >= 0 ? wrow[row] : 0.0f; };
     // Receptive field of the whole tile.
@@ -189,6 +191,7 @@ conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_cou
         }
         const unsigned bal = __ballot_sync(0xffffffffu, keep);
         if (lane == 0) swarp[warp] = __popc(bal);
+        if (W_SMEM && m0 == 0) cp_async_wait_all();
         __syncthreads();
         int off = kept, tot = 0;
         for (int w = 0; w < nwarps; ++w) {
@@ -199,8 +202,8 @@ conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_cou
         kept += tot;
         __syncthreads();
         int head = 0;
-        while (kept - head >= CONV_SUB || (last_round && head < kept) || (last_round && kept == 0)) {
-            const int cnt = min(CONV_SUB, kept - head);
+        while (kept - head >= SUB || (last_round && head < kept) || (last_round && kept == 0)) {
+            const int cnt = min(SUB, kept - head);
             const bool last = last_round && head + cnt == kept;
             for (int p = warp; p < P; p += nwarps)
                 conv_list_append(lists[p], sev + head, cnt, last, tx0 + p / TY, ty0 + p % TY, fx, fy, C, sk, lane);
@@ -259,7 +262,7 @@ conv_forward_kernel(const Event* __restrict__ ev, const int* __restrict__ ev_cou
             }
         }
         if (m0 >= E || last_round) break;
-        // The events not in a list yet move to the front (fewer than CONV_SUB).
+        // The events not in a list yet move to the front (fewer than SUB).
         ConvEvent mv;
         const int rest = kept - head;
         if (tid < rest) mv = sev[head + tid];
@@ -1170,12 +1173,21 @@ static void conv_plan(int batch, int Xo, int Yo, int C_out, long long ev_cap, in
     }
 }
 
-template <bool W_SMEM, typename... Args>
+// Where the grid is past about a wave (eight CTAs on each of the 152 SMs), a tile has few neurons and a sample cannot carry many
+// events, the CTAs take half the lists' length and half the warps, so that twice as many are resident: 1 filter 5 x 5 over 28 x
+// 28, 128 samples of 10 / 74 / 400 events 37 / 44 / 58 -> 27 / 31 / 55 us (19 / 28 / 97 without lists), 2 filters 3 x 3 x 3 over
+// 28 x 24, 186 samples 56 / 80 / 93 -> 38 / 57 / 74. With many events, or on smaller grids, it is slower: 9 filters 5 x 5 x 15 over
+// 12 x 12, 1024 samples of 2000 events 767 -> 830 us, 2 filters, 128 samples 111 -> 144.
+static bool conv_narrow(long long ctas, int neurons, long long ev_cap) {
+    return ctas >= 8 * 152 && neurons <= 160 && ev_cap < 8192;
+}
+
+template <bool W_SMEM, int SUB, typename... Args>
 static cudaError_t launch_conv_forward(dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
     const cudaError_t e =
-        (cudaError_t)bats::max_dynamic_smem_set((const void*)bats::conv_forward_kernel<W_SMEM>, (int)smem);
+        (cudaError_t)bats::max_dynamic_smem_set((const void*)bats::conv_forward_kernel<W_SMEM, SUB>, (int)smem);
     if (e != cudaSuccess) return e;
-    return bats::launch(bats::conv_forward_kernel<W_SMEM>, grid, threads, smem, stream, args...);
+    return bats::launch(bats::conv_forward_kernel<W_SMEM, SUB>, grid, threads, smem, stream, args...);
 }
 
 extern "C" int bats_conv_forward(const void* events, const int* ev_count, long long ev_cap, const float* weights,
@@ -1191,21 +1203,27 @@ extern "C" int bats_conv_forward(const void* events, const int* ev_count, long l
     const int Xo = X - fx + 1, Yo = Y - fy + 1;
     int TX, TY;
     conv_plan(batch, Xo, Yo, C_out, ev_cap, TX, TY);
-    const int threads = std::max((TX * TY * C_out + 31) / 32 * 32, 32 * std::min(TX * TY, 8));  // (eight warps make lists)
     const int tiles_x = (Xo + TX - 1) / TX, tiles_y = (Yo + TY - 1) / TY;
-    const size_t base_smem = TX * TY * sizeof(bats::ConvList) + (bats::CONV_SUB + threads) * sizeof(bats::ConvEvent);
+    const bool narrow = conv_narrow((long long)tiles_x * tiles_y * batch, TX * TY * C_out, ev_cap);
+    const int threads = std::max((TX * TY * C_out + 31) / 32 * 32, 32 * std::min(TX * TY, narrow ? 4 : 8));  // (they make lists)
+    const size_t list = narrow ? sizeof(bats::ConvList<32>) : sizeof(bats::ConvList<64>);
+    const size_t base_smem = TX * TY * list + ((narrow ? 32 : 64) + threads) * sizeof(bats::ConvEvent);
     const size_t w_smem = (size_t)C_out * ((fx * fy * C) | 1) * sizeof(float);
     const bool w_in_smem = base_smem + w_smem <= 200 * 1024;
     const size_t smem = base_smem + (w_in_smem ? w_smem : 0);
     dim3 grid(tiles_x * tiles_y, batch);
     const bats::SolveConst sk = bats::make_solve_const(c, delta_theta_tau, tau, max_simulation);
     const bats::Event* evs = reinterpret_cast<const bats::Event*>(events);
-    BATS_CUDA(w_in_smem ? launch_conv_forward<true>(grid, threads, smem, stream, evs, ev_count, ev_cap, weights, X, Y,
-                                                    C, fx, fy, C_out, Xo, Yo, TX, TY, tiles_y, k_post, sk, n_spikes, a,
-                                                    x, times, post_exp_tau)
-                        : launch_conv_forward<false>(grid, threads, smem, stream, evs, ev_count, ev_cap, weights, X, Y,
-                                                     C, fx, fy, C_out, Xo, Yo, TX, TY, tiles_y, k_post, sk, n_spikes, a,
-                                                     x, times, post_exp_tau));
+    auto launch = [&](auto w, auto sub) {
+        return launch_conv_forward<w(), sub()>(grid, threads, smem, stream, evs, ev_count, ev_cap, weights, X, Y, C, fx, fy,
+                                               C_out, Xo, Yo, TX, TY, tiles_y, k_post, sk, n_spikes, a, x, times, post_exp_tau);
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    using Half = std::integral_constant<int, 32>;
+    using Full = std::integral_constant<int, 64>;
+    BATS_CUDA(w_in_smem ? (narrow ? launch(Yes{}, Half{}) : launch(Yes{}, Full{}))
+                        : (narrow ? launch(No{}, Half{}) : launch(No{}, Full{})));
     BATS_CUDA(cudaGetLastError());
     return BATS_OK;
 }

@@ -18,21 +18,11 @@
 // The suffix sums are accumulated in the reference's order (ascending k from p, fused
 // multiply-add), so SA_p equals the reference's cumul_f1 for the same pre spike bit for bit.
 #include "common.cuh"
+#include "async_copy.cuh"
 #include "pipeline.cuh"
 #include "abi_util.h"
 
 namespace bats {
-
-// Asynchronous 4- and 8-byte global -> shared copies (cp.async): every copy of a staging loop is in
-// flight at once, with no register round trip; cp_async_wait_all() waits for the thread's copies.
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 
 // One thread per (sample, post neuron): recurrent (reset) errors in place, factors, suffix tables.
 //   recurrent: propagate_recurrent_errors.cu:17-22   factors: compute_factors.cu:20-30

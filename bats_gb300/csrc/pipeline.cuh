@@ -5,6 +5,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "async_copy.cuh"
 
 namespace bats {
 
@@ -12,10 +13,6 @@ constexpr unsigned long long BATS_WAIT_NS = 2000000000ull;  // give up after 2 s
 constexpr uint32_t BATS_SUSPEND_NS = 2000;                   // per try_wait: sleep until the phase completes,
                                                              // at most this long
 constexpr int BATS_STATUS_TIMEOUT = 1;
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
