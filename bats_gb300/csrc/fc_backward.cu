@@ -260,21 +260,49 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
     int n_in = 0;
     if (n_spikes) {
         n_in = lane < cnt ? min(max(n_spikes[nb + lane], 0), K) : 0;
-    } else {  // the slots before the first +inf, a row on the lanes (K <= 32)
-#pragma unroll 16
-        for (int r = 0; r < cnt; ++r) {
-            const unsigned silent = __ballot_sync(0xffffffffu, lane >= K || isinf(t[(nb + r) * K + lane]));
-            if (lane == r) n_in = silent ? __ffs(silent) - 1 : 32;
+    } else {  // the slots before the first +inf: the rows' slots as they lie, 32 at a time, eight loads in flight
+        const float* rows = t + nb * K;
+        unsigned silent = 0u;  // lane i: which of the slots 32 i .. are +inf
+        for (int i0 = 0; i0 < K; i0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int q = (i0 + u) * 32 + lane;
+                v[u] = i0 + u < K && q < cnt * K ? rows[q] : BATS_INF;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const unsigned b = __ballot_sync(0xffffffffu, isinf(v[u]));
+                if (lane == i0 + u) silent = b;
+            }
         }
+        // Lane r: the K bits of its row.
+        const int bit = lane * K, word = bit >> 5;
+        const unsigned lo = __shfl_sync(0xffffffffu, silent, word), hi = __shfl_sync(0xffffffffu, silent, min(31, word + 1));
+        const unsigned row = __funnelshift_r(lo, hi, bit & 31) | (K < 32 ? ~0u << K : 0u);
+        if (lane < cnt) n_in = row ? __ffs(row) - 1 : 32;
     }
-    // Inclusive prefix of the counts over the warp's lanes.
-    int incl = n_in;
+    if (!__any_sync(0xffffffffu, n_in > 0)) {  // silent neurons
+        if (lane < cnt) {
+            for (int k = 0; k < n_before; ++k) err_out[(nb + lane) * K + k] = 0.0f;
+            nvalid[nb + lane] = 0;
+            if (head_t) {
+                head_t[nb + lane] = make_float2(BATS_INF, BATS_INF);
+                head_ab[nb + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        }
+        return;
+    }
+    // Inclusive prefix over the warp's lanes of the entries: the counts, and one more for a full row of 32, so that slot k of
+    // neighbouring neurons lies in different banks (K 32, all slots valid, 800 neurons, 256 samples: 241 -> 200 us).
+    const int room = n_in + (n_in == 32 ? 1 : 0);
+    int incl = room;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
     }
-    const int excl = incl - n_in;
+    const int excl = incl - room;
     int r0 = 0, base = 0;
     while (r0 < 32) {
         const unsigned in_round = __ballot_sync(0xffffffffu, lane >= r0 && incl - base <= CAP);
@@ -283,13 +311,13 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
         const bool mine = lane >= r0 && lane < r1;
         const int off = excl - base;  // this lane's first compact entry (valid when mine)
         if (mine)
-            for (int k = 0; k < n_in; ++k) sm.owner[off + k] = (unsigned char)lane;
+            for (int k = 0; k < room; ++k) sm.owner[off + k] = (unsigned char)lane;
         __syncwarp();
         for (int q0 = 0; q0 < V; q0 += 32) {
             const int q = q0 + lane;
             const int r = q < V ? sm.owner[q] : 0;
             const int ro = __shfl_sync(0xffffffffu, excl, r) - base;
-            if (q < V) {
+            if (q < V && q - ro < 32) {
                 const long long src = (nb + r) * K + (q - ro);
                 cp_async4(sm.t + q, t + src);
                 cp_async4(sm.z + q, z + src);
@@ -333,8 +361,11 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
             }
         }
         // Tables: a lane per four consecutive entries of a neuron, each entry's sums upwards from its own spike, the four
-        // chains side by side; the first two entries also into (t, x), for the head.
+        // chains side by side; the first two entries also into (t, x), for the head. Where most lanes have a neuron of about as
+        // many spikes, the lanes are the neurons, four entries further on each time: all sums of a step are then equally long
+        // (248 neurons, 677 samples, K 10, half the slots valid: 22.9 -> 20.7 us).
         const int fours = (n + 3) >> 2;
+        const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)fours);
         int fours_incl = fours;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -342,16 +373,20 @@ bwd_prep_counted_kernel(const float* __restrict__ t, const int* __restrict__ n_s
             if (lane >= o) fours_incl += y;
         }
         const int fours_all = __shfl_sync(0xffffffffu, fours_incl, 31), fours_from = fours_incl - fours;
-        __syncwarp();
-        for (int g = 0; g < fours; ++g) sm.owner[fours_from + g] = (unsigned char)lane;
-        __syncwarp();
-        for (int i0 = 0; i0 < fours_all; i0 += 32) {
-            const int i = i0 + lane;
-            const int r = i < fours_all ? sm.owner[i] : 0;
+        const bool even = 32 * most <= 2 * fours_all;
+        if (!even) {
+            __syncwarp();
+            for (int g = 0; g < fours; ++g) sm.owner[fours_from + g] = (unsigned char)lane;
+            __syncwarp();
+        }
+        const int steps = even ? most : (fours_all + 31) >> 5;
+        for (int st = 0; st < steps; ++st) {
+            const int i = 32 * st + lane;
+            const int r = even ? lane : i < fours_all ? sm.owner[i] : 0;
             const int ro = __shfl_sync(0xffffffffu, excl, r) - base;
             const int nr = __shfl_sync(0xffffffffu, n, r);
-            const int p0 = 4 * (i - __shfl_sync(0xffffffffu, fours_from, r));
-            if (i < fours_all) {
+            const int p0 = 4 * (even ? st : i - __shfl_sync(0xffffffffu, fours_from, r));
+            if (even ? p0 < nr : i < fours_all) {
                 float sa[4] = {0.0f, 0.0f, 0.0f, 0.0f}, sb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 for (int k = p0; k < nr; ++k) {
                     const float ek = sm.e[ro + k], fa = sm.a[ro + k], fb = sm.z[ro + k];
@@ -1055,11 +1090,13 @@ static int launch_prep_layer(const float* post_times, const float* a, const floa
 }
 
 // The prep without factors (K <= 32), by the number of warps of 32 neurons. Up to twenty per SM: without counts the layer
-// kernel (no rounds and no search for the counts: 300 neurons, 256 samples, all 30 slots valid 46 us, 83 in the counted kernel; 10
-// neurons 21 / 40), with counts one warp per CTA, so that they spread over the SMs, and all 32 x 32 slots in one round (10
-// neurons, all valid 25 us, 56 in rounds of 128 slots; 800 neurons, 64 samples, 8.9 valid 28 / 40). Beyond, where the shared
-// memory of whole rows leaves ten warps on an SM, the counted kernel with rounds of 128 slots, eight warps per CTA (800
-// neurons, 256 samples: 42 us, 46 in one round; without counts 54 / 64 in the layer kernel).
+// kernel (no rounds and no search for the counts: 300 neurons, 256 samples, all 30 slots valid 41 us, 83 in the counted kernel; 10
+// neurons 19 / 40), with counts one warp per CTA, so that they spread over the SMs, and all slots in one round (10
+// neurons, all valid 21 us, 56 in rounds of 128 slots; 800 neurons, 64 samples, 8.9 valid 28 / 40), of 32 x 10 slots where K
+// allows, so that more CTAs fit (300 neurons, 256 samples, K 5, all valid 12.5 -> 8.6 us). Beyond, where the shared
+// memory of whole rows leaves ten warps on an SM, the counted kernel with rounds of 128 slots, eight warps per CTA (800 neurons, 256
+// samples, K 30, a fifth / half / all slots valid: 39 / 83 / 142 us with counts, 41 / 84 / 141 without, 77 / 101 / 107 in the
+// layer kernel).
 static int launch_prep(const float* post_times, const int* n_spikes, const float* a, const float* x,
                        const float* post_exp_tau, const float* errors, float* errors_out, long long total, int k_post,
                        float c, float tau, float delta_theta_tau, void* tables, int* nvalid, void* cursor_heads,
@@ -1070,8 +1107,12 @@ static int launch_prep(const float* post_times, const int* n_spikes, const float
         BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<128, 8>, (unsigned)((warps + 7) / 8), 256, 0, stream, post_times,
             n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
             reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab, clear));
+    else if (n_spikes && k_post <= 10)
+        BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<320, 1>, (unsigned)warps, 32, 0, stream, post_times,
+            n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
+            reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab, clear));
     else if (n_spikes)
-        BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<1024, 1>, (unsigned)warps, 32, 0, stream, post_times,
+        BATS_CUDA(bats::launch(bats::bwd_prep_counted_kernel<1056, 1>, (unsigned)warps, 32, 0, stream, post_times,
             n_spikes, a, x, post_exp_tau, errors, errors_out, total, k_post, c, tau, delta_theta_tau,
             reinterpret_cast<float2*>(tables), nvalid, h.t, h.ab, clear));
     else
