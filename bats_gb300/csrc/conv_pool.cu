@@ -1476,7 +1476,12 @@ extern "C" int bats_pool_forward(const int* n_spikes, const float* times, int ba
                  "pool_forward: null pointer");
     const long long total = (long long)batch * (X / 2) * (Y / 2) * C;
     const int per = std::min(bats::POOL_NEURONS, bats::POOL_SMEM / bats::pool_neuron_bytes(K));
-    if (per > 0) {
+    // The merge in shared memory where its rows leave room for enough neurons, or where there are few (thread per neuron / shared,
+    // in us, a third of the slots filled; K 200: 3780 neurons 266 / 200, 7168 267 / 306, 23040 448 / 1065; K 64: 13440 88 / 83,
+    // 45360 208 / 295; K 40: 45360 126 / 105). Rows of one slot lie next to one another as they are (K 1, 918 k neurons 33 / 49, 82 k
+    // 8.4 / 9.3).
+    const bool shared = K > 1 && per > 0 && (K <= 40 || total * K <= 1000000);
+    if (shared) {
         // i / K for i < per * K as the high word of i * inv_k: exact while i * K < 2^32.
         const unsigned inv_k = K > 1 ? (unsigned)(((1ULL << 32) + K - 1) / K) : 0;
         BATS_CUDA(bats::launch(bats::pool_forward_shared_kernel, (unsigned)((total + per - 1) / per), (4 * per + 31) / 32 * 32,
