@@ -23,10 +23,11 @@ constexpr int CONV_WINDOW = 1024;  // events per shared-memory window (two windo
 // (indices and times, coalesced loads by the other warps, one window ahead of the ranking). Warp 0 ranks each
 // window's events in order of appearance, 32 at a time (events of the same neuron ranked by
 // __match_any_sync), writing each spike into its slot, with the per-neuron counts in shared memory when
-// SMEM_COUNTS: a 32-event step then waits on shared memory only. Finally all warps set the slots past each
-// neuron's count to +inf (row by row, contiguous stores) and write the counts.
-// What bounds it: the rows past the counts (a warp per row, 30 to 40 instructions each) where samples are few: four warps took
-// 38 us for a sample of 500 events over 700 rows of 32, sixteen take 19.
+// SMEM_COUNTS: a 32-event step then waits on shared memory only. Finally all threads set the slots past each
+// neuron's count to +inf (along the sample's slots, contiguous stores) and write the counts.
+// What bounds it: the ranking's chain of 32-event steps, then the slots past the counts. With a warp per row of slots, 30 to 40
+// instructions whatever its length, a sample of 500 events over 700 rows of 32 took 19 us (four warps 38), now 15; 1000 samples
+// of 500 events over 700 rows of one slot 51 -> 13 us.
 constexpr int TRAIN_WARPS = 16;
 
 template <bool SMEM_COUNTS>
@@ -107,13 +108,17 @@ events_to_trains_kernel(const int* __restrict__ indices, const float* __restrict
         for (int o = 16; o >= 1; o >>= 1) dropped += __shfl_xor_sync(0xffffffffu, dropped, o);
         if (lane == 0 && dropped && overflow) atomicAdd(overflow, dropped);
     }
-    // +inf past each neuron's spikes; the ranking above wrote only the slots below the counts.
-#pragma unroll 4
-    for (int j = warp; j < n_neurons; j += blockDim.x >> 5) {
-        float* row = out_times + tb + (long long)j * k_cap;
-        const int n = cnt[j];
-        for (int k = lane; k < k_cap; k += 32)
-            if (k >= n) row[k] = BATS_INF;
+    // +inf past each neuron's spikes; the ranking above wrote only the slots below the counts. The threads lie along the
+    // sample's slots.
+    const int dj = (int)blockDim.x / k_cap, dk = (int)blockDim.x - dj * k_cap;
+    for (int j = tid / k_cap, k = tid - j * k_cap; j < n_neurons;) {
+        if (k >= cnt[j]) out_times[tb + (long long)j * k_cap + k] = BATS_INF;
+        j += dj;
+        k += dk;
+        if (k >= k_cap) {
+            k -= k_cap;
+            ++j;
+        }
     }
     if (SMEM_COUNTS)
         for (int q = tid; q < n_neurons; q += blockDim.x) out_counts[(long long)s * n_neurons + q] = cnt[q];
@@ -122,8 +127,8 @@ events_to_trains_kernel(const int* __restrict__ indices, const float* __restrict
 static int launch_events_to_trains(const int* indices, const float* times, const int* offsets, int batch,
                                    int max_events, int n_neurons, int k_cap, float* out_times, int* out_counts,
                                    int* overflow, cudaStream_t stream) {
-    // Sixteen warps while the samples leave SMs idle; four, of which more samples fit, past a few per SM (measured at 700 neurons,
-    // sixteen / four: 1 sample 19 / 38 us, 256: 19 / 36, 1024: 87 / 72).
+    // Sixteen warps while the samples leave SMs idle; four, of which more samples fit, past a few per SM (measured at 700 neurons
+    // with a warp per row, sixteen / four: 1 sample 19 / 38 us, 256: 19 / 36, 1024: 87 / 72).
     const int threads = 32 * (batch <= 152 * 4 ? TRAIN_WARPS : CONV_WARPS);
     if (n_neurons <= CONV_SMEM_NEURONS)
         BATS_CUDA(bats::launch(events_to_trains_kernel<true>, batch, threads, (size_t)n_neurons * sizeof(int),
