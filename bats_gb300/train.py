@@ -213,12 +213,15 @@ class FCTrainStep:
         return {f"L{li + 1}.grad_adam": f"L{li + 1}.prep" for li in range(1, len(self.specs))}
 
     def _joined_launches(self):
-        """The first layer's gradient, where it is the larger part of the gradients (by slots times neurons): its CTAs fill
-        the GPU about once, and placed around another gradient's last CTAs some SMs get a third more of them than
-        others (1024-1024-20 neurons, 4096 samples: 7.03 ms a step, 6.62 with the wait; 784-800-800-10, 256 samples, where
-        the second layer's is larger: 1.308 and 1.321 ms)."""
+        """The first layer's gradient, where it is the larger part of the gradients (by slots times neurons) and large: its CTAs
+        then fill the GPU for long, and placed around another gradient's last CTAs some SMs get a third more of them than others
+        (us a step apart / with the wait: 1024-1024-20 neurons, 16 slots an input, 4096 samples 5917 / 5521, 1024 samples 1532 /
+        1526; 784-800-10, 4096 samples 2366 / 2290). Smaller ones gain more beside it (1024 samples 643 / 657; 300-200-10, 8
+        slots, 4096 samples 853 / 876; 700-64-20, 16 slots, 300 samples 181 / 202), and so do those that are the smaller part
+        (784-800-800-10, 256 samples 1124 / 1172)."""
         work = [ev.n_neurons * ev.k * spec.n_neurons for ev, spec in zip(self.ev, self.specs)]
-        return ("L1.grad_adam",) if len(work) > 1 and work[0] >= sum(work[1:]) else ()
+        large = self.B * work[0] >= 2_500_000_000  # batch x slots x neurons
+        return ("L1.grad_adam",) if len(work) > 1 and work[0] >= sum(work[1:]) and large else ()
 
     def _enqueue(self, main, aux=None) -> None:
         """Enqueue one step on the torch stream `main` (and `aux`: see enqueue_launches)."""
