@@ -753,7 +753,11 @@ extern "C" int bats_lif_forward_fc_default_algo(int batch, int n_post, int ev_ca
     //   at most 8 neurons (three quarters of a tile idle): always (4 neurons, 4096 samples: 199 / 343)
     //   at most 16: 20 warps (12 neurons, 1024 samples 66 / 74, 168 / 164; 16 and 4096: 715 / 433, above the line)
     //   at most 32: 16 warps (32 neurons, 256 samples: 50 / 87, 118 / 148, 259 / 363; 512 samples: 214 / 160, above)
-    //     (output layers, which spike; silent ones pay: 24 neurons, 256 samples of 718 events 56 / 42)
+    //     These are output layers, which spike, on batches of uneven samples, where a tile lasts as long as its longest one: 32
+    //     neurons, 256 samples of 2400 events, sigma of their logarithm 0.3, 6 spikes a neuron 262 / 380 to 575. Layers that
+    //     stay silent pay (24 neurons, 256 samples of 718 events 54 / 40, of 2880 197 / 127), and so do even batches of few
+    //     spikes (32 neurons, 256 samples of 719, 2 spikes 70 / 50); no host knows either. (Tiles through the quiet beginning
+    //     and a second launch of warps per neuron from there: silent 132 us at 2880 events, but 30 us on top of every spiking layer.)
     //   wider: 8 warps (131 neurons, 32 samples: 31 / 64, 70 / 156, 136 / 388; silent layers 15 / 21, 44 / 58; twice as
     //   many warps are still faster where the neurons spike, 52 / 70, 120 / 158, but not where they are silent, 79 / 58)
     const long long warps = (long long)batch * n_post;
