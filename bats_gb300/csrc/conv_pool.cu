@@ -18,9 +18,11 @@
 //
 // Backward (replaces compute_weights_gradient_conv and propagate_errors_to_pre_spikes_conv,
 // .../Backpropagation/compute_weights_gradient_conv.cu:11-61, propagate_errors_to_pre_spikes_conv.cu:11-89):
-// one CTA per sample, one thread per filter tap (c_out, dx, dy); per event the thread looks up the
-// post neuron (x-dx, y-dy, c_out), its first spike after the event, and adds the gradient to the
-// filter entry it owns (no atomics) and the weighted error term to the event's error.
+// per event and filter tap (c_out, dx, dy), the post neuron (x-dx, y-dy, c_out)'s first spike after the event gives a
+// gradient term and a weighted error term. A cluster of eight CTAs per sample (group), each with a copy of the filter gradient
+// in shared memory, added up in rank order; no atomics. With the events grouped by input position: a thread per tap
+// (conv_backward_taps_kernel) or, where few neurons spike, a lane per event (conv_backward_grouped_kernel); without,
+// conv_backward_cluster_kernel in time order. Filters too large for shared memory: one CTA per sample (conv_backward_kernel).
 //
 // Pooling (replaces aggregate_spikes_conv + argsort, .../Inference/aggregate_spikes_conv.cu:6-43,
 // Wrappers/Inference/aggregate_spikes_conv.py:10-28; backward bats/Layers/PoolingLayer.py:55-66):

@@ -1018,8 +1018,8 @@ bwd_pre_err_narrow_kernel(const Event* __restrict__ ev, const int* __restrict__ 
 // Sums the per-tile partials of each event in tile order and writes the sum to the event's slot.
 __global__ void pre_err_scatter_kernel(const float* __restrict__ partial, const Event* __restrict__ ev,
                                        const int* __restrict__ ev_slot, const int* __restrict__ ev_count,
-                                       long long ev_cap, int n_tiles, long long slots_per_sample, float tau_s,
-                                       float tau, float* __restrict__ pre_err) {
+                                       long long ev_cap, int n_tiles, long long slots_per_sample,
+                                       float* __restrict__ pre_err) {
     pdl_prologue();
     const int s = blockIdx.y;
     const int E = ev_count[s];
@@ -1280,19 +1280,14 @@ extern "C" int bats_weights_gradient(const void* events, const int* ev_count, co
         if (events_bucketed)
             flags = reinterpret_cast<int*>(static_cast<char*>(workspace) + grad_partials_bytes(groups, n_post, n_pre));
     }
-    const int tile = grad_tile_for(n_post);
-    if (tile == 32)
+    if (grad_tile_for(n_post) == 32)
         BATS_CUDA(launch_grad<32>(events, ev_count, events_bucketed, bucket_offsets, n_buckets, ev_cap, post_times,
                                   tables, nvalid, cursor_heads, batch, n_post, k_post, n_pre, group, groups, part,
                                   flags, stream));
-    else if (tile == 64)
+    else
         BATS_CUDA(launch_grad<64>(events, ev_count, events_bucketed, bucket_offsets, n_buckets, ev_cap, post_times,
                                   tables, nvalid, cursor_heads, batch, n_post, k_post, n_pre, group, groups, part,
                                   flags, stream));
-    else
-        BATS_CUDA(launch_grad<128>(events, ev_count, events_bucketed, bucket_offsets, n_buckets, ev_cap, post_times,
-                                   tables, nvalid, cursor_heads, batch, n_post, k_post, n_pre, group, groups, part,
-                                   flags, stream));
     if (group == 1) return BATS_OK;  // per-sample gradient (B, N_post, N_pre)
     BATS_CUDA(launch_reduce(part, n_post, n_pre, groups, mean ? (float)batch : 1.0f, grad, flags, GRAD_FLAG_TILE,
                             (n_post + GRAD_FLAG_TILE - 1) / GRAD_FLAG_TILE, n_buckets, stream));
@@ -1330,19 +1325,14 @@ extern "C" int bats_weights_gradient_adam(const void* events, const int* ev_coun
     } else {
         BATS_REQUIRE(grad, BATS_ERR_NULL, "weights_gradient_adam: one group (group >= batch) needs grad");
     }
-    const int tile = grad_tile_for(n_post);
-    if (tile == 32)
+    if (grad_tile_for(n_post) == 32)
         BATS_CUDA(launch_grad<32>(events, ev_count, events_bucketed, bucket_offsets, n_buckets, ev_cap, post_times,
                                   tables, nvalid, cursor_heads, batch, n_post, k_post, n_pre, group, groups, part,
                                   flags, stream));
-    else if (tile == 64)
+    else
         BATS_CUDA(launch_grad<64>(events, ev_count, events_bucketed, bucket_offsets, n_buckets, ev_cap, post_times,
                                   tables, nvalid, cursor_heads, batch, n_post, k_post, n_pre, group, groups, part,
                                   flags, stream));
-    else
-        BATS_CUDA(launch_grad<128>(events, ev_count, events_bucketed, bucket_offsets, n_buckets, ev_cap, post_times,
-                                   tables, nvalid, cursor_heads, batch, n_post, k_post, n_pre, group, groups, part,
-                                   flags, stream));
     dim3 grid((n_pre + 31) / 32, (n_post + 31) / 32), block(32, 8);
     if (grad && groups > 1 && (long long)grid.x * grid.y < 2 * 152) {
         // Few weight tiles (a narrow layer) for many partials: the tile grid would leave most SMs idle while
@@ -1363,7 +1353,7 @@ extern "C" int bats_weights_gradient_adam(const void* events, const int* ev_coun
 
 extern "C" size_t bats_pre_errors_workspace_bytes(int batch, long long ev_cap, int n_post) {
     if (n_post <= 32) return 0;  // narrow layers: event-parallel kernel, no partials
-    const int tile = n_post <= 32 ? 32 : (n_post <= 64 ? 64 : 128);
+    const int tile = n_post <= 64 ? 64 : 128;
     const long long tiles = (n_post + tile - 1) / tile;
     return (size_t)batch * ev_cap * tiles * sizeof(float);
 }
@@ -1387,9 +1377,9 @@ static int launch_pre_err(const void* events, const int* ev_count, long long ev_
 
 static int pre_errors_impl(const void* events, const int* ev_slot, const int* ev_count, long long ev_cap,
                            const float* weights_t, int ld, const float* post_times, const void* tables,
-                               const int* nvalid, int batch, int n_post, int k_post, int n_pre, int k_pre,
-                               float tau_s, float tau, float* pre_errors, void* workspace, size_t workspace_bytes,
-                               bool zero, cudaStream_t stream) {
+                           const int* nvalid, int batch, int n_post, int k_post, int n_pre, int k_pre, float tau_s,
+                           float tau, float* pre_errors, void* workspace, size_t workspace_bytes, bool zero,
+                           cudaStream_t stream) {
     BATS_REQUIRE(batch >= 0 && n_post >= 0 && n_pre >= 0 && k_post > 0 && k_pre > 0 && ld >= n_post && ld % 4 == 0,
                  BATS_ERR_BAD_SHAPE, "pre_errors: bad shape");
     if (batch == 0 || n_pre == 0) return BATS_OK;
@@ -1420,11 +1410,7 @@ static int pre_errors_impl(const void* events, const int* ev_slot, const int* ev
     BATS_CUDA((cudaError_t)bats::device_status(&status));
     int rc;
     int tiles;
-    if (n_post <= 32) {
-        rc = launch_pre_err<32>(events, ev_count, ev_cap, weights_t, ld, post_times, tables, nvalid, batch, n_post,
-                                k_post, tau_s, tau, part, status, stream);
-        tiles = (n_post + 31) / 32;
-    } else if (n_post <= 64) {
+    if (n_post <= 64) {
         rc = launch_pre_err<64>(events, ev_count, ev_cap, weights_t, ld, post_times, tables, nvalid, batch, n_post,
                                 k_post, tau_s, tau, part, status, stream);
         tiles = (n_post + 63) / 64;
@@ -1437,7 +1423,7 @@ static int pre_errors_impl(const void* events, const int* ev_slot, const int* ev
     // A few CTAs per sample, striding over its events (most samples have far fewer events than slots).
     dim3 g2((unsigned)std::min<long long>((ev_cap + 255) / 256, 4), batch);
     BATS_CUDA(bats::launch(bats::pre_err_scatter_kernel, g2, 256, 0, stream, part,
-        reinterpret_cast<const bats::Event*>(events), ev_slot, ev_count, ev_cap, tiles, slots, tau_s, tau, pre_errors));
+        reinterpret_cast<const bats::Event*>(events), ev_slot, ev_count, ev_cap, tiles, slots, pre_errors));
     BATS_CUDA(cudaGetLastError());
     return BATS_OK;
 }

@@ -739,7 +739,7 @@ static int forward_fc_impl(const void* events, const int* ev_count, long long ev
     if (pick && 100 * w128 >= 115 * w64 && w64 * batch <= 152 * 20)
         return bats::launch_tile<64, 8, 6>(screen, events, ev_count, ev_cap, weights_t, ld, batch, n_post, k_post, sk,
                                              n_spikes, a, x, times, post_exp_tau, status, pad, stream);
-    // 8-event stages: half the shared memory of 16-event stages, so 7 CTAs (28 consumer warps) fit on an SM
+    // 8-event stages: half the shared memory of 16-event stages (26 KB), so 8 CTAs (32 consumer warps) fit on an SM
     // instead of 4, and a replay after a possible crossing covers fewer events.
     return bats::launch_tile<128, 8, 6>(screen, events, ev_count, ev_cap, weights_t, ld, batch, n_post, k_post, sk,
                                           n_spikes, a, x, times, post_exp_tau, status, pad, stream);

@@ -1,7 +1,6 @@
 // Per-sample time sort of all pre-synaptic spikes of a layer (one CTA per sample).
-// The sort runs in shared memory whenever the sample's items fit (up to 17408 items with 16-bit slot
-// values for batches of at most 152 samples, 7680 for larger ones), else in a per-sample slice of the
-// caller's workspace.
+// The sort runs in shared memory whenever the sample's items fit (16448 items with 16-bit slot values for batches of at most
+// 152 samples, 6720 for larger ones; 12320 and 4096 with 32-bit ones), else in a per-sample slice of the caller's workspace.
 //
 // Replaces get_sorted_spikes_indices + the three take_along_axis gathers + compute_pre_exps
 // (bats/CudaKernels/Wrappers/Inference/get_sorted_spikes_indices.py:7-17,
@@ -9,7 +8,7 @@
 // The reference sorts every (neuron, slot) of the batch on the device with argpartition after a
 // host sync on the largest spike count; here every sample's valid slots (time < +inf) are
 // gathered into shared memory, dealt into equal spans of the sample's time and ranked inside their span by
-// (time, slot) (crowded or very large samples by an LSD radix sort), so the event list needs no host sync and no
+// (time, slot) (samples of many equal times and very large ones by an LSD radix sort), so the event list needs no host sync and no
 // padding to the batch maximum. Ties keep slot order, which makes the order deterministic.
 //
 // CTA b sorts sample b, or sample sample_order[b] when an order is given (the samples longest first: on a
@@ -32,20 +31,11 @@ constexpr int SORT_WIDE_CAP = 1024;
 // Items held in shared memory (two key buffers and two value buffers): slot values are 16-bit when the
 // layer has at most 65536 slots (cap = n_pre * k_pre), else 32-bit. Batches of at most SORT_SMALL_BATCH
 // samples (no more CTAs than a GB300 has SMs: one CTA per SM costs no parallelism) get as many items as
-// 227 KB holds (SortCaps max_u16 / max_u32); larger batches keep two CTAs per SM (u16 / u32 items, at most
-// 113 KB with the counters). Samples with more valid slots than that sort in global scratch. The capacities
-// leave room for the counters (SortShared: 18.5 KB at 256 threads, 34.9 KB at 512).
+// 227 KB holds beside the counters (SortShared: 34.9 KB at 512 threads); larger batches keep two CTAs per SM, at most
+// 113 KB each. Samples with more valid slots than that sort in global scratch. (Layers of up to SORT_WIDE_CAP slots
+// always fit.)
 constexpr int SORT_SMALL_BATCH = 152;
-template <int T>
-struct SortCaps;
-template <>
-struct SortCaps<256> {
-    static constexpr int max_u16 = 17408, max_u32 = 13312, u16 = 7680, u32 = 4096;
-};
-template <>
-struct SortCaps<512> {
-    static constexpr int max_u16 = 16448, max_u32 = 12320, u16 = 6720, u32 = 4096;
-};
+constexpr int SORT_ROOM_MAX_U16 = 16448, SORT_ROOM_MAX_U32 = 12320, SORT_ROOM_U16 = 6720, SORT_ROOM_U32 = 4096;
 
 template <int T>
 struct SortShared {
@@ -553,15 +543,11 @@ sort_events_kernel(const float* __restrict__ times, const int* __restrict__ pre_
 #include "abi_util.h"
 
 // Shared-memory items and value width for a batch of samples with cap slots each (see SORT_SMALL_BATCH).
-template <int T>
-static int sort_room(bool small, bool u16) {
-    using C = bats::SortCaps<T>;
-    return u16 ? (small ? C::max_u16 : C::u16) : (small ? C::max_u32 : C::u32);
-}
 static void sort_plan(int batch, long long cap, int* smem_cap, bool* u16) {
     *u16 = cap <= 65536;
     const bool small = batch <= bats::SORT_SMALL_BATCH;
-    const int room = cap > bats::SORT_WIDE_CAP ? sort_room<512>(small, *u16) : sort_room<256>(small, *u16);
+    const int room = *u16 ? (small ? bats::SORT_ROOM_MAX_U16 : bats::SORT_ROOM_U16)
+                          : (small ? bats::SORT_ROOM_MAX_U32 : bats::SORT_ROOM_U32);
     *smem_cap = (int)std::min<long long>(room, (cap + 31) / 32 * 32);
 }
 
@@ -616,12 +602,11 @@ static int sort_events_impl(const float* pre_times, const int* pre_counts, int b
     bool u16;
     sort_plan(batch, cap, &smem_cap, &u16);
     unsigned char* scratch = reinterpret_cast<unsigned char*>(workspace);
-    const bool wide = cap > bats::SORT_WIDE_CAP;
     cudaError_t err;
-    if (u16)
-        err = wide ? launch_sort<uint16_t, 512>(SORT_ARGS) : launch_sort<uint16_t, 256>(SORT_ARGS);
+    if (!u16)  // (wide)
+        err = launch_sort<uint32_t, 512>(SORT_ARGS);
     else
-        err = wide ? launch_sort<uint32_t, 512>(SORT_ARGS) : launch_sort<uint32_t, 256>(SORT_ARGS);
+        err = cap > bats::SORT_WIDE_CAP ? launch_sort<uint16_t, 512>(SORT_ARGS) : launch_sort<uint16_t, 256>(SORT_ARGS);
     BATS_CUDA(err);
     return BATS_OK;
 }

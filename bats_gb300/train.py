@@ -252,8 +252,8 @@ class FCTrainStep:
         return arr
 
     def native_step(self) -> None:
-        """One training step as a single call of the C ABI's bats_fc_train_step: the same launches, arguments
-        and results as step()."""
+        """One training step as a single call of the C ABI's bats_fc_train_step: the same results as step(), by the same
+        launches on one stream (its pre-errors' other slots are filled with 0 each time instead of kept so)."""
         import ctypes
         layers = self.native_layers()
         need = K.call_size("bats_fc_train_step_workspace_bytes", self.B, ctypes.cast(layers, ctypes.c_void_p),
