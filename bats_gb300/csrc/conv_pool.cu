@@ -548,7 +548,6 @@ conv_backward_taps_kernel(const Event* __restrict__ ev_b, const int* __restrict_
     __shared__ int sslot[32], scc[32];
     __shared__ ConvVote vote;
     const int s0 = (int)blockIdx.y * group, s_end = min(batch, s0 + group);
-    if (form == ConvForm::CHOOSE) conv_vote_count(vote, vs, boff, nvalid, sh);
     const float inv_tau_s = 1.0f / tau_s, inv_tau = 1.0f / tau;  // the error terms' factors, as reciprocals
     const int rank = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -564,12 +563,14 @@ conv_backward_taps_kernel(const Event* __restrict__ ev_b, const int* __restrict_
     const float* Wk = W;
     if (W_SMEM) {
         float* sWf = reinterpret_cast<float*>(kcount + C);
-        for (int q = tid; q < total; q += blockDim.x) sWf[q] = W[q];
+        for (int q = tid; q < total; q += blockDim.x) cp_async4(sWf + q, W + q);
         Wk = sWf;
     }
+    if (form == ConvForm::CHOOSE) conv_vote_count(vote, vs, boff, nvalid, sh);
     const bool has_tap = tid < taps;
     const int co = has_tap ? tid / (sh.fx * sh.fy) : 0, dx = has_tap ? tid / sh.fy % sh.fx : 0;
     const int dy = has_tap ? tid % sh.fy : 0;
+    if (W_SMEM) cp_async_wait_all();
     __syncthreads();
     if (form == ConvForm::CHOOSE && conv_events_form(vote, vs, sh, batch)) {  // uniform over the grid
         if (rank == 0 && tid == 0) grad[(long long)blockIdx.y * total] = __uint_as_float(CONV_LEFT);
